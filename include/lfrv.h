@@ -231,7 +231,7 @@ int lfrv_render_view_dev(lfrv_ctx *ctx, const lfrv_config *cfg, int algorithm,
  * No single reference counterpart: the reference renders one target per process run (main, sources/main.cpp:
  * 349-357). A batch renders many target views, each with its own light field, sizes and options, on device
  * buffers and the context's stream. IBR_gradient jobs with faithful = 0 run warp, set-up and hole filling one
- * after another, then share one persistent CG launch (k_cg_batch) in which every job keeps its own tiles,
+ * after another, then share persistent CG launches (k_cg_strip) in which every job keeps its own blocks,
  * dot products, stop rule and statistics; other jobs run as lfrv_render_view_dev would. The call returns when
  * every output is written. */
 typedef struct lfrv_view_job {

@@ -1985,8 +1985,8 @@ extern "C" int lfrv_render_view_warm_dev(lfrv_ctx *ctx, lfrv_warmstart *net, con
 }
 
 // ====================================================================== batched targets
-// IBR_gradient jobs with the corrected CG share one k_cg_batch launch (per launch at most as many jobs as resident
-// blocks); every other job runs on its own. Per gradient job the batch pool holds U, gx, gy, r, dA, dB (14 N
+// IBR_gradient jobs with the corrected CG share k_cg_strip launches (each as many jobs as fit on chip together); every
+// other job runs on its own. Per gradient job the batch pool holds U, gx, gy, r, dA, dB (14 N
 // floats) and 8 doubles of state.
 // Host-buffer calls pass host_out (per job: a pinned host destination, or nullptr) and sent (per job, zeroed): an
 // IBR_gradient job's output is then copied to host_out as soon as its CG is done, on the copy stream, while the next
@@ -2190,9 +2190,9 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
         if (st && st->energy_trace && st->trace_capacity > 0) trace_total += (size_t)st->trace_capacity;
     }
     if (trace_total) ws.trace.ensure(sizeof(double) * trace_total);
-    // A job with at least as many 64 x 16 tiles as the batched launch has resident blocks fills the GPU on its own:
-    // it gains nothing from sharing a launch, so it runs the single-target persistent CG (shared-memory resident
-    // or TMA form) on its pool buffers, one after another on the context stream. The others share k_cg_batch.
+    // A job that needs more than half of the GPU's blocks on chip gains nothing from sharing a launch (nor does one
+    // too large for it): it runs the single-target CG on its pool buffers, one after another on the context stream.
+    // The others share launches of as many jobs as fit the GPU together.
     const int resident = cg_batch_resident_blocks();
     // a job's final output (the CG's iterate) to its host destination, after what the context stream has queued
     auto send = [&](const Slot &sl) {
@@ -2207,8 +2207,8 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
     std::vector<size_t> grouped;
     for (size_t q = 0; q < batched.size(); ++q) {
         const Slot &sl = batched[q];
-        const long long ntiles = (long long)((sl.G.W + 63) / 64) * ((sl.G.H + 15) / 16);
-        if (ntiles < resident) {
+        const int need = cg_batch_blocks(sl.G.W, sl.G.H, kCgBatchMaxRows);
+        if (need > 0 && 2 * need <= resident) {
             grouped.push_back(q);
             continue;
         }
@@ -2228,76 +2228,86 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
         check_launch("batched job CG");
         send(sl);
     }
-    // the CG of the other gradient jobs, in launches of at most `resident` jobs
-    for (size_t first = 0; first < grouped.size(); first += (size_t)resident) {
-        const size_t cnt = std::min(grouped.size() - first, (size_t)resident);
-        std::vector<CgProblem> probs(cnt);
-        std::vector<int> tiles(cnt);
-        long long total = 0;
-        for (size_t q = 0; q < cnt; ++q) {
-            const Geometry &G = batched[grouped[first + q]].G;
-            tiles[q] = ((G.W + 63) / 64) * ((G.H + 15) / 16);
-            total += tiles[q];
+    // the CG of the other gradient jobs: groups of jobs that fit the GPU together, one launch each. All groups'
+    // descriptors (problems, the problem of every block, barrier words) go up in one copy.
+    struct Group {
+        size_t first, cnt, off_probs, off_blocks, off_bars;
+        int R, used;
+    };
+    std::vector<Group> groups;
+    std::vector<CgProblem> probs(grouped.size());
+    for (size_t q = 0; q < grouped.size(); ++q) {
+        const Slot &sl = batched[grouped[q]];
+        const lfrv_config &cfg = *jobs[sl.job].cfg;
+        float *U = base + sl.off;
+        CgProblem &P = probs[q];
+        P = CgProblem{};
+        P.W = sl.G.W;
+        P.H = sl.G.H;
+        P.max_iter = cfg.cg_max_iter;
+        P.gap_tol = cfg.cg_gap_tol;
+        P.gx = U + 3 * sl.G.N;
+        P.gy = U + 4 * sl.G.N;
+        P.U = sl.seeded ? U + 14 * sl.G.N + 16 : U;
+        P.dA = U + 8 * sl.G.N;
+        P.dB = U + 11 * sl.G.N;
+        P.state = reinterpret_cast<double *>(U + 14 * sl.G.N);
+        P.U0 = sl.seeded ? U : nullptr;
+        const lfrv_stats *jst = jobs[sl.job].stats;
+        const bool traced = jst && jst->energy_trace && jst->trace_capacity > 0;
+        P.trace = traced ? ws.trace.as<double>() + trace_off[grouped[q]] : nullptr;
+        P.trace_cap = traced ? jst->trace_capacity : 0;
+    }
+    size_t meta_bytes = 0;
+    for (size_t first = 0; first < grouped.size();) {
+        Group g{};
+        g.first = first;
+        int need = 0;
+        while (first + g.cnt < grouped.size()) {
+            const CgProblem &P = probs[first + g.cnt];
+            const int b = cg_batch_blocks(P.W, P.H, kCgBatchMaxRows);
+            if (need + b > resident) break;
+            need += b;
+            ++g.cnt;
         }
-        // blocks in proportion to the tiles, at least one each, no more than resident in all
-        std::vector<int> nb(cnt);
-        int used = 0;
-        for (size_t q = 0; q < cnt; ++q) {
-            nb[q] = std::max(1, (int)((long long)resident * tiles[q] / std::max(1LL, total)));
-            nb[q] = std::min(nb[q], tiles[q]);
-            used += nb[q];
+        g.R = cg_batch_rows(&probs[first], (int)g.cnt);
+        for (size_t q = 0; q < g.cnt; ++q) {
+            CgProblem &P = probs[first + q];
+            P.b0 = g.used;
+            P.nb = cg_batch_blocks(P.W, P.H, g.R);
+            g.used += P.nb;
         }
-        while (used > resident) {  // trim the largest allocations
-            size_t big = 0;
-            for (size_t q = 1; q < cnt; ++q)
-                if (nb[q] > nb[big]) big = q;
-            --nb[big];
-            --used;
+        auto place = [&](size_t bytes) {
+            const size_t off = meta_bytes;
+            meta_bytes += (bytes + 255) / 256 * 256;
+            return off;
+        };
+        g.off_probs = place(sizeof(CgProblem) * g.cnt);
+        g.off_blocks = place(sizeof(int) * g.used);
+        g.off_bars = place(sizeof(unsigned int) * 8 * g.cnt);
+        groups.push_back(g);
+        first += g.cnt;
+    }
+    if (!groups.empty()) {
+        std::vector<char> meta(meta_bytes, 0);  // (the barrier words start at zero)
+        for (const Group &g : groups) {
+            std::memcpy(&meta[g.off_probs], &probs[g.first], sizeof(CgProblem) * g.cnt);
+            int *bp = reinterpret_cast<int *>(&meta[g.off_blocks]);
+            for (size_t q = 0; q < g.cnt; ++q)
+                for (int k = 0; k < probs[g.first + q].nb; ++k) bp[probs[g.first + q].b0 + k] = (int)q;
         }
-        std::vector<int> block_prob(used);
-        int b0 = 0;
-        for (size_t q = 0; q < cnt; ++q) {
-            const Slot &sl = batched[grouped[first + q]];
-            const lfrv_config &cfg = *jobs[sl.job].cfg;
-            float *U = base + sl.off;
-            CgProblem &P = probs[q];
-            P.W = sl.G.W;
-            P.H = sl.G.H;
-            P.tiles_x = (sl.G.W + 63) / 64;
-            P.ntiles = tiles[q];
-            P.b0 = b0;
-            P.nb = nb[q];
-            P.max_iter = cfg.cg_max_iter;
-            P.gap_tol = cfg.cg_gap_tol;
-            P.gx = U + 3 * sl.G.N;
-            P.gy = U + 4 * sl.G.N;
-            P.U = sl.seeded ? U + 14 * sl.G.N + 16 : U;
-            P.r = U + 5 * sl.G.N;
-            P.dA = U + 8 * sl.G.N;
-            P.dB = U + 11 * sl.G.N;
-            P.state = reinterpret_cast<double *>(U + 14 * sl.G.N);
-            P.U0 = sl.seeded ? U : nullptr;
-            const lfrv_stats *jst = jobs[sl.job].stats;
-            const bool traced = jst && jst->energy_trace && jst->trace_capacity > 0;
-            P.trace = traced ? ws.trace.as<double>() + trace_off[grouped[first + q]] : nullptr;
-            P.trace_cap = traced ? jst->trace_capacity : 0;
-            for (int k = 0; k < nb[q]; ++k) block_prob[b0 + k] = (int)q;
-            b0 += nb[q];
+        ws.batch_meta.ensure(meta_bytes);
+        LFRV_CUDA(cudaMemcpyAsync(ws.batch_meta.p, meta.data(), meta_bytes, cudaMemcpyHostToDevice, s));
+        char *d_meta = ws.batch_meta.as<char>();
+        GridBarrier gb = fresh_barrier(c);
+        double *part = partial_buf(c, (size_t)14 * resident);
+        for (const Group &g : groups) {
+            gb.count = reinterpret_cast<unsigned int *>(d_meta + g.off_bars);
+            LFRV_CUDA(launch_cg_batch(reinterpret_cast<const CgProblem *>(d_meta + g.off_probs),
+                                      reinterpret_cast<const int *>(d_meta + g.off_blocks), g.R, g.used, part,
+                                      part + (size_t)7 * resident, gb, s, c->launches));
+            for (size_t q = 0; q < g.cnt; ++q) send(batched[grouped[g.first + q]]);
         }
-        ws.batch_meta.ensure(sizeof(CgProblem) * cnt + sizeof(int) * (used + cnt) + 64);
-        char *meta = ws.batch_meta.as<char>();
-        CgProblem *d_probs = reinterpret_cast<CgProblem *>(meta);
-        int *d_block_prob = reinterpret_cast<int *>(meta + sizeof(CgProblem) * cnt);
-        int *d_done = d_block_prob + used;
-        LFRV_CUDA(cudaMemcpyAsync(d_probs, probs.data(), sizeof(CgProblem) * cnt, cudaMemcpyHostToDevice, s));
-        LFRV_CUDA(cudaMemcpyAsync(d_block_prob, block_prob.data(), sizeof(int) * used, cudaMemcpyHostToDevice, s));
-        double *part = partial_buf(c, (size_t)8 * used);
-        const GridBarrier gb = fresh_barrier(c);
-        LFRV_CUDA(launch_cg_batch(d_probs, d_block_prob, (int)cnt, used, part, part + 4 * (size_t)used, d_done, gb, s,
-                                  c->launches));
-        for (size_t q = 0; q < cnt; ++q) send(batched[grouped[first + q]]);
-        // the next launch rewrites the descriptors in batch_meta (the host vectors were staged by the copies)
-        if (first + cnt < grouped.size()) LFRV_CUDA(cudaStreamSynchronize(s));
     }
     // the corrected IBR_color jobs in lockstep (beside the batched CG on the context stream): every round enqueues
     // each running job's certificate, waits once for all of them, then enqueues each job's next FISTA step

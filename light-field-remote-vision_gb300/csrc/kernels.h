@@ -227,24 +227,31 @@ int tv_fgp_default_variant(bool extended);
 // The gap above which the FGP runs in FP32 (its certificate floor is near 4e-4): double-float takes over below it.
 constexpr double kTvExtendedBelow = 2e-3;
 
-// One target of a batched CG launch (k_cg_batch): its image, buffers and the contiguous range of blocks that
-// work on it. state: [0..2] delta, [3] E, [4] gap, [5] iterations (written by the problem's first block).
+// One target of an on-chip CG launch (k_cg_strip): its image, buffers and, in a batched launch, the contiguous range of
+// blocks that work on it. dA, dB: 3 N floats each (the exchanged borders). state: [0..2] gamma = |r|^2, [3] E, [4] gap,
+// [5] iterations (written by the problem's first block).
 struct CgProblem {
-    int W, H, tiles_x, ntiles;
+    int W, H;
     int b0, nb;
     int max_iter;
     double gap_tol;
     const float *gx, *gy;
-    float *U, *r, *dA, *dB;
+    float *U, *dA, *dB;
     double *state;
     const float *U0;  // anchor when U holds a seed (nullptr: U is the anchor)
     double *trace;    // energy after each iteration (nullptr: none), at most trace_cap entries
     int trace_cap;
 };
-// Blocks of a batched launch: as many as can be resident with k_cg_batch's shape.
+// Blocks of a batched launch: as many as can be resident at once.
 int cg_batch_resident_blocks();
-cudaError_t launch_cg_batch(const CgProblem *d_probs, const int *d_block_prob, int nprob, int blocks, double *partA,
-                            double *partB, int *done, GridBarrier gb, cudaStream_t st, LaunchCounter &lc);
+// Rows per unit (R) of a batched launch of `count` problems (their W and H), 0 when they do not fit together; blocks of
+// one of them at R (0: its borders do not fit dA and dB).
+int cg_batch_rows(const CgProblem *probs, int count);
+int cg_batch_blocks(int W, int H, int R);
+constexpr int kCgBatchMaxRows = 28;
+// gb.count: 8 zeroed words per problem. partA, partB: 7 doubles per block each.
+cudaError_t launch_cg_batch(const CgProblem *d_probs, const int *d_block_prob, int R, int blocks, double *partA,
+                            double *partB, GridBarrier gb, cudaStream_t st, LaunchCounter &lc);
 
 // Persistent ROF instantiations (iterations per super-step x block size), chosen per image size by the host's
 // autotuner; v indexes them.

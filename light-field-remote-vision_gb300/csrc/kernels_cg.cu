@@ -788,23 +788,42 @@ __global__ void __launch_bounds__(kPersistThreads) k_cg_persistent(int W, int H,
     }
 }
 
-// Shared-memory resident form of the corrected CG (the iteration of k_cg_persistent) for images of at most
-// kResMaxTiles tiles per SM. Block b owns tiles b, b + G, ... and keeps r (3 planes) and d (3 planes with a
-// one-pixel halo) of each in shared memory for the whole solve; only u stays in global memory. The phases
-// exchange tile borders alone, through `bord` (set 0: r; sets 1, 2: d by iteration parity, since phase A still
-// reads the previous iteration's d as d_old):
-//   phase A: d = r + beta d_old on the interior; the halo's d from the neighbours' published r and d_old
-//            borders; q = A d, d . q; publish the border rows and columns of d;
-//   phase B: the halo's d from the neighbours' new borders; q = A d; u += alpha d; r -= alpha q, r . r;
-//            publish the borders of r.
-// Per pixel the arithmetic is k_cg_persistent's. Borders written by other blocks are read through L2 (__ldcg)
-// after the grid barrier that follows their writing.
-constexpr int kResThreads = kTileX * kTileY;          // one tile pixel per thread
-constexpr int kResMaxTiles = 7;                       // tiles per block: 7 x 26.5 KB of shared memory
-constexpr int kResPix = kTileX * kTileY;              // r plane (interior only)
-constexpr int kResPlane = kHaloY * kHaloX;            // d plane with its halo: 18 x 66 floats
-constexpr int kResBorder = 2 * kTileX + 2 * kTileY;   // border values per plane: top, bottom, left, right rows
-constexpr size_t kResTileBytes = (size_t)3 * (kResPix + kResPlane) * sizeof(float);
+// On-chip strip form of the corrected CG (units of 64 x R pixels and one channel, kStripUnits spatial units per SM,
+// R <= 28).
+//
+// One warp owns one unit: lane l holds columns 2l and 2l + 1 of its rows. r (with a ring of ghost cells) and s = A d
+// stay in shared memory, x and d in registers (they meet no neighbour), so an iteration touches no global memory
+// beyond the units' borders. A ghost cell inside the image is a copy of the neighbour unit's pixel; one outside it
+// repeats the border pixel, which is the operator's one-sided difference there, so the stencil has no border cases.
+//
+// One barrier per iteration (Chronopoulos and Gear's form of CG): with w = A r, gamma = r . r and delta = r . w,
+//   beta = gamma / gamma_old, alpha = gamma / (delta - beta gamma / alpha_old),
+//   s = w + beta s, d = r + beta d, x += alpha d, r -= alpha s,
+// which are CG's iterates with both dot products of an iteration in one reduction. A unit publishes the border of
+// its w (not of r) before the barrier; afterwards the neighbours apply the same recurrence to their copies of its
+// border (s_h = w_h + beta s_h, r_h -= alpha s_h), so their halo of r equals the owner's r bit for bit without a
+// second exchange. Borders and block partials are double-buffered by iteration parity: a block that has passed the
+// barrier writes the next set while a slower one still reads this one. A step whose denominator is not positive
+// (rounding at FP32's floor, long after the certified gap) restarts from the residual (beta = 0).
+// Dot products: FP32 per lane and warp, FP64 across warps and blocks, as in the streamed form.
+//
+// Measured against the shared-memory form with two barriers an iteration that stood here before: 1024^2 (152 blocks,
+// R = 28) 154 -> 100 us for 7 iterations, 512^2 12.1 -> 5.0 us an iteration, 64^2 9.3 -> 3.4 us. Bound at 1024^2 by the
+// walks (about 160 cycles a row of a warp, three warps a scheduler), below 512^2 by the reduction, the barrier and the
+// FP64 scalars between two iterations.
+constexpr int kStripUnits = 4;                               // spatial units per block
+constexpr int kStripWarps = kStripUnits * 3, kStripThreads = kStripWarps * 32;
+constexpr int kStripCols = 64;
+constexpr int kStripClusterBlocks = 16, kStripClusterR = 8;
+constexpr int kStripSlots = 7;                               // gamma x 3, delta x 3, the starting energy
+
+constexpr int kStripRow = kStripCols + 4;                    // a row of r: 2 words (ghost in the second), 64 columns, ghost
+
+// per warp: r with its ghost rows (and one row read ahead of need), s
+__host__ __device__ constexpr int strip_warp_floats(int R) { return (R + 3) * kStripRow + R * kStripCols; }
+constexpr size_t strip_smem(int R) { return sizeof(float) * kStripWarps * (size_t)strip_warp_floats(R); }
+// top row, bottom row, left column, right column
+__host__ __device__ constexpr int strip_border(int R) { return 2 * kStripCols + 2 * R; }
 
 // a / b in FP64 for the solver's scalars: an FP32 reciprocal refined by Newton steps in FP64 (a few dependent
 // FMAs instead of the full division sequence, whose latency sits on the path every block waits for). The
@@ -820,429 +839,311 @@ __device__ __forceinline__ double res_div(double a, double b) {
     return fma(r, fma(-b, q, a), q);
 }
 
-// Halo slot p (in [0, kResBorder)) of a tile at tile coordinates (tx, ty): its index in a d plane, and the
-// neighbour tile and border slot it is read from (nt = -1: outside the image, the value is 0). Border slots:
-// top row [0, 64), bottom row [64, 128), left column [128, 144), right column [144, 160).
-__device__ __forceinline__ void res_halo_slot(int p, int t, int tx, int ty, int tiles_x, int tiles_y, int &si,
-                                              int &nt, int &np) {
-    nt = -1;
-    np = 0;
-    if (p < kTileX) {  // row above <- bottom row of the tile above
-        si = p + 1;
-        if (ty > 0) nt = t - tiles_x, np = kTileX + p;
-    } else if (p < 2 * kTileX) {  // row below <- top row of the tile below
-        const int q = p - kTileX;
-        si = (kTileY + 1) * kHaloX + q + 1;
-        if (ty + 1 < tiles_y) nt = t + tiles_x, np = q;
-    } else if (p < 2 * kTileX + kTileY) {  // left column <- right column of the tile to the left
-        const int q = p - 2 * kTileX;
-        si = (q + 1) * kHaloX;
-        if (tx > 0) nt = t - 1, np = 2 * kTileX + kTileY + q;
-    } else {  // right column <- left column of the tile to the right
-        const int q = p - 2 * kTileX - kTileY;
-        si = (q + 1) * kHaloX + kHaloX - 1;
-        if (tx + 1 < tiles_x) nt = t + 1, np = 2 * kTileX + q;
-    }
+// cg_start_values for one channel at (x, y): the initial residual; e receives the pixel's energy. Branch-free (a
+// neighbour outside the image is the pixel itself, a gradient across the border 0), so that the loads of several
+// pixels are in flight together.
+__device__ __forceinline__ float strip_start(int W, int H, int x, int y, const float *gX, const float *gY,
+                                             const float *u, const float *u0, float &e) {
+    const size_t o = (size_t)y * W + x;
+    const float uc = u[o];
+    const float ul = u[x > 0 ? o - 1 : o], ur = u[x < W - 1 ? o + 1 : o];
+    const float uu = u[y > 0 ? o - W : o], ud = u[y < H - 1 ? o + W : o];
+    const float gxo = x < W - 1 ? __ldg(gX + o) : 0.f, gyo = y < H - 1 ? __ldg(gY + o) : 0.f;
+    const float gxl = x > 0 ? __ldg(gX + o - 1) : 0.f, gyu = y > 0 ? __ldg(gY + o - W) : 0.f;
+    const float dv = u0 ? u0[o] - uc : 0.f;
+    const float ex = ur - uc - gxo, ey = ud - uc - gyo;
+    e = 0.5f * (dv * dv + ex * ex + ey * ey);
+    const float lx = 2.f * uc - ul - ur + gxo - gxl, ly = 2.f * uc - uu - ud + gyo - gyu;
+    return dv - (lx + ly);
 }
 
-__global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(int W, int H, const float *__restrict__ gX,
-                                                                const float *__restrict__ gY, float *__restrict__ U,
-                                                                const float *__restrict__ U0,
-                                                                float *__restrict__ bord, double *__restrict__ partA,
-                                                                double *__restrict__ partB, GridBarrier gb,
-                                                                int max_iter, double gap_tol,
-                                                                double *__restrict__ state,
-                                                                double *__restrict__ trace, int trace_cap) {
-    extern __shared__ __align__(16) float res_smem[];
-    __shared__ double sh[4], s_delta[3], s_dE[3];
-    __shared__ float s_coef[3];
-    __shared__ int s_stop;
-    __shared__ int s_x0[kResMaxTiles], s_y0[kResMaxTiles], s_inner[kResMaxTiles];
-    __shared__ short s_slotD[kResBorder], s_slotR[kResBorder];  // border slot -> index in a d / r plane
-    const size_t N = (size_t)W * H;
-    const int tiles_x = (W + kTileX - 1) / kTileX, tiles_y = (H + kTileY - 1) / kTileY, ntiles = tiles_x * tiles_y;
-    const int nk = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    const int lx = threadIdx.x % kTileX, ly = threadIdx.x / kTileX;
-    const int si = (ly + 1) * kHaloX + lx + 1;  // this thread's pixel in a d plane
-    float *Rs = res_smem;                       // [tile][plane][kResPix]
-    float *Ds = res_smem + (size_t)nk * 3 * kResPix;  // [tile][plane][kResPlane]
-    const float lambda = 1.0f;
-    unsigned int gen = 0;
-    auto tile_of = [&](int k) { return (int)blockIdx.x + k * (int)gridDim.x; };
-    auto border = [&](int set, int t, int c) { return bord + ((size_t)(set * ntiles + t) * 3 + c) * kResBorder; };
-    if ((int)threadIdx.x < nk) {
-        const int t = tile_of(threadIdx.x), x0 = (t % tiles_x) * kTileX, y0 = (t / tiles_x) * kTileY;
-        s_x0[threadIdx.x] = x0;
-        s_y0[threadIdx.x] = y0;
-        // no pixel of an inner tile sits on the image border: its operator needs no one-sided differences
-        s_inner[threadIdx.x] = (x0 > 0 && y0 > 0 && x0 + kTileX < W && y0 + kTileY < H) ? 1 : 0;
-    }
-    if ((int)threadIdx.x < kResBorder) {
-        const int p = threadIdx.x;
-        int px, py;  // tile pixel of border slot p
-        if (p < kTileX) px = p, py = 0;
-        else if (p < 2 * kTileX) px = p - kTileX, py = kTileY - 1;
-        else if (p < 2 * kTileX + kTileY) px = 0, py = p - 2 * kTileX;
-        else px = kTileX - 1, py = p - 2 * kTileX - kTileY;
-        s_slotD[p] = (short)((py + 1) * kHaloX + px + 1);
-        s_slotR[p] = (short)(py * kTileX + px);
+// Sums of nslots slots (slot s: count FP64 values at p + s * stride) into out[s]: warp s, a fixed order. The loads of
+// a lane are in flight together; the tree is only as deep as the lanes that hold values (FP64 latency is on the path
+// of every iteration).
+__device__ __forceinline__ void strip_reduce(const double *p, int count, size_t stride, int nslots, double *out) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (wid < nslots) {
+        const double *q = p + (size_t)wid * stride;
+        double t = 0.0;
+        for (int base = 0; base < count; base += 128) {
+            double v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = base + lane + 32 * j < count ? __ldcg(q + base + lane + 32 * j) : 0.0;
+            if (count > 32) v[0] = (v[0] + v[1]) + (v[2] + v[3]);
+            t = base ? t + v[0] : v[0];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            if (count > o) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) out[wid] = t;
     }
     __syncthreads();
-    // Border values of every own tile, one (tile, plane, slot) item at a time: d from the interior of the
-    // shared d planes (D = true) or r from the r planes, into border set `set`.
-    // (item j = (k * 3 + c) * kResBorder + p lands at border(set, tile k, c)[p], i.e. at
-    // bord + (set * ntiles + blockIdx.x) * 3 kResBorder + j + k (gridDim.x - 1) 3 kResBorder)
-    auto publish = [&](int set, bool D) {
-        float *base = bord + ((size_t)set * ntiles + blockIdx.x) * 3 * kResBorder;
-        const size_t kstep = (size_t)(gridDim.x - 1) * 3 * kResBorder;
-        for (int j = threadIdx.x; j < nk * 3 * kResBorder; j += kResThreads) {
-            const int q = j / kResBorder, p = j - q * kResBorder, k = q / 3;  // q = k * 3 + c
-            const float v = D ? Ds[q * kResPlane + s_slotD[p]] : Rs[q * kResPix + s_slotR[p]];
-            base[j + k * kstep] = v;
-        }
-    };
-    // Halo of every own tile's d planes from the neighbours' borders: border(sa) + b_c border(sb) (sb < 0:
-    // border(sa) alone; 0 outside the image). load_halo issues all of a thread's loads into hv / hi,
-    // store_halo writes them to the planes, so other work can run while the loads are in flight.
-    constexpr int kItems = (kResMaxTiles * 3 * kResBorder + kResThreads - 1) / kResThreads;
-    float hv[kItems];
-    int hi[kItems];
-    auto load_halo = [&](int sa, int sb, float b0, float b1, float b2) {
-#pragma unroll
-        for (int u = 0; u < kItems; ++u) {
-            const int j = (int)threadIdx.x + u * kResThreads;
-            hv[u] = 0.f;
-            hi[u] = -1;
-            if (j < nk * 3 * kResBorder) {
-                const int k = j / (3 * kResBorder), rem = j - k * 3 * kResBorder, c = rem / kResBorder;
-                const int t = tile_of(k);
-                int hs, nt, np;
-                res_halo_slot(rem - c * kResBorder, t, t % tiles_x, t / tiles_x, tiles_x, tiles_y, hs, nt, np);
-                hi[u] = (k * 3 + c) * kResPlane + hs;
-                if (nt >= 0) {
-                    hv[u] = __ldcg(border(sa, nt, c) + np);
-                    if (sb >= 0) hv[u] += (c == 0 ? b0 : (c == 1 ? b1 : b2)) * __ldcg(border(sb, nt, c) + np);
-                }
+}
+
+// probs == nullptr: one problem (`one`) on the whole grid; else block b works on problem block_prob[b]. Every
+// problem has its own barrier words (gb.count + 8 * problem) and its own columns of the partial arrays.
+template <int R>
+__global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem one, const CgProblem *__restrict__ probs,
+                                                               const int *__restrict__ block_prob, double *partA,
+                                                               double *partB, GridBarrier gb, int cluster) {
+    constexpr int NB = strip_border(R);
+    static_assert(R <= 32, "a ghost column is one value per lane");
+    extern __shared__ __align__(16) float strip_mem[];
+    __shared__ double sh[8], s_dE[3], s_den[3], s_ig[3], s_ia[3];
+    __shared__ float s_coef[6], red[kStripWarps][3];
+    __shared__ int s_stop;
+    const int pid = probs ? block_prob[blockIdx.x] : 0;
+    const CgProblem P = probs ? probs[pid] : one;
+    const int W = P.W, H = P.H, lb = (int)blockIdx.x - P.b0, G = (int)gridDim.x;
+    const size_t N = (size_t)W * H;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = warp % 3;
+    const int cols = (W + kStripCols - 1) / kStripCols, rows = (H + R - 1) / R;
+    const int u = lb * kStripUnits + warp / 3;
+    const bool active = u < cols * rows;
+    const int ry = u / cols, cx = u - ry * cols;
+    const int x = cx * kStripCols + 2 * lane, y0 = ry * R;
+    const int nrows = active ? min(R, H - y0) : 0;
+    const bool ina = active && x < W, inb = active && x + 1 < W;
+    const bool top = ry == 0, bottom = y0 + nrows == H;
+    const bool left = cx > 0, right = cx + 1 < cols;  // a unit on that side
+    const bool edgeL = lane == 0, edge = lane == 0 || lane == 31;
+    const bool borderL = x == 0, borderA = x == W - 1, borderB = x + 1 == W - 1;  // image columns 0 and W - 1
+    float *Rw = strip_mem + (size_t)warp * strip_warp_floats(R) + kStripRow + 2;  // row 0, column 0
+    float *Rl = Rw + 2 * lane;                                                   // this lane's pair in row 0
+    float2 *Ss = reinterpret_cast<float2 *>(Rw - 2 + (R + 2) * kStripRow) + lane;
+    float *U = P.U + (size_t)c * N;
+    const float *U0 = P.U0 ? P.U0 + (size_t)c * N : nullptr;
+    GridBarrier bar = gb;
+    bar.count = gb.count + 8 * pid;
+    unsigned int gen = 0;
+    auto border = [&](int set, int unit) { return (set ? P.dB : P.dA) + ((size_t)unit * 3 + c) * NB; };
+    auto pair = [](float *p) -> float2 & { return *reinterpret_cast<float2 *>(p); };
+    float2 X[R], D[R];
+    float2 st = {}, sb = {};     // s on the ghost rows
+    float sl = 0.f, sr = 0.f;    // s on the ghost columns (row = lane)
+    float e = 0.f;
+    // ---- start: r = b - A x on the unit and its ghost ring (outside the image: the border pixel), F(x)
+    if (active) {
+        auto start = [&](int px, int py, float &en) {
+            return strip_start(W, H, min(max(px, 0), W - 1), min(max(py, 0), H - 1), P.gx, P.gy, U, U0, en);
+        };
+        float e0, e1, none;
+        {
+            // the ghost ring
+            const float2 gt = make_float2(start(x, y0 - 1, none), start(x + 1, y0 - 1, none));
+            const float2 gb2 = make_float2(start(x, y0 + nrows, none), start(x + 1, y0 + nrows, none));
+            const float gl = start(cx * kStripCols - 1, y0 + min(lane, nrows - 1), none);
+            const float gr = start((cx + 1) * kStripCols, y0 + min(lane, nrows - 1), none);
+            pair(Rl - kStripRow) = gt;
+            pair(Rl + nrows * kStripRow) = gb2;
+            if (lane < nrows) {
+                Rw[lane * kStripRow - 1] = gl;
+                Rw[lane * kStripRow + kStripCols] = gr;
             }
         }
-    };
-    auto store_halo = [&]() {
-#pragma unroll
-        for (int u = 0; u < kItems; ++u)
-            if (hi[u] >= 0) Ds[hi[u]] = hv[u];
-    };
-    // q = A d at this thread's pixel of plane Dc (inner tiles: the interior formula of box_op, same arithmetic)
-    auto op_at = [&](const float *Dc, bool inner, int x, int y) {
-        if (inner) {
-            const float c = Dc[si];
-            const float lxv = 2.f * c - Dc[si - 1] - Dc[si + 1];
-            const float lyv = 2.f * c - Dc[si - kHaloX] - Dc[si + kHaloX];
-            return lambda * c + lxv + lyv;
+#pragma unroll 4
+        for (int j = 0; j < nrows; ++j) {
+            pair(Rl + j * kStripRow) = make_float2(start(x, y0 + j, e0), start(x + 1, y0 + j, e1));
+            e += (ina ? e0 : 0.f) + (inb ? e1 : 0.f);
+            Ss[j * 32] = make_float2(0.f, 0.f);
         }
-        return box_op<kHaloX>([&](int i) { return Dc[i]; }, si, x, y, W, H, lambda);
-    };
-    // ---- phase 0: r = b - A x and the energy F(x); d_old = 0 (interior and published borders)
-    {
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int k = 0; k < nk; ++k) {
-            const int x = s_x0[k] + lx, y = s_y0[k] + ly;
-            float rv[3] = {0.f, 0.f, 0.f};
-            if (x < W && y < H) cg_start_values(W, H, N, (size_t)y * W + x, x, y, gX, gY, U, U0, lambda, rv, acc);
+        __syncwarp();
+    }
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                Rs[(k * 3 + c) * kResPix + threadIdx.x] = rv[c];
-                Ds[(k * 3 + c) * kResPlane + si] = 0.f;
-            }
+    for (int j = 0; j < R; ++j) {
+        X[j] = D[j] = make_float2(0.f, 0.f);
+        if (j < nrows) {
+            if (ina) X[j].x = __ldcg(U + (size_t)(y0 + j) * W + x);
+            if (inb) X[j].y = __ldcg(U + (size_t)(y0 + j) * W + x + 1);
+        }
+    }
+    // walks the rows: f(j, r of row j, w = A r of row j); the next row is read before f may overwrite row j
+    auto walk = [&](auto f) {
+        float2 up = pair(Rl - kStripRow), cur = pair(Rl), nxt = pair(Rl + kStripRow);
+        float l = Rl[-1], q = Rl[2];
+        float *row = Rl + kStripRow;
+#pragma unroll 4
+        for (int j = 0; j < nrows; ++j, row += kStripRow) {
+            float2 w;
+            w.x = cur.x + (2.f * cur.x - l - cur.y) + (2.f * cur.x - up.x - nxt.x);
+            w.y = cur.y + (2.f * cur.y - cur.x - q) + (2.f * cur.y - up.y - nxt.y);
+            const float2 after = pair(row + kStripRow);
+            l = row[-1];
+            q = row[2];
+            f(j, cur, w);
+            up = cur;
+            cur = nxt;
+            nxt = after;
+        }
+    };
+    // dot products of the current r, w's border into set `set`, block partials into part
+    auto dots = [&](int set, double *part, bool energy) {
+        float g0 = 0.f, g1 = 0.f, d0 = 0.f, d1 = 0.f;
+        float *B = border(set, active ? u : 0);
+        float2 *Brow = reinterpret_cast<float2 *>(B) + lane;
+        float *col = edgeL ? B + 2 * kStripCols : B + 2 * kStripCols + R;
+        if (active)
+            walk([&](int j, float2 v, float2 w) {
+                if (j == 0) Brow[0] = w;
+                if (j == nrows - 1) Brow[32] = w;
+                if (edge) *col = edgeL ? w.x : w.y;
+                ++col;
+                g0 = fmaf(v.x, v.x, g0);
+                g1 = fmaf(v.y, v.y, g1);
+                d0 = fmaf(v.x, w.x, d0);
+                d1 = fmaf(v.y, w.y, d1);
+            });
+        float g = (ina ? g0 : 0.f) + (inb ? g1 : 0.f), d = (ina ? d0 : 0.f) + (inb ? d1 : 0.f), q = energy ? e : 0.f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            g += __shfl_down_sync(0xffffffffu, g, o);
+            d += __shfl_down_sync(0xffffffffu, d, o);
+            if (energy) q += __shfl_down_sync(0xffffffffu, q, o);
+        }
+        if (lane == 0) {
+            red[warp][0] = g;
+            red[warp][1] = d;
+            red[warp][2] = q;
         }
         __syncthreads();
-        publish(0, false);
-        publish(2, true);
-        block_partials_f(acc, 4, partB, gridDim.x);
-    }
-    if (!grid_sync(gb, gen)) return;
-    block_reduce_partials(partB, gridDim.x, 4, sh);
-    if (threadIdx.x < 3) s_delta[threadIdx.x] = sh[threadIdx.x];
-    double E = sh[3];  // thread 0's copy is the one in use
-    float beta[3] = {0.f, 0.f, 0.f};
-    int it = 0;
-    __syncthreads();
-    for (;; ++it) {
-        if (threadIdx.x == 0) {
+        if (threadIdx.x < 6) {
+            const float *v = &red[threadIdx.x % 3][threadIdx.x / 3];
+            static_assert(kStripUnits == 4, "four units per channel");
+            part[(size_t)threadIdx.x * G + blockIdx.x] =
+                ((double)v[0] + (double)v[9]) + ((double)v[18] + (double)v[27]);
+        } else if (threadIdx.x == 6 && energy) {
+            double t = 0.0;
+#pragma unroll
+            for (int k = 0; k < kStripWarps; ++k) t += (double)red[k][2];
+            part[(size_t)6 * G + blockIdx.x] = t;
+        }
+    };
+    auto sync_all = [&]() {
+        if (cluster) {
+            asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+            return true;
+        }
+        if (P.nb == 1) {
+            __syncthreads();
+            return true;
+        }
+        return grid_sync(bar, gen, (unsigned int)P.nb);
+    };
+    dots(0, partA, true);
+    // The FP64 scalars. An FP64 operation has a latency of some dozens of cycles, so the path every warp waits for
+    // holds only beta, the denominator and an FP32 quotient (warp 0, one channel per lane) beside the stop test (warp
+    // 1); the quotients that the next iteration needs (1 / gamma, 1 / alpha, the energy's decrease) follow on nine
+    // lanes of the last warp while the others go on (an FP64 instruction holds the SM's pipe as long for one lane as
+    // for 32).
+    double E = 0.0;  // warp 1's copy is the one in use
+    if (threadIdx.x < 3) s_ig[threadIdx.x] = s_ia[threadIdx.x] = 0.0;
+    for (int it = 0;; ++it) {
+        if (!sync_all()) return;
+        const int set = it & 1;
+        // the neighbours' borders, in flight while the partials are summed
+        float2 wt = {}, wb = {};
+        float wl = 0.f, wr = 0.f;
+        if (active && !top) wt = __ldcg(reinterpret_cast<const float2 *>(border(set, u - cols)) + 32 + lane);
+        if (active && !bottom) wb = __ldcg(reinterpret_cast<const float2 *>(border(set, u + cols)) + lane);
+        if (lane < nrows && left) wl = __ldcg(border(set, u - 1) + 2 * kStripCols + R + lane);
+        if (lane < nrows && right) wr = __ldcg(border(set, u + 1) + 2 * kStripCols + lane);
+        strip_reduce((set ? partB : partA) + P.b0, P.nb, (size_t)G, it == 0 ? kStripSlots : 6, sh);
+        if (threadIdx.x < 3) {
+            const double gam = sh[threadIdx.x], del = sh[3 + threadIdx.x];
+            double beta = gam * s_ig[threadIdx.x], den = fma(-beta, gam * s_ia[threadIdx.x], del);
+            if (!(den > 0.0)) {
+                beta = 0.0;
+                den = del;
+            }
+            const float fd = (float)den;
+            float alpha = 0.f;
+            if (den > 0.0) alpha = fd > 1e-30f && fd < 1e30f ? __fdiv_rn((float)gam, fd) : (float)(gam / den);
+            s_coef[threadIdx.x] = alpha;
+            s_coef[3 + threadIdx.x] = (float)beta;
+            s_den[threadIdx.x] = den;
+        }
+        if (threadIdx.x == 32) {
+            if (it == 0) E = sh[6];
+            else {
+                E = E - s_dE[0] - s_dE[1] - s_dE[2];
+                if (lb == 0 && P.trace && it <= P.trace_cap) P.trace[it - 1] = E;
+            }
             // gap = bound / (E - bound) <= gap_tol, tested without the division
-            const double bound = (s_delta[0] + s_delta[1] + s_delta[2]) / (2.0 * (double)lambda);
-            const double room = E - bound;
-            s_stop = (it >= max_iter || (gap_tol > 0 && room > 0 && bound <= gap_tol * room)) ? 1 : 0;
+            const double bound = 0.5 * (sh[0] + sh[1] + sh[2]), room = E - bound;
+            s_stop = (it >= P.max_iter || (P.gap_tol > 0 && room > 0 && bound <= P.gap_tol * room)) ? 1 : 0;
+            if (s_stop && lb == 0) {
+                P.state[0] = sh[0];
+                P.state[1] = sh[1];
+                P.state[2] = sh[2];
+                P.state[3] = E;
+                P.state[4] = room > 0 ? bound / room : 1e300;
+                P.state[5] = (double)it;
+            }
         }
         __syncthreads();
         if (s_stop) break;
-        const int dold = 1 + ((it + 1) & 1), dnew = 1 + (it & 1);
-        // ---- phase A: d = r + beta d_old (halo from the neighbours' borders, interior in place); publish d's
-        // borders; q = A d and d . q
-        load_halo(0, dold, beta[0], beta[1], beta[2]);
-        for (int k = 0; k < nk; ++k)
+        if (warp == kStripWarps - 1 && lane < 9) {
+            const int k = lane % 3, what = lane / 3;
+            const double gam = sh[k], den = s_den[k];
+            const bool step = gam > 0.0 && den > 0.0;
+            const double q = step ? res_div(what == 0 ? 1.0 : (what == 1 ? den : gam), what == 2 ? den : gam) : 0.0;
+            if (what == 0) s_ig[k] = q;
+            else if (what == 1) s_ia[k] = q;
+            else s_dE[k] = 0.5 * gam * q;
+        }
+        const float alpha = s_coef[c], beta = s_coef[3 + c];
+        // (rows past the unit hold nothing that is read later)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                float *d = Ds + (k * 3 + c) * kResPlane + si;
-                *d = Rs[(k * 3 + c) * kResPix + threadIdx.x] + beta[c] * *d;
+        for (int j = 0; j < R; ++j) {
+            const float2 v = pair(Rl + j * kStripRow);
+            D[j].x = fmaf(beta, D[j].x, v.x);
+            D[j].y = fmaf(beta, D[j].y, v.y);
+            X[j].x = fmaf(alpha, D[j].x, X[j].x);
+            X[j].y = fmaf(alpha, D[j].y, X[j].y);
+        }
+        if (active) {
+            __syncwarp();
+            walk([&](int j, float2 v, float2 w) {
+                float2 q = Ss[j * 32];
+                q.x = fmaf(beta, q.x, w.x);
+                q.y = fmaf(beta, q.y, w.y);
+                Ss[j * 32] = q;
+                float2 n = make_float2(fmaf(-alpha, q.x, v.x), fmaf(-alpha, q.y, v.y));
+                __syncwarp();  // every lane has read row j and its neighbours
+                float *cell = Rl + j * kStripRow;
+                if (borderA) n.y = n.x;
+                if (ina) pair(cell) = n;
+                if (borderL) cell[-1] = n.x;
+                if (borderB) cell[2] = n.y;
+                if (top && j == 0) pair(cell - kStripRow) = n;
+                if (bottom && j == nrows - 1) pair(cell + kStripRow) = n;
+            });
+            auto ghost = [&](float &sv, float &rv, float wv) {
+                sv = fmaf(beta, sv, wv);
+                rv = fmaf(-alpha, sv, rv);
+            };
+            if (!top) {
+                float2 &g = pair(Rl - kStripRow);
+                ghost(st.x, g.x, wt.x);
+                ghost(st.y, g.y, wt.y);
             }
-        store_halo();
-        __syncthreads();
-        publish(dnew, true);
-        float accA[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int k = 0; k < nk; ++k) {
-            const int x = s_x0[k] + lx, y = s_y0[k] + ly;
-            if (x >= W || y >= H) continue;
-            const bool inner = s_inner[k] != 0;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const float *Dc = Ds + (k * 3 + c) * kResPlane;
-                accA[c] += Dc[si] * op_at(Dc, inner, x, y);
+            if (!bottom) {
+                float2 &g = pair(Rl + nrows * kStripRow);
+                ghost(sb.x, g.x, wb.x);
+                ghost(sb.y, g.y, wb.y);
             }
+            if (lane < nrows && left) ghost(sl, Rw[lane * kStripRow - 1], wl);
+            if (lane < nrows && right) ghost(sr, Rw[lane * kStripRow + kStripCols], wr);
+            __syncwarp();
         }
-        block_partials_f(accA, 3, partA, gridDim.x);
-        if (!grid_sync(gb, gen)) return;
-        block_reduce_partials(partA, gridDim.x, 3, sh);
-        // the three step lengths on three threads (the FP64 divisions side by side)
-        if (threadIdx.x < 3) {
-            const int c = threadIdx.x;
-            const double alpha_d = (sh[c] > 0) ? res_div(s_delta[c], sh[c]) : 0.0;
-            s_coef[c] = (float)alpha_d;
-            s_dE[c] = 0.5 * alpha_d * s_delta[c];
-        }
-        __syncthreads();
-        const float alpha[3] = {s_coef[0], s_coef[1], s_coef[2]};
-        if (threadIdx.x == 0) {
-            E = E - s_dE[0] - s_dE[1] - s_dE[2];
-            if (blockIdx.x == 0 && trace && it < trace_cap) trace[it] = E;
-        }
-        // ---- phase B: the halo's d from the neighbours' new borders; u += alpha d, r -= alpha A d, r . r;
-        // publish r's borders
-        load_halo(dnew, -1, 0.f, 0.f, 0.f);
-        store_halo();
-        __syncthreads();
-        float accB[4] = {0.f, 0.f, 0.f, 0.f};
-        // u of the next tile is loaded while the current one is updated
-        auto load_u = [&](int k, float u3[3]) {
-            const int x = s_x0[k] + lx, y = s_y0[k] + ly;
-            const bool in = x < W && y < H;
-            const size_t o = (size_t)y * W + x;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) u3[c] = in ? __ldcg(U + c * N + o) : 0.f;
-        };
-        float ucur[3] = {0.f, 0.f, 0.f};
-        if (nk > 0) load_u(0, ucur);
-        for (int k = 0; k < nk; ++k) {
-            float unext[3] = {0.f, 0.f, 0.f};
-            if (k + 1 < nk) load_u(k + 1, unext);
-            const int x = s_x0[k] + lx, y = s_y0[k] + ly;
-            if (x < W && y < H) {
-                const bool inner = s_inner[k] != 0;
-                const size_t o = (size_t)y * W + x;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float *Dc = Ds + (k * 3 + c) * kResPlane;
-                    float *Rc = Rs + (k * 3 + c) * kResPix + threadIdx.x;
-                    const float qv = op_at(Dc, inner, x, y);
-                    U[c * N + o] = ucur[c] + alpha[c] * Dc[si];
-                    const float rv = *Rc - alpha[c] * qv;
-                    *Rc = rv;
-                    accB[c] += rv * rv;
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < 3; ++c) ucur[c] = unext[c];
-        }
-        __syncthreads();
-        publish(0, false);
-        block_partials_f(accB, 3, partB, gridDim.x);
-        if (!grid_sync(gb, gen)) return;
-        block_reduce_partials(partB, gridDim.x, 3, sh);
-        if (threadIdx.x < 3) {
-            const int c = threadIdx.x;
-            s_coef[c] = (s_delta[c] > 0) ? (float)res_div(sh[c], s_delta[c]) : 0.f;
-            s_delta[c] = sh[c];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < 3; ++c) beta[c] = s_coef[c];
+        dots(set ^ 1, set ? partA : partB, false);
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const double bound = (s_delta[0] + s_delta[1] + s_delta[2]) / (2.0 * (double)lambda);
-        state[0] = s_delta[0];
-        state[1] = s_delta[1];
-        state[2] = s_delta[2];
-        state[3] = E;
-        state[4] = (E - bound) > 0 ? bound / (E - bound) : 1e300;
-        state[5] = (double)it;
-    }
-}
-
-// Batched corrected CG: many targets (CgProblem) in one cooperative launch. Each problem owns the blocks
-// [b0, b0 + nb) (block_prob maps a block to its problem), so its tiles, block partials and FP64 scalars never mix
-// with another problem's; all problems share the grid barriers. A problem that has met its stop rule idles;
-// done[p] (written by the problem's first block at the top of every iteration) tells every block, after the next
-// barrier, whether all problems have stopped, and then the whole grid leaves together. Per problem the
-// arithmetic is k_cg_persistent<false>'s.
-__global__ void __launch_bounds__(kPersistThreads) k_cg_batch(const CgProblem *__restrict__ probs,
-                                                              const int *__restrict__ block_prob, int nprob,
-                                                              double *partA, double *partB, int *done,
-                                                              GridBarrier gb) {
-    __shared__ double sh[8];
-    __shared__ float tile[3][kHaloY][kHaloX];
-    __shared__ float s_coef[3];
-    __shared__ int s_stop, s_all;
-    const int pid = block_prob[blockIdx.x];
-    const CgProblem P = probs[pid];
-    const int W = P.W, H = P.H;
-    const size_t N = (size_t)W * H;
-    const int lb = (int)blockIdx.x - P.b0;  // block index within the problem
-    const int G = (int)gridDim.x;
-    const float lambda = 1.0f;
-    float *U = P.U, *r = P.r;
-    unsigned int gen = 0;
-    // ---- phase 0 (as k_cg_persistent): r = b - A x and F(x)
-    {
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        for (size_t o = (size_t)lb * blockDim.x + threadIdx.x; o < N; o += (size_t)P.nb * blockDim.x) {
-            cg_start_pixel(W, H, N, o, P.gx, P.gy, U, P.U0, r, lambda, acc);
-        }
-        block_partials_f(acc, 4, partB, G);
-    }
-    if (!grid_sync(gb, gen)) return;
-    // the problem's partials sit at [slot * G + b0, slot * G + b0 + nb): one warp per slot sums them in a fixed order
-    auto reduce_own = [&](const double *part, int nslots) { reduce_slots(part + P.b0, P.nb, (size_t)G, nslots, sh); };
-    reduce_own(partB, 4);
-    double delta[3] = {sh[0], sh[1], sh[2]};
-    double E = sh[3];
-    double gap = 1e300;
-    float beta[3] = {0.f, 0.f, 0.f};
-    const float *dold = r;
-    float *dnew = P.dA;
-    int it = 0, stopped_at = -1;
-    const int tiles_x = P.tiles_x, ntiles = P.ntiles;
-    for (;; ++it) {
-        if (threadIdx.x == 0) {
-            if (stopped_at < 0) {
-                const double bound = (delta[0] + delta[1] + delta[2]) / (2.0 * (double)lambda);
-                gap = (E - bound) > 0 ? bound / (E - bound) : 1e300;
-                if (it >= P.max_iter || (P.gap_tol > 0 && gap <= P.gap_tol)) stopped_at = it;
-            }
-            s_stop = stopped_at >= 0 ? 1 : 0;
-            if (lb == 0) done[pid] = s_stop;
-        }
-        __syncthreads();
-        const bool idle = s_stop != 0;
-        // ---- phase A (skipped by a stopped problem)
-        {
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            if (!idle) {
-                for (int t = lb; t < ntiles; t += P.nb) {
-                    const int x0 = (t % tiles_x) * kTileX, y0 = (t / tiles_x) * kTileY;
-                    for (int k = threadIdx.x; k < 3 * kHaloY * kHaloX; k += blockDim.x) {
-                        const int c = k / (kHaloY * kHaloX), rem = k % (kHaloY * kHaloX);
-                        const int gx = x0 - 1 + rem % kHaloX, gy = y0 - 1 + rem / kHaloX;
-                        float v = 0.f;
-                        if (gx >= 0 && gx < W && gy >= 0 && gy < H) {
-                            const size_t o = c * N + (size_t)gy * W + gx;
-                            v = __ldcg(r + o) + beta[c] * __ldcg(dold + o);
-                        }
-                        tile[c][rem / kHaloX][rem % kHaloX] = v;
-                    }
-                    __syncthreads();
-                    for (int p = threadIdx.x; p < kTileX * kTileY; p += blockDim.x) {
-                        const int lx = p % kTileX, ly = p / kTileX, x = x0 + lx, y = y0 + ly;
-                        if (x >= W || y >= H) continue;
-                        const size_t o = (size_t)y * W + x;
 #pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            const float qv = tile_op(tile[c], lx + 1, ly + 1, x, y, W, H, lambda);
-                            const float dcv = tile[c][ly + 1][lx + 1];
-                            dnew[c * N + o] = dcv;
-                            acc[c] += dcv * qv;
-                        }
-                    }
-                    __syncthreads();
-                }
-            }
-            block_partials_f(acc, 3, partA, G);
+    for (int j = 0; j < R; ++j) {
+        if (j < nrows) {
+            if (ina) U[(size_t)(y0 + j) * W + x] = X[j].x;
+            if (inb) U[(size_t)(y0 + j) * W + x + 1] = X[j].y;
         }
-        if (!grid_sync(gb, gen)) return;
-        // every problem wrote done[] before this barrier: leave together once all have stopped
-        if (threadIdx.x == 0) {
-            int all = 1;
-            for (int q = 0; q < nprob; ++q) all &= __ldcg(done + q);
-            s_all = all;
-        }
-        __syncthreads();
-        if (s_all) break;
-        if (!idle) reduce_own(partA, 3);
-        if (threadIdx.x == 0 && !idle) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const double alpha_d = (sh[c] > 0) ? delta[c] / sh[c] : 0.0;
-                s_coef[c] = (float)alpha_d;
-                E -= 0.5 * alpha_d * delta[c];
-            }
-            if (lb == 0 && P.trace && it < P.trace_cap) P.trace[it] = E;
-        }
-        __syncthreads();
-        const float alpha[3] = {s_coef[0], s_coef[1], s_coef[2]};
-        // ---- phase B
-        {
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            if (!idle) {
-                for (int t = lb; t < ntiles; t += P.nb) {
-                    const int x0 = (t % tiles_x) * kTileX, y0 = (t / tiles_x) * kTileY;
-                    for (int k = threadIdx.x; k < 3 * kHaloY * kHaloX; k += blockDim.x) {
-                        const int c = k / (kHaloY * kHaloX), rem = k % (kHaloY * kHaloX);
-                        const int gx = x0 - 1 + rem % kHaloX, gy = y0 - 1 + rem / kHaloX;
-                        tile[c][rem / kHaloX][rem % kHaloX] =
-                            (gx >= 0 && gx < W && gy >= 0 && gy < H) ? __ldcg(dnew + c * N + (size_t)gy * W + gx) : 0.f;
-                    }
-                    __syncthreads();
-                    for (int p = threadIdx.x; p < kTileX * kTileY; p += blockDim.x) {
-                        const int lx = p % kTileX, ly = p / kTileX, x = x0 + lx, y = y0 + ly;
-                        if (x >= W || y >= H) continue;
-                        const size_t o = (size_t)y * W + x;
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            const float qv = tile_op(tile[c], lx + 1, ly + 1, x, y, W, H, lambda);
-                            const float dv = tile[c][ly + 1][lx + 1];
-                            U[c * N + o] = __ldcg(U + c * N + o) + alpha[c] * dv;
-                            const float rv = __ldcg(r + c * N + o) - alpha[c] * qv;
-                            r[c * N + o] = rv;
-                            acc[c] += rv * rv;
-                        }
-                    }
-                    __syncthreads();
-                }
-            }
-            block_partials_f(acc, 3, partB, G);
-        }
-        if (!grid_sync(gb, gen)) return;
-        if (!idle) {
-            reduce_own(partB, 3);
-            if (threadIdx.x == 0) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    s_coef[c] = (delta[c] > 0) ? (float)(sh[c] / delta[c]) : 0.f;
-                    delta[c] = sh[c];
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int c = 0; c < 3; ++c) beta[c] = s_coef[c];
-            dold = dnew;
-            dnew = (dnew == P.dA) ? P.dB : P.dA;
-        }
-    }
-    if (lb == 0 && threadIdx.x == 0) {
-        P.state[0] = delta[0];
-        P.state[1] = delta[1];
-        P.state[2] = delta[2];
-        P.state[3] = E;
-        P.state[4] = gap;
-        P.state[5] = (double)(stopped_at >= 0 ? stopped_at : it);
     }
 }
 
@@ -1675,41 +1576,128 @@ cudaError_t launch_poisson_jacobi(int W, int H, int iters, const float *gx, cons
     return cudaSuccess;
 }
 
+// ------------------------------------------------------------------ strip CG: rule and launch
+static int strip_sms() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+static int strip_blocks(int W, int H, int R) {
+    const int units = ((W + kStripCols - 1) / kStripCols) * ((H + R - 1) / R);
+    return (units + kStripUnits - 1) / kStripUnits;
+}
+
+static constexpr int kStripRows[] = {4, 8, 16, kCgBatchMaxRows};
+
+// Whether the borders of the units fit in dA and in dB (3 N floats each); very thin images do not.
+static bool strip_fits(int W, int H, int R) {
+    return (size_t)((W + kStripCols - 1) / kStripCols) * ((H + R - 1) / R) * 3 * strip_border(R) <= (size_t)3 * W * H;
+}
+
+// Rows per unit for a W x H image on at most `blocks` blocks (one per SM): the smallest R of one cluster while R is
+// at most kStripClusterR, else the smallest R that fits the grid (an iteration's arithmetic is proportional to R,
+// its barrier is not); 0: the image does not fit on chip.
+static int strip_rows(int W, int H, int blocks) {
+    for (int R : kStripRows)
+        if (R <= kStripClusterR && strip_fits(W, H, R) && strip_blocks(W, H, R) <= std::min(kStripClusterBlocks, blocks))
+            return R;
+    for (int R : kStripRows)
+        if (strip_fits(W, H, R) && strip_blocks(W, H, R) <= blocks) return R;
+    return 0;
+}
+
+template <int R>
+static cudaError_t launch_strip_r(int blocks, const CgProblem &one, const CgProblem *probs, const int *block_prob,
+                                  double *partA, double *partB, GridBarrier gb, cudaStream_t st) {
+    const void *kern = (const void *)k_cg_strip<R>;
+    const size_t smem = strip_smem(R);
+    int dev = 0;
+    cudaGetDevice(&dev);
+    // the attributes are per device: set the first time each device launches here
+    static std::mutex mu;
+    static int state[64] = {};  // 1: set, 2: set and one cluster of kStripClusterBlocks can be placed
+    int have = 0;
+    if (dev >= 0 && dev < 64) {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!state[dev]) {
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+            state[dev] = 1;
+            if (R <= kStripClusterR &&
+                cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+                cudaLaunchConfig_t cfg = {};
+                cfg.gridDim = dim3(kStripClusterBlocks);
+                cfg.blockDim = dim3(kStripThreads);
+                cfg.dynamicSmemBytes = smem;
+                cudaLaunchAttribute at[1];
+                at[0].id = cudaLaunchAttributeClusterDimension;
+                at[0].val.clusterDim = {kStripClusterBlocks, 1, 1};
+                cfg.attrs = at;
+                cfg.numAttrs = 1;
+                int n = 0;
+                if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1) state[dev] = 2;
+            }
+            cudaGetLastError();
+        }
+        have = state[dev];
+    }
+    int cluster = (!probs && blocks > 1 && blocks <= kStripClusterBlocks && have == 2) ? 1 : 0;
+    void *args[] = {(void *)&one, (void *)&probs, (void *)&block_prob, &partA, &partB, &gb, &cluster};
+    if (cluster) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(kStripThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim = {(unsigned)blocks, 1, 1};
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelExC(&cfg, kern, args);
+    }
+    return cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kStripThreads), args, smem, st);
+}
+
+static cudaError_t launch_strip(int R, int blocks, const CgProblem &one, const CgProblem *probs, const int *block_prob,
+                                double *partA, double *partB, GridBarrier gb, cudaStream_t st) {
+    switch (R) {
+        case 4: return launch_strip_r<4>(blocks, one, probs, block_prob, partA, partB, gb, st);
+        case 8: return launch_strip_r<8>(blocks, one, probs, block_prob, partA, partB, gb, st);
+        case 16: return launch_strip_r<16>(blocks, one, probs, block_prob, partA, partB, gb, st);
+        case kCgBatchMaxRows: return launch_strip_r<kCgBatchMaxRows>(blocks, one, probs, block_prob, partA, partB, gb, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 cudaError_t launch_cg_persistent(int W, int H, const float *gx, const float *gy, float *U, float *r, float *dA,
                                  float *dB, double *partA, double *partB, GridBarrier gb, int max_iter, double gap_tol,
                                  double *state, cudaStream_t st, LaunchCounter &lc, const float *U0,
                                  double *trace, int trace_cap) {
     ProfScope _ps(lc, "cg_persistent", st);
-    const size_t N = (size_t)W * H;
     const int ntiles = ((W + kTileX - 1) / kTileX) * ((H + kTileY - 1) / kTileY);
-    // shared-memory resident form when every block can hold its tiles (one block per SM) and the tile borders
-    // (3 sets x 3 planes x 160 floats per tile) fit in dA
     {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        // the attribute is per device: set it the first time each device launches here
-        static std::mutex attr_mu;
-        static bool attr_set[64] = {};
-        if (dev >= 0 && dev < 64) {
-            std::lock_guard<std::mutex> lock(attr_mu);
-            if (!attr_set[dev]) {
-                cudaFuncSetAttribute(k_cg_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(kResMaxTiles * kResTileBytes));
-                attr_set[dev] = true;
-            }
-        }
-        const int per = (ntiles + sms - 1) / std::max(sms, 1);
-        const size_t smem = (size_t)per * kResTileBytes;
-        if (per <= kResMaxTiles && (size_t)9 * kResBorder * ntiles <= 3 * N &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_resident, kResThreads, smem) == cudaSuccess &&
-            per_sm >= 1) {
-            const int blocks = (ntiles + per - 1) / per;
-            void *args[] = {&W, &H, (void *)&gx, (void *)&gy, &U, (void *)&U0, &dA, &partA, &partB, &gb,
-                            &max_iter, &gap_tol, &state, &trace, &trace_cap};
+        CgProblem one = {};
+        one.W = W;
+        one.H = H;
+        one.max_iter = max_iter;
+        one.gap_tol = gap_tol;
+        one.gx = gx;
+        one.gy = gy;
+        one.U = U;
+        one.dA = dA;
+        one.dB = dB;
+        one.state = state;
+        one.U0 = U0;
+        one.trace = trace;
+        one.trace_cap = trace_cap;
+        const int R = strip_rows(W, H, strip_sms());
+        if (R > 0) {
+            one.nb = strip_blocks(W, H, R);
             lc.add(1);
-            return cudaLaunchCooperativeKernel((const void *)k_cg_resident, dim3(blocks), dim3(kResThreads), args,
-                                               smem, st);
+            return launch_strip(R, one.nb, one, nullptr, nullptr, partA, partB, gb, st);
         }
     }
     // the TMA form needs row pitches of a multiple of 16 bytes (W % 4 == 0) and the driver's encoder
@@ -1738,14 +1726,29 @@ cudaError_t launch_cg_persistent(int W, int H, const float *gx, const float *gy,
     return cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kPersistThreads), args, smem, st);
 }
 
-int cg_batch_resident_blocks() { return coop_blocks((const void *)k_cg_batch, 1 << 30); }
+int cg_batch_resident_blocks() { return strip_sms(); }
 
-cudaError_t launch_cg_batch(const CgProblem *d_probs, const int *d_block_prob, int nprob, int blocks, double *partA,
-                            double *partB, int *done, GridBarrier gb, cudaStream_t st, LaunchCounter &lc) {
+int cg_batch_blocks(int W, int H, int R) { return strip_fits(W, H, R) ? strip_blocks(W, H, R) : 0; }
+
+// The smallest R whose blocks of all the images fit the GPU together (as strip_rows for one image); 0: none.
+int cg_batch_rows(const CgProblem *probs, int count) {
+    const int sms = strip_sms();
+    for (int R : kStripRows) {
+        long long blocks = 0;
+        for (int i = 0; i < count && blocks <= sms; ++i) {
+            const int b = cg_batch_blocks(probs[i].W, probs[i].H, R);
+            blocks += b > 0 ? b : sms + 1;
+        }
+        if (blocks <= sms) return R;
+    }
+    return 0;
+}
+
+cudaError_t launch_cg_batch(const CgProblem *d_probs, const int *d_block_prob, int R, int blocks, double *partA,
+                            double *partB, GridBarrier gb, cudaStream_t st, LaunchCounter &lc) {
     ProfScope _ps(lc, "cg_batch", st);
-    void *args[] = {(void *)&d_probs, (void *)&d_block_prob, &nprob, &partA, &partB, &done, &gb};
     lc.add(1);
-    return cudaLaunchCooperativeKernel((const void *)k_cg_batch, dim3(blocks), dim3(kPersistThreads), args, 0, st);
+    return launch_strip(R, blocks, CgProblem{}, d_probs, d_block_prob, partA, partB, gb, st);
 }
 
 void *tensor_map_encoder() {
