@@ -12,6 +12,7 @@
 // the footprint weights from tau instead of storing A (the reference stores ks^2 floats per source pixel).
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include <cuda_bf16.h>
 
@@ -490,30 +491,43 @@ __device__ __forceinline__ void gradient_setup_global(int x, int y, int W, int H
 
 // Anchor-row form (KS <= 3). The entries of one anchor bucket reach a KS x KS block of target pixels, so
 // instead of every target pixel re-reading the entries of its KS^2 buckets, a lane reads each entry of its
-// buckets once and accumulates all KS^2 taps in registers (partials P[i][j][field]).
+// buckets once and accumulates its taps in registers.
+// A source pixel's overlaps along one axis are (1 - a, a) for KS 2 and (1 - a, 1, a) for KS 3, so two sums per axis
+// carry all of them: Q0 = sum (1 - a) v, Q1 = sum a v, and the middle tap is Q0 + Q1 (terms of one sign, nothing
+// cancels). Four sums per field instead of KS^2: 28 accumulators and 28 multiply-adds per entry, not 63 and 72.
 // A warp owns 64 consecutive anchors of one anchor row, starting at an even column: lane l takes anchor 2l in
 // pass 0 and anchor 2l + 1 in pass 1, and owns pixel columns 2l and 2l + 1. With dsf 2 most source pixels of a
 // box-decimated view land on even anchors, so one pass per parity makes a warp wait for its longest even bucket
 // plus its longest odd bucket, not twice the longest of both. Pixel x of tap row i sums tap j of anchor x - j:
 //   column 2l:      (P0[0] of 2l + P0[2] of 2l - 2) + P1[1] of 2l - 1
 //   column 2l + 1:   P0[1] of 2l + (P1[0] of 2l + 1 + P1[2] of 2l - 1)
-// (P0 / P1: the pass-0 / pass-1 partials; the left terms come from lane l - 1 by shuffle). The block then adds
+// (P0 / P1: the pass-0 / pass-1 tap sums; the left terms come from lane l - 1 by shuffle). The block then adds
 // the KS tap rows of each pixel from shared memory. Every sum has a fixed order, so results are deterministic.
 // Lane 0's columns lack their left anchors, so a warp outputs 62 pixels. The footprint norm is the product of
-// the row and column overlap sums (the KS^2 taps are an outer product), and a tap is visible when both of its
-// overlaps are non-zero. Fields: 0 w A, 1-3 w A v, 4 A, 5-6 A Sobel, 7 visibility. The mask sum (A w) is
-// field 0: the same products added in the same order.
+// the row and column overlap sums (the KS^2 taps are an outer product). Fields: 0 w A, 1-3 w A v, 4 A, 5-6 A Sobel; a
+// pixel is visible when its sum of A is not 0 (no A is negative). The mask sum (A w) is field 0.
+// RPW: anchor rows per warp; one where two would leave SMs without a block (the rows shared between blocks cost less
+// than that). The gathers in flight live in L1, so shared memory is kept small (with 73 KB a block, three blocks took
+// 2.2 ms where two took 1.0 at 2048^2). Measured, two rows and three blocks per SM: 24 views of 512^2 -> 1024^2 119 ->
+// 80 us, 80 views of 1024^2 -> 2048^2 1278 -> 977 us (3.1 TB/s of compulsory reads); one row and two blocks: 80 BF16
+// views of 384^2, dsf 1, 373 -> 223 us. Bound by the latency of the gathers.
 constexpr int kGrWarps = 8;
 constexpr int kGrTXO = 62;  // output pixels per warp row
-constexpr int kGrNF = 8;    // fields per tap-row partial
+constexpr int kGrNF = 7;    // fields per tap-row partial
 
-template <int KS>
+// Sums a pixel row is kept in until they are added, one per warp that contributes: its tap rows come from KS
+// consecutive anchor rows, so from KS warps at one row each and from two (its own and the one before) at two.
+template <int KS, int RPW>
+__host__ __device__ constexpr int gradient_rows_slots() {
+    return RPW == 1 ? KS : 2;
+}
+template <int KS, int RPW>
 constexpr size_t gradient_rows_smem() {
-    return sizeof(float) * (kGrWarps * 2 - (KS - 1)) * KS * kGrNF * kGrTXO;
+    return sizeof(float) * (kGrWarps * RPW - (KS - 1)) * gradient_rows_slots<KS, RPW>() * kGrNF * kGrTXO;
 }
 
-template <int KS, typename TS>
-__global__ void __launch_bounds__(kGrWarps * 32, 2) k_gradient_setup_rows(int W, int H, int n, int dsf, int BW,
+template <int KS, typename TS, int RPW>
+__global__ void __launch_bounds__(kGrWarps * 32, RPW == 2 ? 3 : 2) k_gradient_setup_rows(int W, int H, int n, int dsf, int BW,
                                                                        const unsigned int *__restrict__ start,
                                                                        const unsigned int *__restrict__ entries,
                                                                        const float *__restrict__ tau,
@@ -524,165 +538,148 @@ __global__ void __launch_bounds__(kGrWarps * 32, 2) k_gradient_setup_rows(int W,
                                                                        float *__restrict__ U, float *__restrict__ gx,
                                                                        float *__restrict__ gy,
                                                                        float *__restrict__ mask) {
-    constexpr int TY = kGrWarps * 2 - (KS - 1);  // output pixel rows per block
-    constexpr int NA = 7;                        // accumulated fields
-    extern __shared__ float gr_part[];           // [TY][KS][kGrNF][kGrTXO]: (pixel row, tap row, field, pixel)
-    pdl_trigger();                               // the hole list, launched next, waits for this grid's completion
+    constexpr int TY = kGrWarps * RPW - (KS - 1);  // output pixel rows per block
+    constexpr int NF = kGrNF, NS = gradient_rows_slots<KS, RPW>();
+    extern __shared__ float gr_part[];  // [TY][NS][NF][kGrTXO]: (pixel row, contributing warp, field, pixel)
+    pdl_trigger();                      // the hole list, launched next, waits for this grid's completion
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int x0 = blockIdx.x * kGrTXO, y0 = blockIdx.y * TY;
     const int BH = H + KS - 1;
     const int lx = 2 * lane - 2;  // this lane's first pixel column inside the tile
-    // warp w takes anchor rows 2w and 2w + 1: one of each parity (with dsf = 2 the populated anchors mostly sit
-    // on even rows, so rows w and w + 8 would leave half the warps idle)
-    for (int q = 0; q < 2; ++q) {
-        const int rr = 2 * warp + q;
+    // warp w takes the consecutive anchor rows RPW w, RPW w + 1, ...: with two, one of each parity (with dsf = 2 the
+    // populated anchors mostly sit on even rows, so rows w and w + 8 would leave half the warps idle)
+#pragma unroll 1
+    for (int q = 0; q < RPW; ++q) {
+        const int rr = RPW * warp + q;
         const int ay = y0 - (KS - 1) + rr, by = ay + KS - 1;
-        bool iny[KS];
-#pragma unroll
-        for (int i = 0; i < KS; ++i) iny[i] = (0 <= ay + i && ay + i <= H - 1);
+        // overlaps of the in-image taps: the first and last tap count when inside, the middle one always is unless
+        // the whole row lies outside
+        const bool y_first = 0 <= ay && ay <= H - 1, y_last = 0 <= ay + KS - 1 && ay + KS - 1 <= H - 1;
+        const float y_mid = (KS == 3 && 0 <= ay + 1 && ay + 1 <= H - 1) ? 1.f : 0.f;
 #pragma unroll 1
         for (int pass = 0; pass < 2; ++pass) {
             const int ax = x0 - 2 + 2 * lane + pass, bx = ax + KS - 1;
-            bool inx[KS];
+            const bool x_first = 0 <= ax && ax <= W - 1, x_last = 0 <= ax + KS - 1 && ax + KS - 1 <= W - 1;
+            const float x_mid = (KS == 3 && 0 <= ax + 1 && ax + 1 <= W - 1) ? 1.f : 0.f;
+            float Q[2][2][NF];
 #pragma unroll
-            for (int j = 0; j < KS; ++j) inx[j] = (0 <= ax + j && ax + j <= W - 1);
-            float P[KS][KS][NA];
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int i = 0; i < KS; ++i)
+                for (int j = 0; j < 2; ++j)
 #pragma unroll
-                for (int j = 0; j < KS; ++j)
-#pragma unroll
-                    for (int f = 0; f < NA; ++f) P[i][j][f] = 0.f;
-            unsigned int anyb = 0;
+                    for (int f = 0; f < NF; ++f) Q[i][j][f] = 0.f;
             if (bx >= 0 && bx < BW && by < BH) {
                 const size_t b = (size_t)by * BW + bx;
                 const unsigned int s = __ldg(start + b), e = __ldg(start + b + 1);
-                // software pipeline: the entry index three ahead and the source data of the next two entries
-                // are in flight while the current entry is accumulated
                 struct Src {
                     float tx, ty, w, c0, c1, c2, s0, s1;
                 };
-                auto fetch = [&](unsigned int ent) {
-                    const int v = (int)(ent >> 24), m = (int)(ent & 0xFFFFFFu);
-                    const TS *iv = img + (size_t)v * 3 * n;
-                    const TS *gv = vgrad + (size_t)v * 2 * n;
-                    Src d;
-                    d.tx = __ldg(tau + (size_t)v * 2 * n + m);
-                    d.ty = __ldg(tau + (size_t)v * 2 * n + n + m);
-                    d.w = ldv(wgt + (size_t)v * n + m);
-                    d.c0 = ldv(iv + m);
-                    d.c1 = ldv(iv + n + m);
-                    d.c2 = ldv(iv + 2 * n + m);
-                    d.s0 = ldv(gv + m);
-                    d.s1 = ldv(gv + n + m);
-                    return d;
+                auto fetch = [&](unsigned int ent, Src &d) {
+                    const size_t vn = (size_t)(ent >> 24) * (size_t)n, m = ent & 0xFFFFFFu;
+                    const float *tv = tau + 2 * vn + m;
+                    const TS *iv = img + 3 * vn + m, *gv = vgrad + 2 * vn + m;
+                    d.tx = __ldg(tv);
+                    d.ty = __ldg(tv + n);
+                    d.w = ldv(wgt + vn + m);
+                    d.c0 = ldv(iv);
+                    d.c1 = ldv(iv + n);
+                    d.c2 = ldv(iv + 2 * (size_t)n);
+                    d.s0 = ldv(gv);
+                    d.s1 = ldv(gv + n);
                 };
-                Src cur = {}, nx1 = {};
-                unsigned int ent_next = 0;
-                if (s < e) cur = fetch(__ldg(entries + s));
-                if (s + 1 < e) nx1 = fetch(__ldg(entries + s + 1));
-                if (s + 2 < e) ent_next = __ldg(entries + s + 2);
-                for (unsigned int k = s; k < e; ++k) {
-                    Src nx2 = {};
-                    if (k + 2 < e) nx2 = fetch(ent_next);
-                    if (k + 3 < e) ent_next = __ldg(entries + k + 3);
-                    const float w = cur.w, c0 = cur.c0, c1 = cur.c1, c2 = cur.c2, s0 = cur.s0, s1 = cur.s1;
-                    const float px = cur.tx - 0.5f, py = cur.ty - 0.5f;
-                    cur = nx1;
-                    nx1 = nx2;
-                    float dx[KS], dy[KS], sx = 0.f, sy = 0.f;
-                    unsigned int xb = 0;
-#pragma unroll
-                    for (int t = 0; t < KS; ++t) {
-                        dx[t] = inx[t] ? fp_overlap(t, KS, ax + t, px, dsf) : 0.0f;
-                        dy[t] = iny[t] ? fp_overlap(t, KS, ay + t, py, dsf) : 0.0f;
-                        sx = __fadd_rn(sx, dx[t]);
-                        sy = __fadd_rn(sy, dy[t]);
-                        xb |= (dx[t] != 0.0f) ? 1u << t : 0u;
-                    }
+                auto add = [&](const Src &d) {
+                    const float px = d.tx - 0.5f, py = d.ty - 0.5f;
+                    const float dx[2] = {fp_overlap(0, KS, ax, px, dsf), fp_overlap(KS - 1, KS, ax + KS - 1, px, dsf)};
+                    const float dy[2] = {fp_overlap(0, KS, ay, py, dsf), fp_overlap(KS - 1, KS, ay + KS - 1, py, dsf)};
+                    const float sx = (x_first ? dx[0] : 0.f) + x_mid + (x_last ? dx[1] : 0.f);
+                    const float sy = (y_first ? dy[0] : 0.f) + y_mid + (y_last ? dy[1] : 0.f);
                     // one reciprocal per entry; A = (dx * (1 / norm)) * dy is within a few ulps of dx dy / norm
                     const float norm = __fmul_rn(sx, sy);
                     const float inv = (norm != 0.0f) ? __frcp_rn(norm) : 1.0f;
-                    const float w0 = w * c0, w1 = w * c1, w2 = w * c2;
+                    const float v[NF] = {d.w, d.w * d.c0, d.w * d.c1, d.w * d.c2, 1.f, d.s0, d.s1};
 #pragma unroll
-                    for (int i = 0; i < KS; ++i) {
-                        anyb |= (dy[i] != 0.0f) ? xb << (i * KS) : 0u;
+                    for (int i = 0; i < 2; ++i) {
                         const float yi = __fmul_rn(dy[i], inv);
 #pragma unroll
-                        for (int j = 0; j < KS; ++j) {
+                        for (int j = 0; j < 2; ++j) {
                             const float A = __fmul_rn(dx[j], yi);
-                            P[i][j][0] += w * A;
-                            P[i][j][1] += A * w0;
-                            P[i][j][2] += A * w1;
-                            P[i][j][3] += A * w2;
-                            P[i][j][4] += A;
-                            P[i][j][5] += A * s0;
-                            P[i][j][6] += A * s1;
+#pragma unroll
+                            for (int f = 0; f < NF; ++f) Q[i][j][f] = f == 4 ? Q[i][j][f] + A : fmaf(A, v[f], Q[i][j][f]);
                         }
                     }
+                };
+                // two entries in flight while two are added, and the indices of the two after those
+                Src a = {}, c = {};
+                unsigned int ea = 0, ec = 0;
+                if (s < e) fetch(__ldg(entries + s), a);
+                if (s + 1 < e) fetch(__ldg(entries + s + 1), c);
+                if (s + 2 < e) ea = __ldg(entries + s + 2);
+                if (s + 3 < e) ec = __ldg(entries + s + 3);
+                for (unsigned int k = s; k < e; k += 2) {
+                    add(a);
+                    if (k + 2 < e) fetch(ea, a);
+                    if (k + 4 < e) ea = __ldg(entries + k + 4);
+                    if (k + 1 < e) add(c);
+                    if (k + 3 < e) fetch(ec, c);
+                    if (k + 5 < e) ec = __ldg(entries + k + 5);
                 }
             }
-            // tap rows of this pass into shared memory: pass 0 stores, pass 1 adds (same lane, same slots)
+            // tap rows of this pass into shared memory: the warp's first contribution to a slot stores, the others add
+            // (same lane, same slots)
 #pragma unroll
             for (int i = 0; i < KS; ++i) {
                 const int py = ay + i - y0;  // output pixel row inside the tile
-                float c0[NA], c1[NA];
-                unsigned int v0, v1;
-                const unsigned int bi = anyb >> (i * KS);
-                const unsigned int bl = __shfl_up_sync(0xffffffffu, bi, 1);
-                if (pass == 0) {
+                const bool store = lane >= 1 && py >= 0 && py < TY;
+                const bool first = pass == 0 && (RPW == 1 || q == 0 || i == KS - 1);
+                float *row = gr_part + (size_t)(py * NS + (q + i) / RPW) * NF * kGrTXO + lx;
 #pragma unroll
-                    for (int f = 0; f < NA; ++f) {
-                        const float left = (KS == 3) ? __shfl_up_sync(0xffffffffu, P[i][KS - 1][f], 1) : 0.0f;
-                        c0[f] = (KS == 3) ? P[i][0][f] + left : P[i][0][f];
-                        c1[f] = P[i][1][f];
-                    }
-                    v0 = (bi & 1u) | ((KS == 3) ? (bl >> 2) & 1u : 0u);
-                    v1 = (bi >> 1) & 1u;
-                } else {
-#pragma unroll
-                    for (int f = 0; f < NA; ++f) {
-                        c0[f] = __shfl_up_sync(0xffffffffu, P[i][1][f], 1);
-                        const float left = (KS == 3) ? __shfl_up_sync(0xffffffffu, P[i][KS - 1][f], 1) : 0.0f;
-                        c1[f] = (KS == 3) ? P[i][0][f] + left : P[i][0][f];
-                    }
-                    v0 = (bl >> 1) & 1u;
-                    v1 = (bi & 1u) | ((KS == 3) ? (bl >> 2) & 1u : 0u);
-                }
-                if (lane >= 1 && py >= 0 && py < TY) {
-                    float *row = gr_part + (size_t)(py * KS + i) * kGrNF * kGrTXO + lx;
-#pragma unroll
-                    for (int f = 0; f < NA; ++f) {
-                        float2 *d = reinterpret_cast<float2 *>(row + f * kGrTXO);
+                for (int f = 0; f < NF; ++f) {
+                    // taps 0 and KS - 1 of tap row i
+                    const float t0 = i == 0 ? Q[0][0][f] : (i == KS - 1 ? Q[1][0][f] : Q[0][0][f] + Q[1][0][f]);
+                    const float t1 = i == 0 ? Q[0][1][f] : (i == KS - 1 ? Q[1][1][f] : Q[0][1][f] + Q[1][1][f]);
+                    float c0, c1;
+                    const float last = __shfl_up_sync(0xffffffffu, t1, 1);  // the last tap of lane l - 1
+                    if (KS == 3) {
+                        const float mid = t0 + t1;
                         if (pass == 0) {
-                            *d = make_float2(c0[f], c1[f]);
+                            c0 = t0 + last;
+                            c1 = mid;
+                        } else {
+                            c0 = __shfl_up_sync(0xffffffffu, mid, 1);
+                            c1 = t0 + last;
+                        }
+                    } else if (pass == 0) {
+                        c0 = t0;
+                        c1 = t1;
+                    } else {
+                        c0 = last;
+                        c1 = t0;
+                    }
+                    if (store) {
+                        float2 *d = reinterpret_cast<float2 *>(row + f * kGrTXO);
+                        if (first) {
+                            *d = make_float2(c0, c1);
                         } else {
                             const float2 o = *d;
-                            *d = make_float2(o.x + c0[f], o.y + c1[f]);
+                            *d = make_float2(o.x + c0, o.y + c1);
                         }
-                    }
-                    float2 *dv = reinterpret_cast<float2 *>(row + NA * kGrTXO);
-                    if (pass == 0) {
-                        *dv = make_float2(v0 ? 1.f : 0.f, v1 ? 1.f : 0.f);
-                    } else {
-                        const float2 o = *dv;
-                        *dv = make_float2((o.x != 0.f || v0) ? 1.f : 0.f, (o.y != 0.f || v1) ? 1.f : 0.f);
                     }
                 }
             }
         }
     }
     __syncthreads();
-    // add the tap rows of every pixel in order and normalise (as SetupAcc::store)
+    // add the slots of every pixel in order and normalise (as SetupAcc::store)
     const size_t N = (size_t)W * H;
     for (int p = threadIdx.x; p < TY * kGrTXO; p += kGrWarps * 32) {
         const int px = p % kGrTXO, ly = p / kGrTXO, x = x0 + px, y = y0 + ly;
         if (x >= W || y >= H) continue;
         SetupAcc acc;
-        float any = 0.f;
 #pragma unroll
-        for (int i = 0; i < KS; ++i) {
-            const float *c = gr_part + (size_t)(ly * KS + i) * kGrNF * kGrTXO + px;
+        for (int i = 0; i < NS; ++i) {
+            // (KS 2, two rows per warp: a warp's second row gets both tap rows from that warp)
+            if (KS == 2 && RPW == 2 && i == 1 && ((ly + 1) & 1)) continue;
+            const float *c = gr_part + (size_t)(ly * NS + i) * NF * kGrTXO + px;
             acc.wn += c[0 * kGrTXO];
             acc.u0 += c[1 * kGrTXO];
             acc.u1 += c[2 * kGrTXO];
@@ -690,10 +687,9 @@ __global__ void __launch_bounds__(kGrWarps * 32, 2) k_gradient_setup_rows(int W,
             acc.nrm += c[4 * kGrTXO];
             acc.g0 += c[5 * kGrTXO];
             acc.g1 += c[6 * kGrTXO];
-            any += c[7 * kGrTXO];
         }
         acc.g2 = acc.wn;
-        acc.any = any != 0.f;
+        acc.any = acc.nrm != 0.f;
         acc.store((size_t)y * W + x, N, s2, vis, U, gx, gy, mask);
     }
 }
@@ -1600,15 +1596,27 @@ static void gradient_setup_ks(const Geometry &G, const Buckets &B, const float *
                               const TS *vgrad, const TS *wgt, float s2, uint8_t *vis, float *U, float *gx,
                               float *gy, float *mask, cudaStream_t st) {
     if constexpr (KS <= 3) {
-        constexpr int TY = kGrWarps * 2 - (KS - 1);
-        constexpr size_t smem = gradient_rows_smem<KS>();
-        static std::once_flag once;
-        std::call_once(once, [] {
-            cudaFuncSetAttribute(k_gradient_setup_rows<KS, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        });
-        const dim3 g((G.W + kGrTXO - 1) / kGrTXO, (G.H + TY - 1) / TY);
-        k_gradient_setup_rows<KS, TS><<<g, kGrWarps * 32, smem, st>>>(G.W, G.H, G.n, G.dsf, B.BW, B.start, B.entries,
-                                                                    tau, img, vgrad, wgt, s2, vis, U, gx, gy, mask);
+        // two anchor rows per warp unless that gives the GPU fewer than two blocks per SM
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        auto launch = [&](auto rpw) {
+            constexpr int RPW = decltype(rpw)::value, TY = kGrWarps * RPW - (KS - 1);
+            constexpr size_t smem = gradient_rows_smem<KS, RPW>();
+            static std::once_flag once;
+            std::call_once(once, [] {
+                cudaFuncSetAttribute(k_gradient_setup_rows<KS, TS, RPW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem);
+            });
+            const dim3 g((G.W + kGrTXO - 1) / kGrTXO, (G.H + TY - 1) / TY);
+            k_gradient_setup_rows<KS, TS, RPW><<<g, kGrWarps * 32, smem, st>>>(
+                G.W, G.H, G.n, G.dsf, B.BW, B.start, B.entries, tau, img, vgrad, wgt, s2, vis, U, gx, gy, mask);
+        };
+        constexpr int TY2 = kGrWarps * 2 - (KS - 1);
+        if ((long long)((G.W + kGrTXO - 1) / kGrTXO) * ((G.H + TY2 - 1) / TY2) >= 2 * sms)
+            launch(std::integral_constant<int, 2>{});
+        else
+            launch(std::integral_constant<int, 1>{});
     } else {
         k_gradient_setup_px<KS, TS><<<grid2(G.W, G.H, kTile), kTile, 0, st>>>(G.W, G.H, G.n, G.dsf, B.BW, B.start,
                                                                             B.entries, tau, img, vgrad, wgt, s2, vis,
