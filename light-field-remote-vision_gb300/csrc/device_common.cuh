@@ -187,11 +187,11 @@ __device__ __forceinline__ void pixel_of(int m, int w, int n, float rw, int &x, 
 
 // Inverse-map bucket of a source pixel with warp (tx, ty): its footprint anchor offset by ks - 1 on a grid of
 // BW columns (-1: the pixel is not splatted).
-__device__ __forceinline__ long long bucket_of(float tx, float ty, int W, int H, int dsf, int BW) {
+__device__ __forceinline__ int bucket_of(float tx, float ty, int W, int H, int dsf, int BW) {
     if (!in_splat(tx, ty, W, H)) return -1;
     const int ks = dsf + 1;
     const int x0 = fp_anchor(tx - 0.5f, dsf), y0 = fp_anchor(ty - 0.5f, dsf);
-    return (long long)(y0 + ks - 1) * BW + (x0 + ks - 1);
+    return (y0 + ks - 1) * BW + (x0 + ks - 1);  // targets have fewer than 2^29 pixels
 }
 
 // Luminance of the Sobel kernels (vtv_sr_kernels_unstructured.cu:121-130).
