@@ -1100,165 +1100,179 @@ __global__ void k_sobel(int W, int H, const float *__restrict__ rgb, size_t in_s
     }
 }
 
-// Reprojection of the 6 dual components onto the Frobenius ball of radius r (vtv_rof.cu:280-320).
-__device__ __forceinline__ void rof_project(float p[6], float r) {
-    float nn = 0.f;
-    nn += p[0] * p[0] + p[2] * p[2] + p[4] * p[4];
-    nn += p[1] * p[1] + p[3] * p[3] + p[5] * p[5];
-    nn = sqrtf(nn);
-    if (nn > r) {
-        const float s = r / nn;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) p[k] *= s;
-    }
+// Inner ROF iterations, temporally blocked. One iteration is the dual step p += sigma grad_fwd(U) (vtv_rof.cu:118-147),
+// the reprojection of the 6 duals onto the ball of radius g (vtv_rof.cu:280-320) and the primal prox
+// U = (tau F + lambda (U + tau div_bwd p)) / (tau + lambda) (cuda_kernels.cu:504-532). All niter of them run in one
+// cooperative launch: each super-step runs up to K iterations on a (kRofTX + 2 K) x (TY + 2 K) region around a
+// kRofTX x TY tile and writes back the tile, whose values depend only on the region (the halo absorbs one pixel of
+// staleness per iteration from each side). Super-steps read one global (U, P) pair and write the other, with a bounded
+// grid barrier between them; a block with one tile keeps it in registers and reads back only the halo.
+//
+// A thread owns V vertically adjacent pixels: their U, p, tau F and g stay in registers, the neighbours above and
+// below come from registers too except at the ends, and shared memory carries U and the x duals (which the left and
+// right neighbours read) and the y duals of each thread's last pixel. The code of a pixel has no branch for the image:
+//   - a dual whose forward difference does not exist (the last column / row, pixels outside the image) has step 0 in
+//     its direction and starts at 0, so it stays 0, which is what the divergence of the first column / row subtracts;
+//   - what other pixels outside the image hold is finite and read only through a step of 0.
+// Threads whose pixels the tile no longer depends on skip the iteration; what the rest computes beyond that is stale
+// and stays outside the tile.
+// The projection scales by g / |p| only beyond the ball, as g times a reciprocal square root with one Newton step; the
+// prox divides by tau + lambda as a reciprocal product with its remainder corrected.
+//
+// Bound by the chain of an iteration (two block barriers, shared-memory loads, the projection) and by the super-steps'
+// grid barriers, about 3 us each (waiting for the eight neighbouring blocks alone, with a flag each, took longer). 256^2,
+// 300 iterations (K = 8, TY = 16, V = 2, 128 blocks): 524 -> 345 us against the form before it with two scattered
+// pixels per thread, border branches, and IEEE square roots and divisions; V = 4 saves instructions but leaves half the
+// warps (398). K, TY and V are picked per image size by the host's autotuner; all give the same values.
+constexpr int kRofTX = 32;
+template <int K, int TY, int V>
+__host__ __device__ constexpr int rof_threads() {
+    return ((kRofTX + 2 * K) * ((TY + 2 * K) / V) + 31) / 32 * 32;
 }
-
-// All niter inner ROF iterations in one cooperative launch, temporally blocked. One iteration is the dual step
-// p += sigma grad_fwd(U) (vtv_rof.cu:118-147), the reprojection of the 6 duals onto the ball of radius g
-// (vtv_rof.cu:280-320) and the primal prox U = (tau F + lambda (U + tau div_bwd p)) / (tau + lambda)
-// (cuda_kernels.cu:504-532). Each super-step runs up to kRofK iterations on a (kRofTX + 2 kRofK) x
-// (kRofTY + 2 kRofK) region around a kRofTX x kRofTY tile and writes back the tile, whose values depend only on the
-// region (the halo absorbs one pixel of staleness per iteration from each side). Super-steps read one global
-// (U, P) pair and write the other, with a bounded grid barrier between them.
-// Every thread owns the same PPT region pixels in every iteration (their coordinates and border flags are worked
-// out once per tile): their U, P, F and g stay in registers, and shared memory carries only what the neighbours
-// read, U (right and lower neighbours, in the dual step) and the x and y duals (left and upper neighbours, in the
-// prox). The block sizes divide the region into equal shares, so no warp waits at the block barriers for a
-// second pass of the others. K (iterations per super-step) and the block size are template parameters; the
-// host picks an instantiation per image size with a timing autotuner (rof_autotune).
-constexpr int kRofTX = 32, kRofTY = 16;
-template <int K>
+// U and the x duals (3 planes each, one row more than the region and a cell on either side), the segments' last y duals
+template <int K, int TY, int V>
+__host__ __device__ constexpr int rof_plane() {
+    return (kRofTX + 2 * K) * (TY + 2 * K + 1) + 2;
+}
+template <int K, int TY, int V>
+__host__ __device__ constexpr int rof_plane_y() {
+    return (kRofTX + 2 * K) * ((TY + 2 * K) / V + 1);
+}
+template <int K, int TY, int V>
 constexpr size_t rof_smem() {
-    return (size_t)9 * (kRofTX + 2 * K) * (kRofTY + 2 * K) * sizeof(float);  // U 3, x duals 3, y duals 3
+    return sizeof(float) * (size_t)(6 * rof_plane<K, TY, V>() + 3 * rof_plane_y<K, TY, V>());
 }
 
-template <int kRofK, int kRofThreads>
-__global__ void __launch_bounds__(kRofThreads) k_rof_persistent(int W, int H, int niter, float tau, float sigma,
-                                                                float lam, float *U0, float *P0, float *U1,
-                                                                float *P1, const float *__restrict__ F,
-                                                                const float *__restrict__ g, GridBarrier gb) {
-    constexpr int RX = kRofTX + 2 * kRofK, RY = kRofTY + 2 * kRofK, RN = RX * RY;
-    constexpr int PPT = (RN + kRofThreads - 1) / kRofThreads;  // region pixels per thread
+template <int K, int TY, int V>
+__global__ void __launch_bounds__((rof_threads<K, TY, V>())) k_rof_persistent(int W, int H, int niter, float tau,
+                                                                           float sigma, float lam, float *U0,
+                                                                           float *P0, float *U1, float *P1,
+                                                                           const float *__restrict__ F,
+                                                                           const float *__restrict__ g, GridBarrier gb) {
+    constexpr int RX = kRofTX + 2 * K, RY = TY + 2 * K;
+    static_assert(RY % V == 0, "whole segments");
+    constexpr int PL = rof_plane<K, TY, V>(), PY = rof_plane_y<K, TY, V>();
     extern __shared__ float sm[];
-    float *sU = sm, *sPx = sm + 3 * RN, *sPy = sm + 6 * RN;
-    const int tiles_x = (W + kRofTX - 1) / kRofTX, ntiles = tiles_x * ((H + kRofTY - 1) / kRofTY);
+    const int seg = threadIdx.x / RX, lx = threadIdx.x - seg * RX, ly0 = seg * V;
+    const bool mine = seg < RY / V;
+    float *sU = sm + 1 + ly0 * RX + lx, *sPx = sU + 3 * PL;         // this thread's first pixel, plane 0
+    float *sPy = sm + 6 * PL + (seg + 1) * RX + lx;                 // its last pixel's y dual; - RX: the segment above
+    const int tiles_x = (W + kRofTX - 1) / kRofTX, ntiles = tiles_x * ((H + TY - 1) / TY);
+    const bool resident = ntiles <= (int)gridDim.x;  // one tile per block
     const size_t N = (size_t)W * H;
-    const float denom = tau + lam;
-    // flags of an owned pixel: inside the image, its forward differences exist (x, y), its left / upper
-    // neighbour's dual enters the divergence (inside the image and the region), and it is a tile pixel
-    constexpr unsigned kIn = 1, kFx = 2, kFy = 4, kBx = 8, kBy = 16, kTile = 32, kRx = 64, kRy = 128;
-    constexpr int kDistShift = 8;
+    const float denom = tau + lam, rden = __frcp_rn(denom);
+    // distance of the segment's column and of its nearest row from the tile
+    const int dx = max(max(K - lx, lx - (K + kRofTX - 1)), 0);
+    const int dist = max(dx, max(max(K - (ly0 + V - 1), ly0 - (K + TY - 1)), 0));
+    const bool tile_x = mine && lx >= K && lx < K + kRofTX;
     unsigned int gen = 0;
     int step = 0;
-    for (int done = 0; done < niter; done += kRofK, ++step) {
-        const int iters = min(kRofK, niter - done);
+    // shared memory that no thread writes (pads) is read too: finite from here on
+    for (int i = threadIdx.x; i < 6 * PL + 3 * PY; i += blockDim.x) sm[i] = 0.f;
+    __syncthreads();
+    float u[V][3], p[V][6], tf[V][3], r[V], sy[V], sx = 0.f;
+    for (int done = 0; done < niter; done += K, ++step) {
+        const int iters = min(K, niter - done);
         const float *Ui = (step & 1) ? U1 : U0, *Pi = (step & 1) ? P1 : P0;
         float *Uo = (step & 1) ? U0 : U1, *Po = (step & 1) ? P0 : P1;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-            const int rx0 = (t % tiles_x) * kRofTX - kRofK, ry0 = (t / tiles_x) * kRofTY - kRofK;
-            float u[PPT][3], p[PPT][6], f[PPT][3], gg[PPT];
-            unsigned int fl[PPT];
-            size_t go[PPT];
+            const int gx = (t % tiles_x) * kRofTX - K + lx, gy0 = (t / tiles_x) * TY - K + ly0;
+            const bool inx = mine && gx >= 0 && gx < W;
+            sx = inx && gx < W - 1 ? sigma : 0.f;
 #pragma unroll
-            for (int k = 0; k < PPT; ++k) {
-                const int i = threadIdx.x + k * kRofThreads;
-                const int lx = i % RX, ly = i / RX, gx = rx0 + lx, gy = ry0 + ly;
-                const bool in = i < RN && gx >= 0 && gx < W && gy >= 0 && gy < H;
-                unsigned int f0 = 0;
-                if (in) {
-                    f0 |= kIn;
-                    if (gx < W - 1) f0 |= kFx;
-                    if (gy < H - 1) f0 |= kFy;
-                    if (gx > 0) f0 |= kBx;
-                    if (gy > 0) f0 |= kBy;
-                    if (lx + 1 < RX) f0 |= kRx;
-                    if (ly + 1 < RY) f0 |= kRy;
-                    if (lx >= kRofK && lx < kRofK + kRofTX && ly >= kRofK && ly < kRofK + kRofTY) f0 |= kTile;
-                    // distance from the tile (Chebyshev, in pixels)
-                    const int dx = max(max(kRofK - lx, lx - (kRofK + kRofTX - 1)), 0);
-                    const int dy = max(max(kRofK - ly, ly - (kRofK + kRofTY - 1)), 0);
-                    f0 |= (unsigned int)max(dx, dy) << kDistShift;
-                }
-                fl[k] = f0;
+            for (int k = 0; k < V; ++k) {
+                const int gy = gy0 + k;
+                const bool in = inx && gy >= 0 && gy < H;
+                const bool own = tile_x && ly0 + k >= K && ly0 + k < K + TY;
                 const size_t o = in ? (size_t)gy * W + gx : 0;
-                go[k] = o;
+                sy[k] = gy >= 0 && gy < H - 1 ? sigma : 0.f;
+                if (step == 0 || !resident) {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    u[k][c] = in ? __ldcg(Ui + c * N + o) : 0.f;
-                    f[k][c] = in ? __ldg(F + c * N + o) : 0.f;
+                    for (int c = 0; c < 3; ++c) tf[k][c] = in ? tau * __ldg(F + c * N + o) : 0.f;
+                    r[k] = in ? __ldg(g + o) : 0.f;
                 }
+                if (step == 0 || !resident || !own) {
 #pragma unroll
-                for (int c = 0; c < 6; ++c) p[k][c] = in ? __ldcg(Pi + c * N + o) : 0.f;
-                gg[k] = in ? __ldg(g + o) : 0.f;
-                if (i < RN) {
+                    for (int c = 0; c < 3; ++c) u[k][c] = in ? __ldcg(Ui + c * N + o) : 0.f;
+#pragma unroll
+                    for (int c = 0; c < 6; ++c) p[k][c] = in ? __ldcg(Pi + c * N + o) : 0.f;
+                }
+                if (mine) {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        sU[c * RN + i] = u[k][c];
-                        sPx[c * RN + i] = p[k][2 * c];
-                        sPy[c * RN + i] = p[k][2 * c + 1];
+                        sU[c * PL + k * RX] = u[k][c];
+                        sPx[c * PL + k * RX] = p[k][2 * c];
                     }
                 }
+            }
+            if (mine) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) sPy[c * PY] = p[V - 1][2 * c + 1];
             }
             __syncthreads();
             for (int it = 0; it < iters; ++it) {
-                // Only the pixels the tile still depends on are updated: after iteration it the tile needs U within
-                // distance iters - it - 1 of it (the prox), and that prox reads the duals one pixel further out
-                // (the dual step, whose right and lower neighbours' U were updated in the iteration before).
-                // dual step + reprojection: the pixel's own U and p, its right and lower neighbours' U
-                const unsigned int dual_reach = (unsigned int)(iters - it) << kDistShift;
-                const unsigned int prox_reach = (unsigned int)(iters - it - 1) << kDistShift;
+                // after iteration it the tile needs U within distance iters - it - 1 of it, and that prox reads the
+                // duals one pixel further out
+                if (mine && dist <= iters - it) {
+                    float below[3];
 #pragma unroll
-                for (int k = 0; k < PPT; ++k) {
-                    if (!(fl[k] & kIn) || (fl[k] & ~0xFFu) > dual_reach) continue;
-                    const int i = threadIdx.x + k * kRofThreads;
+                    for (int c = 0; c < 3; ++c) below[c] = sU[c * PL + V * RX];
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const float *su = sU + c * RN;
-                        const float uc = u[k][c];
-                        const float ur = (fl[k] & kRx) ? su[i + 1] : 0.f, ud = (fl[k] & kRy) ? su[i + RX] : 0.f;
-                        const float gxv = (fl[k] & kFx) ? ur - uc : 0.f;
-                        const float gyv = (fl[k] & kFy) ? ud - uc : 0.f;
-                        p[k][2 * c] = p[k][2 * c] + sigma * gxv;
-                        p[k][2 * c + 1] = p[k][2 * c + 1] + sigma * gyv;
+                    for (int k = 0; k < V; ++k) {
+                        float n2 = 0.f;
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            const float uc = u[k][c];
+                            const float ur = sU[c * PL + k * RX + 1], ud = k + 1 < V ? u[k + 1 < V ? k + 1 : k][c] : below[c];
+                            const float a = fmaf(sx, ur - uc, p[k][2 * c]), b = fmaf(sy[k], ud - uc, p[k][2 * c + 1]);
+                            p[k][2 * c] = a;
+                            p[k][2 * c + 1] = b;
+                            n2 = fmaf(b, b, fmaf(a, a, n2));
+                        }
+                        // beyond the ball: p *= g / |p| (a negative radius scales always, as |p| > g does)
+                        const float r2 = r[k] < 0.f ? -1.f : r[k] * r[k];
+                        if (n2 > r2) {
+                            const float e = rsqrtf(n2);
+                            const float q = r[k] * fmaf(e * 0.5f, fmaf(-n2 * e, e, 1.f), e);
+#pragma unroll
+                            for (int c = 0; c < 6; ++c) p[k][c] *= q;
+                        }
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) sPx[c * PL + k * RX] = p[k][2 * c];
                     }
-                    rof_project(p[k], gg[k]);
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        sPx[c * RN + i] = p[k][2 * c];
-                        sPy[c * RN + i] = p[k][2 * c + 1];
-                    }
+                    for (int c = 0; c < 3; ++c) sPy[c * PY] = p[V - 1][2 * c + 1];
                 }
                 __syncthreads();
-                // primal prox: the pixel's new duals and its left / upper neighbours'
-#pragma unroll
-                for (int k = 0; k < PPT; ++k) {
-                    if (!(fl[k] & kIn) || (fl[k] & ~0xFFu) > prox_reach) continue;
-                    const int i = threadIdx.x + k * kRofThreads;
-                    const int lx = i % RX, ly = i / RX;
+                if (mine && dist <= iters - it - 1) {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        float st = p[k][2 * c] + p[k][2 * c + 1];
-                        if (fl[k] & kBx) st -= (lx > 0) ? sPx[c * RN + i - 1] : 0.f;
-                        if (fl[k] & kBy) st -= (ly > 0) ? sPy[c * RN + i - RX] : 0.f;
-                        const float unew = u[k][c] + tau * st;
-                        u[k][c] = (tau * f[k][c] + lam * unew) / denom;
-                        sU[c * RN + i] = u[k][c];
+                        float above = sPy[c * PY - RX];
+#pragma unroll
+                        for (int k = 0; k < V; ++k) {
+                            const float py = p[k][2 * c + 1];
+                            const float st = p[k][2 * c] + py - sPx[c * PL + k * RX - 1] - above;
+                            above = py;
+                            const float x = fmaf(lam, fmaf(tau, st, u[k][c]), tf[k][c]), q = x * rden;
+                            u[k][c] = fmaf(fmaf(-denom, q, x), rden, q);
+                            sU[c * PL + k * RX] = u[k][c];
+                        }
                     }
                 }
                 __syncthreads();
             }
 #pragma unroll
-            for (int k = 0; k < PPT; ++k) {
-                if ((fl[k] & (kIn | kTile)) != (kIn | kTile)) continue;
-                const size_t o = go[k];
+            for (int k = 0; k < V; ++k) {
+                const int gy = gy0 + k;
+                if (!(tile_x && inx && ly0 + k >= K && ly0 + k < K + TY && gy < H)) continue;
+                const size_t o = (size_t)gy * W + gx;
 #pragma unroll
                 for (int c = 0; c < 3; ++c) Uo[c * N + o] = u[k][c];
 #pragma unroll
                 for (int c = 0; c < 6; ++c) Po[c * N + o] = p[k][c];
             }
-            __syncthreads();  // the next tile overwrites the staged region
         }
-        if (!grid_sync(gb, gen)) return;
+        if (done + K < niter && !grid_sync(gb, gen)) return;
     }
 }
 
@@ -1797,21 +1811,17 @@ int sobel_partials(int W, int H) { return ((W + 31) / 32) * ((H + 7) / 8); }
 
 // Instantiations the autotuner chooses from: (iterations per super-step, threads per block).
 struct RofVariant {
-    int K, threads;
+    int K, TY, threads;
     const void *kernel;
     size_t smem;
 };
-static const RofVariant kRofVariants[] = {
-    // the region of K = 2, 4, 6, 8, 12 holds 720, 960, 1232, 1536, 2240 pixels: 2, 2, 2, 2 or 3, 4 per thread
-    {2, 384, (const void *)k_rof_persistent<2, 384>, rof_smem<2>()},
-    {4, 480, (const void *)k_rof_persistent<4, 480>, rof_smem<4>()},
-    {6, 640, (const void *)k_rof_persistent<6, 640>, rof_smem<6>()},
-    {8, 768, (const void *)k_rof_persistent<8, 768>, rof_smem<8>()},
-    {8, 512, (const void *)k_rof_persistent<8, 512>, rof_smem<8>()},
-    {12, 576, (const void *)k_rof_persistent<12, 576>, rof_smem<12>()},
-};
+#define LFRV_ROF(K, TY, V) {K, TY, rof_threads<K, TY, V>(), (const void *)k_rof_persistent<K, TY, V>, rof_smem<K, TY, V>()}
+static const RofVariant kRofVariants[] = {LFRV_ROF(4, 16, 2), LFRV_ROF(4, 16, 4),  LFRV_ROF(6, 16, 2),
+                                          LFRV_ROF(8, 16, 2), LFRV_ROF(8, 32, 4),  LFRV_ROF(10, 16, 2),
+                                          LFRV_ROF(6, 8, 2),  LFRV_ROF(8, 8, 2),   LFRV_ROF(4, 32, 2)};
+#undef LFRV_ROF
 int rof_variant_count() { return (int)(sizeof(kRofVariants) / sizeof(kRofVariants[0])); }
-int rof_default_variant() { return 3; }  // K = 8, 768 threads
+int rof_default_variant() { return 3; }  // K = 8, tiles of 32 x 16, two pixels per thread
 
 // Number of super-steps of variant v for niter iterations: the result is in (U1, P1) when it is odd.
 int rof_persistent_steps(int niter, int v) { return (niter + kRofVariants[v].K - 1) / kRofVariants[v].K; }
@@ -1829,7 +1839,7 @@ cudaError_t launch_rof_persistent(int W, int H, int niter, float tau, float sigm
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, R.kernel, R.threads, R.smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    const int ntiles = ((W + kRofTX - 1) / kRofTX) * ((H + kRofTY - 1) / kRofTY);
+    const int ntiles = ((W + kRofTX - 1) / kRofTX) * ((H + R.TY - 1) / R.TY);
     const int blocks = std::min(ntiles, sms * per_sm);
     void *args[] = {&W, &H, &niter, &tau, &sigma, &lam, &U0, &P0, &U1, &P1, (void *)&F, (void *)&g, &gb};
     lc.add(1);
