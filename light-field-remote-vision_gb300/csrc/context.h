@@ -57,7 +57,7 @@ struct Workspace {
     DevBuf hb_in, hb_out;
     // batched calls: the view gradients of each distinct light field, shared by the jobs that render from it
     DevBuf vg_pool;
-    // corrected IBR_color: iterates, data gradients and metric (15 N floats), the FP64 dual / momentum fields (24 N)
+    // corrected IBR_color: iterates, data gradients and metric (15 N floats), the dual / momentum fields (48 N)
     DevBuf tv;
     // the device scene generator's planes and bumps
     DevBuf scene;

@@ -393,14 +393,13 @@ static int rof_autotune(lfrv_ctx *c, int W, int H, float tau, float sigma, float
 // The FGP's counterpart of rof_autotune: every instantiation of the arithmetic in use, timed on scratch copies of
 // the dual (16 iterations) on first use per image size; the fastest is cached. All give the same iterates.
 static int fgp_autotune(lfrv_ctx *c, int W, int H, bool extended, const float *F, const float *lam, const float *linv,
-                        const float *g, const double *P) {
+                        const float *g, const float *P) {
     const long long key = ((long long)W << 33) | ((long long)H << 1) | (extended ? 1 : 0);
     auto it = c->fgp_tuned.find(key);
     if (it != c->fgp_tuned.end()) return it->second;
     const size_t N = (size_t)W * H;
-    c->ws.tune.ensure(sizeof(double) * 24 * N + sizeof(float) * 3 * N);
-    double *P0 = c->ws.tune.as<double>(), *P1 = P0 + 6 * N, *Q0 = P1 + 6 * N, *Q1 = Q0 + 6 * N;
-    float *U = reinterpret_cast<float *>(Q1 + 6 * N);
+    c->ws.tune.ensure(sizeof(float) * 51 * N);
+    float *P0 = c->ws.tune.as<float>(), *P1 = P0 + 12 * N, *Q0 = P1 + 12 * N, *Q1 = Q0 + 12 * N, *U = Q1 + 12 * N;
     cudaStream_t s = c->stream;
     cudaEvent_t e0, e1;
     LFRV_CUDA(cudaEventCreate(&e0));
@@ -409,7 +408,7 @@ static int fgp_autotune(lfrv_ctx *c, int W, int H, bool extended, const float *F
     float best_ms = 1e30f;
     LaunchCounter quiet;  // trial launches are not the caller's kernels
     for (int v = 0; v < tv_fgp_variant_count(extended); ++v) {
-        LFRV_CUDA(cudaMemcpyAsync(P0, P, sizeof(double) * 6 * N, cudaMemcpyDeviceToDevice, s));
+        LFRV_CUDA(cudaMemcpyAsync(P0, P, sizeof(float) * 12 * N, cudaMemcpyDeviceToDevice, s));
         const GridBarrier gb = fresh_barrier(c);
         LFRV_CUDA(cudaEventRecord(e0, s));
         const cudaError_t e = launch_tv_fgp(W, H, 16, F, lam, linv, g, P0, P1, Q0, Q1, U, gb, s, quiet, extended, v);
@@ -500,7 +499,7 @@ struct TvSolve {
     Buckets B{};
     ColorBuffers b{};
     float *u = nullptr, *up = nullptr, *gf = nullptr, *gfp = nullptr, *D = nullptr, *lam = nullptr, *linv = nullptr;
-    double *P0 = nullptr, *P1 = nullptr, *Q0 = nullptr, *Q1 = nullptr;
+    float *P0 = nullptr, *P1 = nullptr, *Q0 = nullptr, *Q1 = nullptr;
     double t = 1.0, E_prev = 1e300, E = 0.0, gap = 1e300;
     bool extended = false, done = false;
     int k = 0, npart = 0;
@@ -513,9 +512,8 @@ struct TvSolve {
         Workspace &ws = c->ws;
         const size_t N = G.N, N3 = 3 * N;
         cudaStream_t s = c->stream;
-        // 15 N floats (u, u_prev, grad f, grad f_prev, D, lam, 1/L), then 24 N doubles (p, its ping-pong copy, q x 2)
-        const size_t fbytes = (sizeof(float) * 15 * N + 255) / 256 * 256;
-        ws.tv.ensure(fbytes + sizeof(double) * 24 * N);
+        // 15 N floats (u, u_prev, grad f, grad f_prev, D, lam, 1/L), then 48 N (p, its ping-pong copy, q x 2: pairs)
+        ws.tv.ensure(sizeof(float) * 63 * N);
         u = ws.tv.as<float>();
         up = u + N3;
         gf = up + N3;
@@ -523,17 +521,17 @@ struct TvSolve {
         D = gfp + N3;
         lam = D + N;
         linv = lam + N;
-        P0 = reinterpret_cast<double *>(ws.tv.as<char>() + fbytes);
-        P1 = P0 + 6 * N;
-        Q0 = P1 + 6 * N;
-        Q1 = Q0 + 6 * N;
+        P0 = linv + N;
+        P1 = P0 + 12 * N;
+        Q0 = P1 + 12 * N;
+        Q1 = Q0 + 12 * N;
         launch_tv_metric(G, B, tau2, b.wgt, as2(), cfg.lambda, D, lam, linv, s, c->launches);
         check_launch("tv metric");
         launch_tv_clamp(N3, ws.U.as<float>(), u, s, c->launches);
         // u_prev = u and grad f(u_prev) = 0: the first step (theta = 0) reads them only through zero factors
         LFRV_CUDA(cudaMemcpyAsync(up, u, sizeof(float) * N3, cudaMemcpyDeviceToDevice, s));
         LFRV_CUDA(cudaMemsetAsync(gfp, 0, sizeof(float) * N3, s));
-        if (meta == 0) LFRV_CUDA(cudaMemsetAsync(P0, 0, sizeof(double) * 6 * N, s));
+        if (meta == 0) LFRV_CUDA(cudaMemsetAsync(P0, 0, sizeof(float) * 12 * N, s));
         npart = tv_gap_partials(G.W, G.H);
         t = 1.0;
         E_prev = 1e300;
@@ -1445,6 +1443,7 @@ extern "C" int lfrv_ctx_create(lfrv_ctx **out, int device) {
     LFRV_CUDA(cudaEventCreate(&c->ev1));
     LFRV_CUDA(cudaEventCreateWithFlags(&c->vg_ready, cudaEventDisableTiming));
     gaussian_kernel_init();
+    set_fgp_beta();
     {
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {

@@ -188,10 +188,11 @@ void launch_tv_metric(const Geometry &G, const Buckets &B, const float *tau, con
 // grad f = as2 sum_i A_i^T res_i (3 planes) from the splat-set residuals of launch_residual.
 void launch_tv_gradf(const Geometry &G, const Buckets &B, const float *tau, const float *res, float as2, float *gf,
                      cudaStream_t st, LaunchCounter &lc);
-// FP64 block partials of J_g(u), sum <grad u, p> and the box term of the certificate (c = gf - lambda div p; p FP64),
+// FP64 block partials of J_g(u), sum <grad u, p> and the box term of the certificate (c = gf - lambda div p; p as
+// launch_tv_fgp's dual),
 // three arrays of tv_gap_partials(W, H) entries each.
 int tv_gap_partials(int W, int H);
-void launch_tv_gap(int W, int H, const float *u, const float *gf, const double *P, const float *g, float lambda,
+void launch_tv_gap(int W, int H, const float *u, const float *gf, const float *P, const float *g, float lambda,
                    double *partial, cudaStream_t st, LaunchCounter &lc);
 // Scalars of a corrected IBR_color solve whose loop runs on the device (a conditional graph): FISTA's t, the
 // previous and current energy, the certified gap, steps taken, the stop and arithmetic flags, the non-finite flag,
@@ -214,14 +215,16 @@ void launch_tv_decide(const double *sums, double dt_alpha, double lambda, double
 // out = clamp(in, 0, 1) over n floats.
 void launch_tv_clamp(size_t n, const float *in, float *out, cudaStream_t st, LaunchCounter &lc);
 // niter FGP iterations on the dual of the weighted ROF problem (one cooperative launch): P0 holds the starting
-// dual (6 FP64 planes: x parts of the 3 channels, then the y parts) and receives the final one; P1, Q0, Q1 are
-// scratch (6 FP64 planes each); U receives clamp(F + lam div p, 0, 1). extended: the dual's arithmetic in
-// double-float (about 44 bits; else FP32), with the same FP64 storage.
+// dual (6 planes: x parts of the 3 channels, then the y parts; each value an unevaluated sum of two floats, the 6 high
+// planes before the 6 low ones) and receives the final one; P1, Q0, Q1 are scratch (12 planes each); U receives clamp(F + lam div p, 0, 1). extended: the dual's arithmetic in
+// double-float (about 44 bits; else FP32), with the same storage.
 // variant: the instantiation (iterations per super-step, block size) the autotuner picked; all give the same
 // iterates (tv_fgp_variant_count per arithmetic; out of range: the default).
 cudaError_t launch_tv_fgp(int W, int H, int niter, const float *F, const float *lam, const float *linv, const float *g,
-                          double *P0, double *P1, double *Q0, double *Q1, float *U, GridBarrier gb, cudaStream_t st,
+                          float *P0, float *P1, float *Q0, float *Q1, float *U, GridBarrier gb, cudaStream_t st,
                           LaunchCounter &lc, bool extended, int variant = -1);
+// The momentum weights, per device (called when a context is created).
+void set_fgp_beta();
 int tv_fgp_variant_count(bool extended);
 int tv_fgp_default_variant(bool extended);
 // The gap above which the FGP runs in FP32 (its certificate floor is near 4e-4): double-float takes over below it.

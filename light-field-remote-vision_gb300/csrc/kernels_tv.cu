@@ -14,6 +14,7 @@
 #include "kernels.h"
 #include "lfrv_internal.h"
 
+#include <cmath>
 #include <mutex>
 #include <type_traits>
 
@@ -65,10 +66,20 @@ __global__ void k_tv_gradf(int W, int H, int n, int dsf, int BW, const unsigned 
     for (int c = 0; c < 3; ++c) gf[c * N + o] = as2 * acc[c];
 }
 
+// A plane of the dual in FP64: it is stored as an unevaluated sum of two floats, the six high planes, then the six low
+// ones (12 N floats). The low planes cost nothing where the arithmetic is FP32, and no load or store of the inner
+// iterations converts (a conversion holds this GPU's narrow FP64 pipe for 16 cycles a warp: with FP64 storage the
+// conversions were a third of the FP32 iterations' time).
+struct TvDualPlane {
+    const float *hi, *lo;
+    __device__ __forceinline__ TvDualPlane(const float *P, int plane, size_t N) : hi(P + plane * N), lo(P + (6 + plane) * N) {}
+    __device__ __forceinline__ double operator[](size_t o) const { return (double)hi[o] + (double)lo[o]; }
+};
+
 // div of a dual field at (x, y): the negative adjoint of the forward gradient with zero at the last column / row.
-template <typename TD>
-__device__ __forceinline__ TD tv_div(const TD *px, const TD *py, int W, int H, int x, int y, size_t o) {
-    TD d = 0;
+__device__ __forceinline__ double tv_div(const TvDualPlane &px, const TvDualPlane &py, int W, int H, int x, int y,
+                                         size_t o) {
+    double d = 0;
     if (x < W - 1) d += px[o];
     if (x > 0) d -= px[o - 1];
     if (y < H - 1) d += py[o];
@@ -81,7 +92,7 @@ __device__ __forceinline__ TD tv_div(const TD *px, const TD *py, int W, int H, i
 // kGapBX x kGapBY patch of pixels.
 constexpr int kGapBX = 32, kGapBY = 8;
 __global__ void __launch_bounds__(kGapBX * kGapBY) k_tv_gap(int W, int H, const float *__restrict__ u,
-                                                            const float *__restrict__ gf, const double *__restrict__ P,
+                                                            const float *__restrict__ gf, const float *__restrict__ P,
                                                             const float *__restrict__ g, float lambda,
                                                             double *__restrict__ partial) {
     __shared__ double red[kGapBX * kGapBY / 32];
@@ -98,7 +109,7 @@ __global__ void __launch_bounds__(kGapBX * kGapBY) k_tv_gap(int W, int H, const 
             const double gxv = x < W - 1 ? (double)uc[o + 1] - (double)uc[o] : 0.0;
             const double gyv = y < H - 1 ? (double)uc[o + W] - (double)uc[o] : 0.0;
             n2 += gxv * gxv + gyv * gyv;
-            const double *px = P + c * N, *py = P + (3 + c) * N;
+            const TvDualPlane px(P, c, N), py(P, 3 + c, N);
             inner += gxv * px[o] + gyv * py[o];
             const double cc = (double)gf[c * N + o] - (double)lambda * tv_div(px, py, W, H, x, y, o);
             box += (double)uc[o] * cc - fmin(0.0, cc);
@@ -137,15 +148,19 @@ __global__ void k_tv_clamp(size_t n, const float *__restrict__ in, float *__rest
 // updated part of the region shrinks by a pixel per iteration to what the tile still depends on). Per iteration:
 //   u = clamp(F + lam div q, 0, 1);  p' = proj_{|.|_F <= g}(q + grad u / L);  q = p' + beta_j (p' - p);  p = p'
 // with beta_j = (s_j - 1) / s_{j+1}, s_0 = 1, s_{j+1} = (1 + sqrt(1 + 4 s_j^2)) / 2 (Beck and Teboulle's FGP).
-// Every thread owns the same PPT region pixels throughout: their q, p, F, lam, 1/L and g stay in registers, and
-// shared memory carries what the neighbours read (u for the gradient, the x and y components of q for the
-// divergence). The block sizes split the region evenly.
-// The dual p and the momentum point q are stored in FP64 (12 planes); u, F, lam, 1/L and g are FP32. TD is the
-// dual's arithmetic type. In FP32 the dual's rounding (a few ulp of |p| <= g) leaves lambda div p, and with it the
+// A thread owns V vertically adjacent pixels throughout: their q, p, u, F, lam, 1/L and g stay in registers, the
+// neighbours above and below come from registers except at the ends, and shared memory carries u, the x components of q
+// and the y components of each thread's last pixel. As in the persistent ROF no pixel has a branch for the image: a dual
+// whose difference does not exist starts at 0 and has step 0, a block with one tile reads back only the halo, and threads
+// the tile no longer depends on skip the iteration.
+// The dual p and the momentum point q are stored as pairs of floats (TvDualPlane); u, F, lam, 1/L and g are FP32. TD is
+// the dual's arithmetic type. In FP32 the dual's rounding (a few ulp of |p| <= g) leaves lambda div p, and with it the
 // certificate's box term, a noise floor near 4e-4 relative at 256^2; with the double-float type below (about 44
 // bits) the certificate reaches 1e-4, as with FP64 (the oracle's FP32 mirror shows the floor, its FP64 dual does
 // not). FP64 arithmetic is slow on this GPU's narrow FP64 pipe and double-float costs several FP32 operations per
 // operation, so the host runs TD = float while the gap is far above its floor and TD = dfloat to finish.
+// 256^2, 200 iterations: FP32 640 -> 228 us, double-float 1890 -> 754, against FP64 storage and momentum weights
+// converted by every thread in every iteration.
 // Double-float arithmetic (an unevaluated sum hi + lo of two floats, about 44 significant bits): the dual's
 // arithmetic where FP32 would leave its noise floor, on the FP32 pipes. Sums use the error-free two-sum (Knuth)
 // and products the FMA-based two-product (Dekker's splitting replaced by fmaf), each renormalised with the
@@ -155,13 +170,8 @@ struct dfloat {
     __device__ __forceinline__ dfloat() : hi(0.f), lo(0.f) {}
     __device__ __forceinline__ dfloat(int v) : hi((float)v), lo(0.f) {}
     __device__ __forceinline__ dfloat(float v) : hi(v), lo(0.f) {}
-    __device__ __forceinline__ dfloat(double v) {
-        hi = __double2float_rn(v);
-        lo = __double2float_rn(v - (double)hi);
-    }
     __device__ __forceinline__ dfloat(float h, float l) : hi(h), lo(l) {}
     __device__ __forceinline__ explicit operator float() const { return hi + lo; }
-    __device__ __forceinline__ explicit operator double() const { return (double)hi + (double)lo; }
 };
 __device__ __forceinline__ dfloat df_fast_two_sum(float a, float b) {
     const float s = __fadd_rn(a, b);
@@ -210,227 +220,252 @@ __device__ __forceinline__ float df_div4(dfloat a0, dfloat a1, dfloat a2, dfloat
     return __fadd_rn(h.hi, __fadd_rn(__fadd_rn(__fadd_rn(h1.lo, h2.lo), h.lo), lo));
 }
 
-constexpr int kFgpTX = 32, kFgpTY = 16;
-template <int K>
-constexpr int fgp_rn() { return (kFgpTX + 2 * K) * (kFgpTY + 2 * K); }
-template <typename TD, int K>
-constexpr size_t fgp_smem() { return (size_t)6 * fgp_rn<K>() * sizeof(TD) + (size_t)3 * fgp_rn<K>() * sizeof(float); }
-constexpr int kFgpBetaTable = 256;
+constexpr int kFgpTX = 32;
+template <int K, int TY, int V>
+__host__ __device__ constexpr int fgp_threads() {
+    return ((kFgpTX + 2 * K) * ((TY + 2 * K) / V) + 31) / 32 * 32;
+}
+// a plane of the region with one row more and a cell on either side; of the segments' last pixels
+template <int K, int TY, int V>
+__host__ __device__ constexpr int fgp_plane() {
+    return (kFgpTX + 2 * K) * (TY + 2 * K + 1) + 2;
+}
+template <int K, int TY, int V>
+__host__ __device__ constexpr int fgp_plane_y() {
+    return (kFgpTX + 2 * K) * ((TY + 2 * K) / V + 1);
+}
+template <typename TD, int K, int TY, int V>
+constexpr size_t fgp_smem() {
+    return sizeof(TD) * 3 * (size_t)(fgp_plane<K, TY, V>() + fgp_plane_y<K, TY, V>()) +
+           sizeof(float) * 3 * (size_t)fgp_plane<K, TY, V>();
+}
 
-template <typename TD, int K, int THREADS>
-__global__ void __launch_bounds__(THREADS) k_tv_fgp(int W, int H, int niter, const float *__restrict__ F,
-                                                    const float *__restrict__ lam, const float *__restrict__ linv,
-                                                    const float *__restrict__ g, double *P0, double *P1, double *Q0,
-                                                    double *Q1, float *__restrict__ U, GridBarrier gb) {
-    constexpr int RX = kFgpTX + 2 * K, RY = kFgpTY + 2 * K, RN = RX * RY;
-    constexpr int PPT = (RN + THREADS - 1) / THREADS;
-    constexpr unsigned kIn = 1, kFx = 2, kFy = 4, kBx = 8, kBy = 16, kTile = 32, kRx = 64, kRy = 128;
-    constexpr int kDistShift = 8;
-    extern __shared__ __align__(16) unsigned char fgp_sm[];
-    TD *sQx = reinterpret_cast<TD *>(fgp_sm), *sQy = sQx + 3 * RN;
-    float *sU = reinterpret_cast<float *>(sQy + 3 * RN);
-    // the momentum weights beta_j of the first kFgpBetaTable iterations, worked out once per block (the FP64
-    // square root and division are long sequences on this GPU's narrow FP64 pipe; later iterations, if any,
-    // continue the sequence inline)
-    __shared__ double s_beta[kFgpBetaTable];
-    __shared__ double s_tail;  // s_j after the table
-    if (threadIdx.x == 0) {
-        double sj = 1.0;
-        for (int j = 0; j < min(niter, kFgpBetaTable); ++j) {
-            const double s1 = 0.5 * (1.0 + sqrt(1.0 + 4.0 * sj * sj));
-            s_beta[j] = (sj - 1.0) / s1;
-            sj = s1;
-        }
-        s_tail = sj;
+// The momentum weights beta_j of the first kFgpBetaTable iterations (high and low float of the FP64 value).
+constexpr int kFgpBetaTable = 256;
+static_assert(kTvInnerIterations <= kFgpBetaTable, "a launch stays within the table");
+__constant__ float2 c_fgp_beta[kFgpBetaTable];
+
+void set_fgp_beta() {
+    float2 t[kFgpBetaTable];
+    double s = 1.0;
+    for (int j = 0; j < kFgpBetaTable; ++j) {
+        const double s1 = 0.5 * (1.0 + std::sqrt(1.0 + 4.0 * s * s)), b = (s - 1.0) / s1;
+        t[j].x = (float)b;
+        t[j].y = (float)(b - (double)t[j].x);
+        s = s1;
     }
+    cudaMemcpyToSymbol(c_fgp_beta, t, sizeof(t));
+}
+
+__device__ __forceinline__ void fgp_load(const float *P, size_t i, size_t lo, float &v) { v = __ldcg(P + i); }
+__device__ __forceinline__ void fgp_load(const float *P, size_t i, size_t lo, dfloat &v) {
+    v = dfloat(__ldcg(P + i), __ldcg(P + i + lo));
+}
+__device__ __forceinline__ void fgp_store(float *P, size_t i, size_t lo, float v) { P[i] = v; }
+__device__ __forceinline__ void fgp_store(float *P, size_t i, size_t lo, dfloat v) {
+    P[i] = v.hi;
+    P[i + lo] = v.lo;
+}
+__device__ __forceinline__ void fgp_beta(int j, float &b) { b = c_fgp_beta[j].x; }
+__device__ __forceinline__ void fgp_beta(int j, dfloat &b) { b = dfloat(c_fgp_beta[j].x, c_fgp_beta[j].y); }
+
+template <typename TD, int K, int TY, int V>
+__global__ void __launch_bounds__((fgp_threads<K, TY, V>())) k_tv_fgp(int W, int H, int niter,
+                                                                      const float *__restrict__ F,
+                                                                      const float *__restrict__ lam,
+                                                                      const float *__restrict__ linv,
+                                                                      const float *__restrict__ g, float *P0, float *P1,
+                                                                      float *Q0, float *Q1, float *__restrict__ U,
+                                                                      GridBarrier gb) {
+    constexpr bool DF = std::is_same<TD, dfloat>::value;
+    constexpr int RX = kFgpTX + 2 * K, RY = TY + 2 * K;
+    static_assert(RY % V == 0, "whole segments");
+    constexpr int PL = fgp_plane<K, TY, V>(), PY = fgp_plane_y<K, TY, V>();
+    extern __shared__ __align__(16) unsigned char fgp_sm[];
+    TD *sQ = reinterpret_cast<TD *>(fgp_sm);
+    float *sF = reinterpret_cast<float *>(sQ + 3 * (PL + PY));
+    const int seg = threadIdx.x / RX, lx = threadIdx.x - seg * RX, ly0 = seg * V;
+    const bool mine = seg < RY / V;
+    TD *sQx = sQ + 1 + ly0 * RX + lx;                   // this thread's first pixel, plane 0
+    TD *sQy = sQ + 3 * PL + (seg + 1) * RX + lx;        // its last pixel; - RX: the segment above
+    float *sU = sF + 1 + ly0 * RX + lx;
+    const int tiles_x = (W + kFgpTX - 1) / kFgpTX, ntiles = tiles_x * ((H + TY - 1) / TY);
+    const bool resident = ntiles <= (int)gridDim.x;  // one tile per block
+    const size_t N = (size_t)W * H, lo = 6 * N;
+    // distance of the segment's column and of its nearest row from the tile
+    const int dx = max(max(K - lx, lx - (K + kFgpTX - 1)), 0);
+    const int dist = max(dx, max(max(K - (ly0 + V - 1), ly0 - (K + TY - 1)), 0));
+    const bool tile_x = mine && lx >= K && lx < K + kFgpTX;
+    // shared memory that no thread writes (pads) is read too: finite from here on
+    for (int i = threadIdx.x; i < 3 * (PL + PY); i += blockDim.x) sQ[i] = TD(0);
+    for (int i = threadIdx.x; i < 3 * PL; i += blockDim.x) sF[i] = 0.f;
     __syncthreads();
-    const int tiles_x = (W + kFgpTX - 1) / kFgpTX, ntiles = tiles_x * ((H + kFgpTY - 1) / kFgpTY);
-    const size_t N = (size_t)W * H;
     unsigned int gen = 0;
-    double s_step = s_tail;  // s_j of the first iteration past the table (every thread follows the same sequence)
     int step = 0;
+    TD q[V][6], p[V][6];
+    float f[V][3], u[V][3], lm[V], lx_inv[V], ly_inv[V], gg[V];
     for (int done = 0; done < niter; done += K, ++step) {
         const int iters = min(K, niter - done);
-        const double *Pi = (step & 1) ? P1 : P0;
-        double *Po = (step & 1) ? P0 : P1;
-        const double *Qi = step == 0 ? P0 : ((step & 1) ? Q1 : Q0);  // q starts at p
-        double *Qo = (step & 1) ? Q0 : Q1;
+        const float *Pi = (step & 1) ? P1 : P0;
+        float *Po = (step & 1) ? P0 : P1;
+        const float *Qi = step == 0 ? P0 : ((step & 1) ? Q1 : Q0);  // q starts at p
+        float *Qo = (step & 1) ? Q0 : Q1;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-            const int rx0 = (t % tiles_x) * kFgpTX - K, ry0 = (t / tiles_x) * kFgpTY - K;
-            TD q[PPT][6], p[PPT][6];
-            float f[PPT][3], lm[PPT], li[PPT], gg[PPT];
-            unsigned int fl[PPT];
-            size_t go[PPT];
+            const int gx = (t % tiles_x) * kFgpTX - K + lx, gy0 = (t / tiles_x) * TY - K + ly0;
+            const bool inx = mine && gx >= 0 && gx < W;
 #pragma unroll
-            for (int k = 0; k < PPT; ++k) {
-                const int i = threadIdx.x + k * THREADS;
-                const int lx = i % RX, ly = i / RX, gx = rx0 + lx, gy = ry0 + ly;
-                const bool in = i < RN && gx >= 0 && gx < W && gy >= 0 && gy < H;
-                unsigned int f0 = 0;
-                if (in) {
-                    f0 |= kIn;
-                    if (gx < W - 1) f0 |= kFx;
-                    if (gy < H - 1) f0 |= kFy;
-                    if (gx > 0) f0 |= kBx;
-                    if (gy > 0) f0 |= kBy;
-                    if (lx + 1 < RX) f0 |= kRx;
-                    if (ly + 1 < RY) f0 |= kRy;
-                    if (lx >= K && lx < K + kFgpTX && ly >= K && ly < K + kFgpTY) f0 |= kTile;
-                    const int dx = max(max(K - lx, lx - (K + kFgpTX - 1)), 0);
-                    const int dy = max(max(K - ly, ly - (K + kFgpTY - 1)), 0);
-                    f0 |= (unsigned int)max(dx, dy) << kDistShift;
-                }
-                fl[k] = f0;
+            for (int k = 0; k < V; ++k) {
+                const int gy = gy0 + k;
+                const bool in = inx && gy >= 0 && gy < H;
+                const bool own = tile_x && ly0 + k >= K && ly0 + k < K + TY;
                 const size_t o = in ? (size_t)gy * W + gx : 0;
-                go[k] = o;
+                if (step == 0 || !resident) {
 #pragma unroll
-                for (int c = 0; c < 6; ++c) {
-                    q[k][c] = in ? (TD)__ldcg(Qi + c * N + o) : TD(0);
-                    p[k][c] = in ? (TD)__ldcg(Pi + c * N + o) : TD(0);
+                    for (int c = 0; c < 3; ++c) f[k][c] = in ? __ldg(F + c * N + o) : 0.f;
+                    lm[k] = in ? __ldg(lam + o) : 0.f;
+                    const float li = in ? __ldg(linv + o) : 0.f;
+                    lx_inv[k] = gx < W - 1 ? li : 0.f;
+                    ly_inv[k] = gy < H - 1 ? li : 0.f;
+                    gg[k] = in ? __ldg(g + o) : 0.f;
                 }
+                if (step == 0 || !resident || !own) {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) f[k][c] = in ? __ldg(F + c * N + o) : 0.f;
-                lm[k] = in ? __ldg(lam + o) : 0.f;
-                li[k] = in ? __ldg(linv + o) : 0.f;
-                gg[k] = in ? __ldg(g + o) : 0.f;
-                if (i < RN) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        sQx[c * RN + i] = q[k][c];
-                        sQy[c * RN + i] = q[k][3 + c];
+                    for (int c = 0; c < 6; ++c) {
+                        q[k][c] = p[k][c] = TD(0);
+                        if (in) {
+                            fgp_load(Qi, c * N + o, lo, q[k][c]);
+                            fgp_load(Pi, c * N + o, lo, p[k][c]);
+                        }
                     }
                 }
+                if (mine) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) sQx[c * PL + k * RX] = q[k][c];
+                }
+            }
+            if (mine) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) sQy[c * PY] = q[V - 1][3 + c];
             }
             __syncthreads();
-            double s = s_step;
             for (int it = 0; it < iters; ++it) {
-                const int j = done + it;
-                double s1 = s;
                 TD beta;
-                if (j < kFgpBetaTable) {
-                    beta = (TD)s_beta[j];
-                } else {
-                    s1 = 0.5 * (1.0 + sqrt(1.0 + 4.0 * s * s));
-                    beta = (TD)((s - 1.0) / s1);
-                }
+                fgp_beta(done + it, beta);
                 // u(q) where the tile still depends on it (values next to the region's edge are stale and stay
                 // outside the tile)
-                const unsigned int u_reach = (unsigned int)(iters - it) << kDistShift;
-                const unsigned int p_reach = (unsigned int)(iters - it - 1) << kDistShift;
-#pragma unroll
-                for (int k = 0; k < PPT; ++k) {
-                    if (!(fl[k] & kIn) || (fl[k] & ~0xFFu) > u_reach) continue;
-                    const int i = threadIdx.x + k * THREADS;
-                    const int lx = i % RX, ly = i / RX;
+                if (mine && dist <= iters - it) {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        float dv;
-                        if constexpr (std::is_same<TD, dfloat>::value) {
-                            const dfloat z;
-                            dv = df_div4((fl[k] & kFx) ? q[k][c] : z,
-                                         ((fl[k] & kBx) && lx > 0) ? sQx[c * RN + i - 1] : z,
-                                         (fl[k] & kFy) ? q[k][3 + c] : z,
-                                         ((fl[k] & kBy) && ly > 0) ? sQy[c * RN + i - RX] : z);
-                        } else {
-                            TD d = 0;
-                            if (fl[k] & kFx) d += q[k][c];
-                            if (fl[k] & kBx) d -= lx > 0 ? sQx[c * RN + i - 1] : TD(0);
-                            if (fl[k] & kFy) d += q[k][3 + c];
-                            if (fl[k] & kBy) d -= ly > 0 ? sQy[c * RN + i - RX] : TD(0);
-                            dv = (float)d;
+                        TD above = sQy[c * PY - RX];
+#pragma unroll
+                        for (int k = 0; k < V; ++k) {
+                            const TD left = sQx[c * PL + k * RX - 1];
+                            float dv;
+                            if constexpr (DF) dv = df_div4(q[k][c], left, q[k][3 + c], above);
+                            else dv = __fsub_rn(__fadd_rn(__fsub_rn(q[k][c], left), q[k][3 + c]), above);
+                            above = q[k][3 + c];
+                            u[k][c] = fminf(1.0f, fmaxf(0.0f, __fmaf_rn(lm[k], dv, f[k][c])));
+                            sU[c * PL + k * RX] = u[k][c];
                         }
-                        sU[c * RN + i] = fminf(1.0f, fmaxf(0.0f, f[k][c] + lm[k] * dv));
                     }
                 }
                 __syncthreads();
                 // p' = proj(q + grad u / L), q = p' + beta (p' - p) (own pixel)
+                if (mine && dist <= iters - it - 1) {
 #pragma unroll
-                for (int k = 0; k < PPT; ++k) {
-                    if (!(fl[k] & kIn) || (fl[k] & ~0xFFu) > p_reach) continue;
-                    const int i = threadIdx.x + k * THREADS;
-                    TD v[6];
-                    TD n2 = 0;
+                    for (int k = 0; k < V; ++k) {
+                        TD v[6];
+                        TD n2 = TD(0);
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const float *uc = sU + c * RN;
-                        const float ui = uc[i];
-                        const float ur = (fl[k] & kRx) ? uc[i + 1] : 0.f;
-                        const float ud = (fl[k] & kRy) ? uc[i + RX] : 0.f;
-                        const float gxv = (fl[k] & kFx) ? ur - ui : 0.f;
-                        const float gyv = (fl[k] & kFy) ? ud - ui : 0.f;
-                        if constexpr (std::is_same<TD, dfloat>::value) {
-                            v[c] = df_add_f(q[k][c], gxv * li[k]);
-                            v[3 + c] = df_add_f(q[k][3 + c], gyv * li[k]);
-                            n2 = df_add_sloppy(df_add_sloppy(n2, v[c] * v[c]), v[3 + c] * v[3 + c]);
-                        } else {
-                            v[c] = q[k][c] + (TD)(gxv * li[k]);
-                            v[3 + c] = q[k][3 + c] + (TD)(gyv * li[k]);
-                            n2 += v[c] * v[c] + v[3 + c] * v[3 + c];
+                        for (int c = 0; c < 3; ++c) {
+                            const float ur = sU[c * PL + k * RX + 1];
+                            const float ud = k + 1 < V ? u[k + 1 < V ? k + 1 : k][c] : sU[c * PL + V * RX];
+                            const float gxv = ur - u[k][c], gyv = ud - u[k][c];
+                            if constexpr (DF) {
+                                v[c] = df_add_f(q[k][c], gxv * lx_inv[k]);
+                                v[3 + c] = df_add_f(q[k][3 + c], gyv * ly_inv[k]);
+                                n2 = df_add_sloppy(df_add_sloppy(n2, v[c] * v[c]), v[3 + c] * v[3 + c]);
+                            } else {
+                                // (the fusions written out: the stop test's step count hangs on these roundings)
+                                v[c] = __fmaf_rn(gxv, lx_inv[k], q[k][c]);
+                                v[3 + c] = __fmaf_rn(gyv, ly_inv[k], q[k][3 + c]);
+                                n2 = __fadd_rn(n2, __fmaf_rn(v[c], v[c], __fmul_rn(v[3 + c], v[3 + c])));
+                            }
                         }
-                    }
-                    // projection onto |p| <= g without a square root or division in the extended type: r = 1 / sqrt(n2)
-                    // from the FP32 estimate and two Newton steps in TD (relative error ~1e-13 in double-float),
-                    // applied only where the ball constraint is active
-                    const TD gv = (TD)gg[k];
-                    TD sc = 1;
-                    if (n2 > gv * gv) {
-                        TD r = (TD)rsqrtf((float)n2);
-                        if (sizeof(TD) == sizeof(double)) {
-                            r = r * (TD(1.5) - TD(0.5) * n2 * r * r);
-                            r = r * (TD(1.5) - TD(0.5) * n2 * r * r);
+                        // projection onto |p| <= g without a square root or division: r = 1 / sqrt(n2) from the FP32
+                        // estimate, in double-float with a Newton step in FP32 and one in TD (relative error ~1e-14),
+                        // applied only where the ball constraint is active
+                        const TD gv = TD(gg[k]);
+                        if (n2 > gv * gv) {
+                            TD sc;
+                            if constexpr (DF) {
+                                const float n = (float)n2, e = rsqrtf(n), r0 = fmaf(e * 0.5f, fmaf(-n * e, e, 1.f), e);
+                                // r0 + r0 (1 - n2 r0^2) / 2: the residual is small, so FP32 carries it
+                                const dfloat h = n2 * (dfloat(r0) * dfloat(r0));
+                                const float d = __fsub_rn(__fsub_rn(1.f, h.hi), h.lo);
+                                sc = gv * df_fast_two_sum(r0, __fmul_rn(0.5f * r0, d));
+                            } else {
+                                sc = gv * rsqrtf(n2);
+                            }
+#pragma unroll
+                            for (int c = 0; c < 6; ++c) v[c] = v[c] * sc;
                         }
-                        sc = gv * r;
+#pragma unroll
+                        for (int c = 0; c < 6; ++c) {
+                            const TD pn = v[c];
+                            if constexpr (DF) q[k][c] = df_add_sloppy(pn, beta * (pn - p[k][c]));
+                            else q[k][c] = __fmaf_rn(beta, __fsub_rn(pn, p[k][c]), pn);
+                            p[k][c] = pn;
+                        }
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) sQx[c * PL + k * RX] = q[k][c];
                     }
 #pragma unroll
-                    for (int c = 0; c < 6; ++c) {
-                        const TD pn = v[c] * sc;
-                        if constexpr (std::is_same<TD, dfloat>::value) q[k][c] = df_add_sloppy(pn, beta * (pn - p[k][c]));
-                        else q[k][c] = pn + beta * (pn - p[k][c]);
-                        p[k][c] = pn;
-                    }
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        sQx[c * RN + i] = q[k][c];
-                        sQy[c * RN + i] = q[k][3 + c];
-                    }
+                    for (int c = 0; c < 3; ++c) sQy[c * PY] = q[V - 1][3 + c];
                 }
                 __syncthreads();
-                s = s1;
             }
 #pragma unroll
-            for (int k = 0; k < PPT; ++k) {
-                if ((fl[k] & (kIn | kTile)) != (kIn | kTile)) continue;
-                const size_t o = go[k];
+            for (int k = 0; k < V; ++k) {
+                const int gy = gy0 + k;
+                if (!(tile_x && inx && ly0 + k >= K && ly0 + k < K + TY && gy < H)) continue;
+                const size_t o = (size_t)gy * W + gx;
 #pragma unroll
                 for (int c = 0; c < 6; ++c) {
-                    Po[c * N + o] = (double)p[k][c];
-                    Qo[c * N + o] = (double)q[k][c];
+                    fgp_store(Po, c * N + o, lo, p[k][c]);
+                    fgp_store(Qo, c * N + o, lo, q[k][c]);
                 }
             }
-            __syncthreads();  // the next tile overwrites the staged region
         }
-        for (int it = 0; it < iters; ++it)
-            if (done + it >= kFgpBetaTable) s_step = 0.5 * (1.0 + sqrt(1.0 + 4.0 * s_step * s_step));
         if (!grid_sync(gb, gen)) return;
     }
-    // the final dual sits in P0 after an even number of super-steps, else in P1; u = clamp(F + lam div p)
+    // the final dual sits in P0 after an even number of super-steps, else in P1; u = clamp(F + lam div p). In FP32 its
+    // low planes are 0, which the solve left in P0 alone
     const int steps = (niter + K - 1) / K;
-    const double *Pf = (steps & 1) ? P1 : P0;
-    double *Pother = (steps & 1) ? P0 : P1;
-    for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < N; o += (size_t)gridDim.x * blockDim.x) {
+    const float *Pf = (steps & 1) ? P1 : P0;
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t o = first; o < N; o += stride) {
         const int x = (int)(o % W), y = (int)(o / W);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const double d = tv_div(Pf + c * N, Pf + (3 + c) * N, W, H, x, y, o);
+            const float *px = Pf + c * N, *py = Pf + (3 + c) * N;
+            double d = 0.0;
+            auto add = [&](const float *v, double sign) {
+                d += sign * (double)__ldcg(v);
+                if constexpr (DF) d += sign * (double)__ldcg(v + lo);
+            };
+            if (x < W - 1) add(px + o, 1.0);
+            if (x > 0) add(px + o - 1, -1.0);
+            if (y < H - 1) add(py + o, 1.0);
+            if (y > 0) add(py + o - W, -1.0);
             U[c * N + o] = fminf(1.0f, fmaxf(0.0f, F[c * N + o] + lam[o] * (float)d));
         }
     }
-    // the caller keeps its dual in P0: copy it there when the last super-step wrote P1
-    if (steps & 1) {
-        if (!grid_sync(gb, gen)) return;  // every block has read P1's neighbours above
-        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < 6 * N; i += (size_t)gridDim.x * blockDim.x)
-            Pother[i] = Pf[i];
-    }
+    // the caller keeps its dual in P0
+    if (steps & 1)
+        for (size_t i = first; i < (DF ? 2 : 1) * lo; i += stride) P0[i] = __ldcg(P1 + i);
+    if (!DF)
+        for (size_t i = first; i < lo; i += stride) P0[lo + i] = 0.f;
 }
 
 // ------------------------------------------------------------------ launchers
@@ -457,7 +492,7 @@ void launch_tv_gradf(const Geometry &G, const Buckets &B, const float *tau, cons
 
 int tv_gap_partials(int W, int H) { return ((W + kGapBX - 1) / kGapBX) * ((H + kGapBY - 1) / kGapBY); }
 
-void launch_tv_gap(int W, int H, const float *u, const float *gf, const double *P, const float *g, float lambda,
+void launch_tv_gap(int W, int H, const float *u, const float *gf, const float *P, const float *g, float lambda,
                    double *partial, cudaStream_t st, LaunchCounter &lc) {
     ProfScope _ps(lc, "tv_gap", st);
     const dim3 gr = tv_grid(W, H, dim3(kGapBX, kGapBY));
@@ -521,28 +556,30 @@ void launch_tv_clamp(size_t n, const float *in, float *out, cudaStream_t st, Lau
     lc.add(1);
 }
 
-// Instantiations the FGP autotuner chooses from, per arithmetic: (iterations per super-step K, threads); the
-// region of K = 2, 4, 6, 8 holds 720, 960, 1232, 1536 pixels, two per thread. All give the same iterates.
+// Instantiations the FGP autotuner chooses from, per arithmetic: iterations per super-step K, tile rows TY, pixels per
+// thread V. All give the same iterates.
 struct FgpVariant {
-    int K, threads;
+    int TY, threads;
     const void *kernel;
     size_t smem;
 };
-static const FgpVariant kFgpFloat[] = {
-    {4, 480, (const void *)k_tv_fgp<float, 4, 480>, fgp_smem<float, 4>()},
-    {6, 640, (const void *)k_tv_fgp<float, 6, 640>, fgp_smem<float, 6>()},
-    {8, 768, (const void *)k_tv_fgp<float, 8, 768>, fgp_smem<float, 8>()},
-};
-static const FgpVariant kFgpDfloat[] = {
-    {2, 384, (const void *)k_tv_fgp<dfloat, 2, 384>, fgp_smem<dfloat, 2>()},
-    {4, 480, (const void *)k_tv_fgp<dfloat, 4, 480>, fgp_smem<dfloat, 4>()},
-};
-int tv_fgp_variant_count(bool extended) { return extended ? 2 : 3; }
-int tv_fgp_default_variant(bool extended) { return extended ? 1 : 2; }
+#define LFRV_FGP(TD, K, TY, V) \
+    {TY, fgp_threads<K, TY, V>(), (const void *)k_tv_fgp<TD, K, TY, V>, fgp_smem<TD, K, TY, V>()}
+static const FgpVariant kFgpFloat[] = {LFRV_FGP(float, 4, 16, 2), LFRV_FGP(float, 6, 16, 2), LFRV_FGP(float, 8, 16, 2),
+                                       LFRV_FGP(float, 8, 8, 2), LFRV_FGP(float, 6, 32, 4)};
+static const FgpVariant kFgpDfloat[] = {LFRV_FGP(dfloat, 2, 16, 1), LFRV_FGP(dfloat, 2, 16, 2),
+                                        LFRV_FGP(dfloat, 4, 16, 2), LFRV_FGP(dfloat, 4, 8, 1),
+                                        LFRV_FGP(dfloat, 6, 16, 2)};
+#undef LFRV_FGP
+int tv_fgp_variant_count(bool extended) {
+    return (int)(extended ? sizeof(kFgpDfloat) / sizeof(FgpVariant) : sizeof(kFgpFloat) / sizeof(FgpVariant));
+}
+int tv_fgp_default_variant(bool extended) { return 2; }
 
 cudaError_t launch_tv_fgp(int W, int H, int niter, const float *F, const float *lam, const float *linv, const float *g,
-                          double *P0, double *P1, double *Q0, double *Q1, float *U, GridBarrier gb, cudaStream_t st,
+                          float *P0, float *P1, float *Q0, float *Q1, float *U, GridBarrier gb, cudaStream_t st,
                           LaunchCounter &lc, bool extended, int variant) {
+    if (niter > kFgpBetaTable) return cudaErrorInvalidValue;
     ProfScope _ps(lc, extended ? "tv_fgp_df" : "tv_fgp", st);
     if (variant < 0 || variant >= tv_fgp_variant_count(extended)) variant = tv_fgp_default_variant(extended);
     const FgpVariant &R = extended ? kFgpDfloat[variant] : kFgpFloat[variant];
@@ -564,7 +601,7 @@ cudaError_t launch_tv_fgp(int W, int H, int niter, const float *F, const float *
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, R.kernel, R.threads, R.smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    const int ntiles = ((W + kFgpTX - 1) / kFgpTX) * ((H + kFgpTY - 1) / kFgpTY);
+    const int ntiles = ((W + kFgpTX - 1) / kFgpTX) * ((H + R.TY - 1) / R.TY);
     const int resident = sms * per_sm;
     // as few blocks as keep the per-block tile count at its minimum (no block waits for a straggler's extra tile)
     const int per_block = (ntiles + resident - 1) / resident;
