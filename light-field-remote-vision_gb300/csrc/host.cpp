@@ -336,14 +336,14 @@ static void sobel_target(lfrv_ctx *c, const Geometry &G, const float *U, float *
     if (abs_slot >= 0) reduce_to(c, np, part, abs_slot);
 }
 
-// Weighted residuals of every view at U (and the intensity energy into sums[slot]).
+// Weighted residuals of every view at U (and the intensity energy into sums[slot]; slot < 0: not computed).
 static void residual(lfrv_ctx *c, const Geometry &G, const float *U, const float *img, const float *tau2,
                      const float *wgt, float s2, float *res, int slot, bool splat_set = false) {
     const int np = residual_partials(G);
-    double *part = partial_buf(c, np);
+    double *part = slot >= 0 ? partial_buf(c, np) : nullptr;
     launch_residual(G, U, img, tau2, wgt, s2, res, part, c->stream, c->launches, splat_set);
     check_launch("residual");
-    reduce_to(c, np, part, slot);
+    if (slot >= 0) reduce_to(c, np, part, slot);
 }
 
 // ------------------------------------------------------------------ autotuner
@@ -540,15 +540,26 @@ struct TvSolve {
         k = 0;
     }
     float as2() const { return cfg.dt_alpha * cfg.sigma_sensor * cfg.sigma_sensor; }
-    void eval() {
+    // the data gradient, the energy's and the certificate's partials, and their sums (slots 1, 4, 5, 6)
+    void sums() {
         const float s2 = cfg.sigma_sensor * cfg.sigma_sensor;
-        residual(c, G, u, img, tau2, b.wgt, s2, b.res, 1, true);
+        const int nres = residual_partials(G);
+        double *part = partial_buf(c, nres + 3 * (size_t)npart);
+        launch_residual(G, u, img, tau2, b.wgt, s2, b.res, part, c->stream, c->launches, true);
         launch_tv_gradf(G, B, tau2, b.res, as2(), gf, c->stream, c->launches);
-        check_launch("tv data gradient");
-        double *part = partial_buf(c, 3 * (size_t)npart);
-        launch_tv_gap(G.W, G.H, u, gf, P0, b.g, cfg.lambda, part, c->stream, c->launches);
-        check_launch("tv gap");
-        for (int q = 0; q < 3; ++q) reduce_to(c, npart, part + (size_t)q * npart, 4 + q);
+        launch_tv_gap(G.W, G.H, u, gf, P0, b.g, cfg.lambda, part + nres, c->stream, c->launches);
+        c->ws.sums.ensure(sizeof(double) * 64);
+        ReduceLists l{};
+        for (int q = 0; q < 4; ++q) {
+            l.partial[q] = q == 0 ? part : part + nres + (size_t)(q - 1) * npart;
+            l.count[q] = q == 0 ? nres : npart;
+            l.out[q] = c->ws.sums.as<double>() + (q == 0 ? 1 : 3 + q);
+        }
+        launch_reduce_final(l, 4, c->stream, c->launches);
+    }
+    void eval() {
+        sums();
+        check_launch("tv certificate");
         LFRV_CUDA(cudaMemcpyAsync(host_sums(c), c->ws.sums.p, sizeof(double) * 7, cudaMemcpyDeviceToHost, c->stream));
     }
     // after the stream has completed: true when the solve has stopped (gap reached or the cap)
@@ -603,7 +614,7 @@ struct TvSolve {
         // everything the captured launches use, allocated and tuned before the capture
         const int vf = fgp_autotune(c, G.W, G.H, false, b.F, lam, linv, b.g, P0);
         const int vd = fgp_autotune(c, G.W, G.H, true, b.F, lam, linv, b.g, P0);
-        partial_buf(c, std::max<size_t>((size_t)residual_partials(G), 3 * (size_t)npart));
+        partial_buf(c, (size_t)residual_partials(G) + 3 * (size_t)npart);
         ws.sums.ensure(sizeof(double) * 64);
         ws.tvloop.ensure(sizeof(TvLoopState));
         const int cap = (st && st->energy_trace) ? st->trace_capacity : 0;
@@ -643,12 +654,7 @@ struct TvSolve {
                 return piece;
             };
             auto eval_decide = [&]() {
-                const float s2 = cfg.sigma_sensor * cfg.sigma_sensor;
-                residual(c, G, u, img, tau2, b.wgt, s2, b.res, 1, true);
-                launch_tv_gradf(G, B, tau2, b.res, as2(), gf, s, c->launches);
-                double *part = partial_buf(c, 3 * (size_t)npart);
-                launch_tv_gap(G.W, G.H, u, gf, P0, b.g, cfg.lambda, part, s, c->launches);
-                for (int q = 0; q < 3; ++q) reduce_to(c, npart, part + (size_t)q * npart, 4 + q);
+                sums();
                 launch_tv_decide(ws.sums.as<double>(), (double)cfg.dt_alpha, (double)cfg.lambda, cfg.cg_gap_tol,
                                  cfg.niter, loop, dtrace, cap, h_loop, h_ext, s, c->launches);
             };
@@ -812,8 +818,8 @@ static void color_solve(lfrv_ctx *c, const lfrv_config &cfg, const float *img, c
     const int trace_cap = trace ? st->trace_capacity : 0;
     auto energy = [&](bool need_tv, int trace_slot = -1) -> float {
         // residual pass (also the data term input of the next iteration) + TV term of the reference energy
-        residual(c, G, ws.U.as<float>(), img, tau2, b.wgt, s2, b.res, 1);
         const bool want_trace = trace_slot >= 0 && trace_slot < trace_cap;
+        residual(c, G, ws.U.as<float>(), img, tau2, b.wgt, s2, b.res, need_tv || want_trace ? 1 : -1);
         if (!need_tv && !want_trace) return 0.0f;
         sobel_target(c, G, ws.U.as<float>(), b.Xq, b.Xq + N, b.vis, 0);
         if (gtb.on) energy_gradients(c, cfg, G, gtb, ws.U.as<float>(), tau2, b.wgt, 3);

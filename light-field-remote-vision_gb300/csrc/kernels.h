@@ -84,6 +84,7 @@ void launch_tau(int V, int w, int h, const float *depth, const WarpCams &cams, i
 // ---- solver stage (kernels_solver.cu)
 void launch_bucket_build(const Geometry &G, const float *tau, Buckets &B, cudaStream_t st, LaunchCounter &lc,
                          bool counted = false);
+// partial (residual_partials(G) entries): the energy's block sums; nullptr: not computed.
 void launch_residual(const Geometry &G, const float *U, const float *img, const float *tau, const float *wgt, float s2,
                      float *res, double *partial, cudaStream_t st, LaunchCounter &lc, bool splat_set = false);
 int residual_partials(const Geometry &G);
@@ -138,6 +139,13 @@ int moving_partials(size_t N);
 void set_gaussian(const float k[11]);
 void launch_blur(int W, int H, const float *in, float *tmp, float *out, cudaStream_t st, LaunchCounter &lc);
 void launch_reduce_final(int count, const double *partial, double *out, cudaStream_t st, LaunchCounter &lc);
+// n lists (at most 4) in one launch, each summed as alone.
+struct ReduceLists {
+    const double *partial[4];
+    double *out[4];
+    int count[4];
+};
+void launch_reduce_final(const ReduceLists &lists, int n, cudaStream_t st, LaunchCounter &lc);
 // One energy-trace entry of IBR_color: *dst = lambda (float)sums[0] + alpha (float)sums[1] (+ beta (float)sums[3]
 // when grad), evaluated in float as the reference's host sums it (coco_vtv_sr_primal_energy_unstructured).
 void launch_trace_energy(const double *sums, float lambda, float alpha, float beta, bool grad, double *dst,

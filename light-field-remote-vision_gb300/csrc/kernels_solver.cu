@@ -271,7 +271,9 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_finish(int nb, unsigned int
 // coco_vtv_sr_primal_energy_unstructured :1560-1608). Outside the gather set A_i U = 0.
 // splat_set: the residual over the splat set instead, zero elsewhere (the corrected IBR_color objective, whose
 // gradient splats over the same set).
-template <int KS>
+// ENERGY: the energy's FP64 terms and their block sum, for the callers that read it (half of the kernel's time at 256^2:
+// some ten FP64 operations per pixel on a pipe that takes 16 cycles a warp).
+template <int KS, bool ENERGY>
 __global__ void __launch_bounds__(256) k_residual(int V, int n, int W, int H, int dsf, const float *__restrict__ U,
                                                   const float *__restrict__ img, const float *__restrict__ tau,
                                                   const float *__restrict__ wgt, float s2,
@@ -309,8 +311,9 @@ __global__ void __launch_bounds__(256) k_residual(int V, int n, int W, int H, in
         rv[m] = d0 * w;
         rv[n + m] = d1 * w;
         rv[2 * n + m] = d2 * w;
-        e = (double)s2 * (double)w * ((double)d0 * d0 + (double)d1 * d1 + (double)d2 * d2);
+        if (ENERGY) e = (double)s2 * (double)w * ((double)d0 * d0 + (double)d1 * d1 + (double)d2 * d2);
     }
+    if (!ENERGY) return;
     const double s = block_sum<256>(e, red);
     if (threadIdx.x == 0) partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
 }
@@ -1331,13 +1334,15 @@ __global__ void __launch_bounds__(kBlurBX * kBlurBY) k_blur_cols(int W, int H, c
     out[(size_t)y * W + xo] = s;
 }
 
-// Deterministic final reduction of FP64 partials (single block).
-__global__ void k_reduce_final(int count, const double *__restrict__ partial, double *__restrict__ out) {
+// Deterministic final reduction of FP64 partials: block b sums list b.
+__global__ void k_reduce_final(const ReduceLists lists) {
     __shared__ double red[32];
+    const int count = lists.count[blockIdx.x];
+    const double *partial = lists.partial[blockIdx.x];
     double s = 0.0;
     for (int i = threadIdx.x; i < count; i += blockDim.x) s += partial[i];
     const double t = block_sum<1024>(s, red);
-    if (threadIdx.x == 0) *out = t;
+    if (threadIdx.x == 0) *lists.out[blockIdx.x] = t;
 }
 
 // One energy-trace entry: the host's float expression lambda e_tv + alpha e_int (+ beta e_grad), without
@@ -1417,8 +1422,16 @@ void launch_residual(const Geometry &G, const float *U, const float *img, const 
                      float *res, double *partial, cudaStream_t st, LaunchCounter &lc, bool splat_set) {
     ProfScope _ps(lc, "residual", st);
     const dim3 b(256), g((G.n + 255) / 256, G.V);
-    LFRV_KS_DISPATCH(G.dsf + 1, k_residual, g, b, st, G.V, G.n, G.W, G.H, G.dsf, U, img, tau, wgt, s2, res, partial,
-                     splat_set ? 1 : 0);
+    auto run = [&](auto kernel) {
+        kernel<<<g, b, 0, st>>>(G.V, G.n, G.W, G.H, G.dsf, U, img, tau, wgt, s2, res, partial, splat_set ? 1 : 0);
+    };
+    switch (G.dsf + 1) {
+        case 2: run(partial ? k_residual<2, true> : k_residual<2, false>); break;
+        case 3: run(partial ? k_residual<3, true> : k_residual<3, false>); break;
+        case 4: run(partial ? k_residual<4, true> : k_residual<4, false>); break;
+        case 5: run(partial ? k_residual<5, true> : k_residual<5, false>); break;
+        default: break;
+    }
     lc.add(1);
 }
 int residual_partials(const Geometry &G) { return ((G.n + 255) / 256) * G.V; }
@@ -1863,10 +1876,18 @@ void launch_blur(int W, int H, const float *in, float *tmp, float *out, cudaStre
     lc.add(2);
 }
 
-void launch_reduce_final(int count, const double *partial, double *out, cudaStream_t st, LaunchCounter &lc) {
+void launch_reduce_final(const ReduceLists &lists, int n, cudaStream_t st, LaunchCounter &lc) {
     ProfScope _ps(lc, "reduce_final", st);
-    k_reduce_final<<<1, 1024, 0, st>>>(count, partial, out);
+    k_reduce_final<<<n, 1024, 0, st>>>(lists);
     lc.add(1);
+}
+
+void launch_reduce_final(int count, const double *partial, double *out, cudaStream_t st, LaunchCounter &lc) {
+    ReduceLists l{};
+    l.count[0] = count;
+    l.partial[0] = partial;
+    l.out[0] = out;
+    launch_reduce_final(l, 1, st, lc);
 }
 
 void launch_trace_energy(const double *sums, float lambda, float alpha, float beta, bool grad, double *dst,

@@ -581,11 +581,12 @@ void launch_zbuffer_splat(int V, int w, int h, const float *depth, const WarpCam
     k_zsplat<<<dim3((n + per_block - 1) / per_block, V), 256, 0, st>>>(V, w, h, depth, cams, W, H, zkey, defer);
     lc.add(1);
     if (defer_q) {
-        // as many warps as three blocks per SM hold (the counts are read on the device)
+        // as many warps as three blocks per SM hold (the counts are read on the device), fewer for few quads: a block's
+        // launch costs more there than a longer loop
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        launch_pdl(k_zsplat_defer, dim3(3 * std::max(sms, 1)), dim3(256), 0, st, w, h, depth, cams, W, H, zkey, defer);
+        launch_pdl(k_zsplat_defer, dim3((unsigned)std::min<long long>(3 * std::max(sms, 1), (long long)V * n / 1024 + 8)), dim3(256), 0, st, w, h, depth, cams, W, H, zkey, defer);
         lc.add(1);
     }
 }
