@@ -104,10 +104,8 @@ def algorithmic_bytes(kernel: str, V: int, n: int, N: int, ks: int, cg_iters: in
         "hole_fill_iter": None,
         "sobel": 12 * V * n + 8 * V * n,
         "u_gradient": (8 + 4 + 8) * V * n + 4 * V * n + 4 * N + 12 * N,
-        "cg_init": 12 * N + 8 * N + 24 * N,
-        "cg_apply": 12 * N + 12 * N,
-        "cg_update": 48 * N + 24 * N,
-        "cg_dir": 24 * N + 12 * N,
+        # start: U, g read, r and d written; five iterations: d read, q written; U, r, d, q read, U, r, d written
+        "cg_faithful": 20 * N + 24 * N + 5 * (24 * N + 48 * N + 36 * N),
         "cg_energy": 24 * N + 8 * N,
         "rof_iter": 88 * N,
         # all inner iterations of one ISTA step in one launch: 88 B per target pixel per iteration

@@ -1042,8 +1042,8 @@ static void u_gradient(lfrv_ctx *c, const Geometry &G, const Buckets &B, const f
     check_launch("gradient splat");
 }
 
-// possion_conj_grad with the reference's loop (faithful, defect D1): 5 iterations, host-side scalars as the
-// reference computes them (sources/solver.cu:612-676).
+// possion_conj_grad with the reference's loop (faithful, defect D1): 5 iterations, its scalars on the device (sources/
+// solver.cu:612-676). With an energy trace, one launch per iteration and the energy of each iterate after it.
 static int cg_faithful(lfrv_ctx *c, int W, int H, const float *gx, const float *gy, float *U,
                        double *trace = nullptr) {
     Workspace &ws = c->ws;
@@ -1052,54 +1052,28 @@ static int cg_faithful(lfrv_ctx *c, int W, int H, const float *gx, const float *
     ws.r.ensure(3 * N * sizeof(float));
     ws.d.ensure(3 * N * sizeof(float));
     ws.q.ensure(3 * N * sizeof(float));
-    float *r = ws.r.as<float>(), *d = ws.d.as<float>(), *q = ws.q.as<float>();
-    const int np = cg_partials(W, H);
-    double *part = partial_buf(c, 3 * (size_t)np);
-    // energy trace: the quadratic energy of each iterate against the starting image u0
+    const int np = cg_partials(W, H), iterations = 5;
+    const size_t npart = (size_t)persistent_partials();
+    // the quadratic energy of each iterate is taken against the starting image u0
     const int trace_cap = trace ? c->pending.trace_cap : 0;
     if (trace) {
         ws.U0.ensure(3 * N * sizeof(float));
         LFRV_CUDA(cudaMemcpyAsync(ws.U0.p, U, 3 * N * sizeof(float), cudaMemcpyDeviceToDevice, s));
     }
-    ws.sums.ensure(sizeof(double) * 64);
-    double *sums = ws.sums.as<double>();
-    auto reduce3 = [&](double out[3]) {
-        launch_reduce_segments(np, 3, part, sums, s, c->launches);
-        check_launch("reduce3");
-        LFRV_CUDA(cudaMemcpyAsync(out, sums, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
-        sync(c);
-    };
-    const float lambda = 1.0f;  // possion_conj_grad: lambda = 1.0 (solver.cu:541)
-    double delta[3];
-    launch_cg_init(W, H, U, gx, gy, r, d, true, part, s, c->launches);
-    check_launch("cg init");
-    reduce3(delta);
-    double dAlpha[3] = {0, 0, 0};
-    const float beta[3] = {1.0f, 1.0f, 1.0f};
-    int it;
-    for (it = 0; it < 5; ++it) {
-        double dq[3], rr[3];
-        launch_cg_apply(W, H, d, lambda, q, part, s, c->launches);
-        check_launch("cg apply");
-        reduce3(dq);
-        float alpha[3];
-        for (int ch = 0; ch < 3; ++ch) {
-            dAlpha[ch] += dq[ch];
-            alpha[ch] = (float)delta[ch] / (float)dAlpha[ch];
-        }
-        launch_cg_update(W, H, alpha, d, q, U, r, part, s, c->launches);
-        check_launch("cg update");
-        reduce3(rr);
-        for (int ch = 0; ch < 3; ++ch) dAlpha[ch] = (double)alpha[ch] + rr[ch];
-        launch_cg_dir(W, H, beta, r, d, s, c->launches);
-        check_launch("cg dir");
+    double *part = partial_buf(c, 8 * npart + (trace ? 3 * (size_t)np : 0));
+    double *state = solver_state(c) + 9;
+    const int step = trace ? 1 : iterations;
+    for (int it = 0; it < iterations; it += step) {
+        const GridBarrier gb = fresh_barrier(c);
+        LFRV_CUDA(launch_cg_faithful(W, H, gx, gy, U, ws.r.as<float>(), ws.d.as<float>(), ws.q.as<float>(), part,
+                                     part + 4 * npart, gb, it, step, state, s, c->launches));
         if (it < trace_cap) {
-            launch_cg_energy(W, H, U, ws.U0.as<float>(), gx, gy, part, s, c->launches);
-            launch_reduce_final(np, part, trace + it, s, c->launches);
+            launch_cg_energy(W, H, U, ws.U0.as<float>(), gx, gy, part + 8 * npart, s, c->launches);
+            launch_reduce_final(np, part + 8 * npart, trace + it, s, c->launches);
             check_launch("cg energy trace");
         }
     }
-    return it;
+    return iterations;
 }
 
 // Corrected CG: one persistent launch (FP32 iterates, FP64 dot products, certified-gap stop on the device).

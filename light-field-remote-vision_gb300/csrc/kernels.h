@@ -169,14 +169,6 @@ void launch_hole_fill_iter(int W, int H, const int *holes, int nholes, const flo
                            double *partial, cudaStream_t st, LaunchCounter &lc);
 int hole_fill_partials(int nholes);
 void launch_hole_list(int W, int H, const uint8_t *vis, int *holes, int *count, cudaStream_t st, LaunchCounter &lc);
-void launch_cg_init(int W, int H, const float *U, const float *gx, const float *gy, float *r, float *d, bool faithful,
-                    double *partial, cudaStream_t st, LaunchCounter &lc);
-void launch_cg_apply(int W, int H, const float *d, float lambda, float *q, double *partial, cudaStream_t st,
-                     LaunchCounter &lc);
-void launch_cg_update(int W, int H, const float alpha[3], const float *d, const float *q, float *U, float *r,
-                      double *partial, cudaStream_t st, LaunchCounter &lc);
-void launch_cg_dir(int W, int H, const float beta[3], const float *r, float *d, cudaStream_t st, LaunchCounter &lc);
-void launch_reduce_segments(int count, int nseg, const double *partial, double *out, cudaStream_t st, LaunchCounter &lc);
 int cg_partials(int W, int H);
 
 // Persistent (cooperative) solvers. The grid barrier's counter and error flag are zeroed before each launch;
@@ -284,6 +276,11 @@ cudaError_t launch_cg_persistent(int W, int H, const float *gx, const float *gy,
 cudaError_t launch_hole_fill_persistent(int W, int H, const int *holes, const int *count, float *A, float *B,
                                         double *part, GridBarrier gb, int max_iter, double *state, cudaStream_t st,
                                         LaunchCounter &lc);
+// Iterations first .. first + count - 1 of the reference's CG loop; r, d, q: 3 N floats each, partA / partB: 4 doubles per
+// block (persistent_partials) each, state: 6 doubles, all kept between the launches of one solve.
+cudaError_t launch_cg_faithful(int W, int H, const float *gx, const float *gy, float *U, float *r, float *d, float *q,
+                               double *partA, double *partB, GridBarrier gb, int first, int count, double *state,
+                               cudaStream_t st, LaunchCounter &lc);
 void launch_cg_energy(int W, int H, const float *U, const float *U0, const float *gx, const float *gy, double *partial,
                       cudaStream_t st, LaunchCounter &lc);
 

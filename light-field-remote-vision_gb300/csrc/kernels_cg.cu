@@ -226,18 +226,6 @@ __device__ __forceinline__ void cg_start_pixel(int W, int H, size_t N, size_t o,
     for (int c = 0; c < 3; ++c) r[c * N + o] = rv[c];
 }
 
-
-__device__ __forceinline__ float cg_op(const float *d, int W, int H, int x, int y, size_t o, float lambda) {
-    float lx, ly;
-    if (x == 0) lx = d[o] - d[o + 1];
-    else if (x < W - 1) lx = 2.f * d[o] - d[o - 1] - d[o + 1];
-    else lx = d[o] - d[o - 1];
-    if (y == 0) ly = d[o] - d[o + W];
-    else if (y < H - 1) ly = 2.f * d[o] - d[o - W] - d[o + W];
-    else ly = d[o] - d[o - W];
-    return lambda * d[o] + lx + ly;
-}
-
 // partial layout: [3][nblocks]
 __device__ __forceinline__ void cg_block3(double a0, double a1, double a2, double *partial) {
     __shared__ double red[3][8];
@@ -268,94 +256,6 @@ __device__ __forceinline__ void cg_block3(double a0, double a1, double a2, doubl
     }
 }
 
-// r0 = b - A x0 (initConjGrad, sources/solver.cu:383-467), d = r0, delta = r0 . r0; faithful counts the last
-// row twice.
-__global__ void __launch_bounds__(256) k_cg_init(int W, int H, const float *__restrict__ U, const float *__restrict__ gX,
-                                                 const float *__restrict__ gY, float *__restrict__ r,
-                                                 float *__restrict__ d, int faithful, double *__restrict__ partial) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    const size_t N = (size_t)W * H;
-    double acc[3] = {0, 0, 0};
-    if (x < W && y < H) {
-        const size_t o = (size_t)y * W + x;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const float *u = U + c * N;
-            float lx, ly;
-            if (x == 0) lx = u[o] - u[o + 1] + gX[o];
-            else if (x < W - 1) lx = 2.f * u[o] - u[o - 1] - u[o + 1] + gX[o] - gX[o - 1];
-            else lx = u[o] - u[o - 1] - gX[o - 1];
-            if (y == 0) ly = u[o] - u[o + W] + gY[o];
-            else if (y < H - 1) ly = 2.f * u[o] - u[o - W] - u[o + W] + gY[o] - gY[o - W];
-            else ly = u[o] - u[o - W] - gY[o - W];
-            const float rv = -(lx + ly);
-            r[c * N + o] = rv;
-            d[c * N + o] = rv;
-            acc[c] = (double)rv * rv * ((faithful && y == H - 1) ? 2.0 : 1.0);
-        }
-    }
-    cg_block3(acc[0], acc[1], acc[2], partial);
-}
-
-// q = A d and d . q per channel.
-__global__ void __launch_bounds__(256) k_cg_apply(int W, int H, const float *__restrict__ d, float lambda,
-                                                  float *__restrict__ q, double *__restrict__ partial) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    const size_t N = (size_t)W * H;
-    double acc[3] = {0, 0, 0};
-    if (x < W && y < H) {
-        const size_t o = (size_t)y * W + x;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const float qv = cg_op(d + c * N, W, H, x, y, o, lambda);
-            q[c * N + o] = qv;
-            acc[c] = (double)d[c * N + o] * qv;
-        }
-    }
-    cg_block3(acc[0], acc[1], acc[2], partial);
-}
-
-// x += alpha d, r -= alpha q, r . r per channel (alpha per channel on the device).
-__global__ void __launch_bounds__(256) k_cg_update(int W, int H, float3 alpha, const float *__restrict__ d, const float *__restrict__ q,
-                                                   float *__restrict__ U, float *__restrict__ r,
-                                                   double *__restrict__ partial) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    const size_t N = (size_t)W * H;
-    double acc[3] = {0, 0, 0};
-    if (x < W && y < H) {
-        const size_t o = (size_t)y * W + x;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const float a = (c == 0) ? alpha.x : (c == 1) ? alpha.y : alpha.z;
-            U[c * N + o] += a * d[c * N + o];
-            const float rv = r[c * N + o] - a * q[c * N + o];
-            r[c * N + o] = rv;
-            acc[c] = (double)rv * rv;
-        }
-    }
-    cg_block3(acc[0], acc[1], acc[2], partial);
-}
-
-__global__ void k_cg_dir(int W, int H, float3 beta, const float *__restrict__ r, float *__restrict__ d) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= W || y >= H) return;
-    const size_t N = (size_t)W * H, o = (size_t)y * W + x;
-    d[o] = r[o] + beta.x * d[o];
-    d[N + o] = r[N + o] + beta.y * d[N + o];
-    d[2 * N + o] = r[2 * N + o] + beta.z * d[2 * N + o];
-}
-
-// Reduces nseg consecutive segments of `count` partials each (one block per segment).
-__global__ void k_reduce_segments(int count, const double *__restrict__ partial, double *__restrict__ out) {
-    __shared__ double red[32];
-    const double *p = partial + (size_t)blockIdx.x * count;
-    double s = 0.0;
-    for (int i = threadIdx.x; i < count; i += blockDim.x) s += p[i];
-    const double t = block_sum<1024>(s, red);
-    if (threadIdx.x == 0) out[blockIdx.x] = t;
-}
-
-// 1/2 ||u - u0||^2 + 1/2 ||grad u - g||^2 summed over channels (FP64), channel-summed partials in slot 0.
 __global__ void __launch_bounds__(256) k_cg_energy(int W, int H, const float *__restrict__ U, const float *__restrict__ U0,
                                                    const float *__restrict__ gX, const float *__restrict__ gY,
                                                    double *__restrict__ partial) {
@@ -473,6 +373,98 @@ __device__ __forceinline__ float ldcg_op(const float *d, int W, int H, int x, in
     else if (y < H - 1) ly = 2.f * c - __ldcg(d + o - W) - __ldcg(d + o + W);
     else ly = c - __ldcg(d + o - W);
     return lambda * c + lx + ly;
+}
+
+// possion_conj_grad's loop (sources/solver.cu:526-699) as the reference runs it, iterations `first` .. first + count - 1
+// in one cooperative launch: beta = 1, the step's denominator dAlpha accumulated over the iterations and receiving
+// alpha + r . r after each, r0 . r0 counting the last row twice. Two grid barriers an iteration: after q = A d with d . q,
+// and after the update of u, r and d with r . r. state: [0..2] r0 . r0, [3..5] dAlpha, carried from launch to launch.
+// Bound by the barriers at small images and by the streams of r, d, q and U at large ones; the scalars stay on the device
+// because a copy back for each (11 of them) cost more than the arithmetic: a whole call with host arrays, 9 views of 256^2,
+// took 607 us with host-stepped kernels and takes 375 us.
+__global__ void __launch_bounds__(kPersistThreads) k_cg_faithful(int W, int H, const float *__restrict__ gX,
+                                                                 const float *__restrict__ gY, float *U, float *r,
+                                                                 float *d, float *q, double *partA, double *partB,
+                                                                 GridBarrier gb, int first, int count, double *state) {
+    __shared__ double sh[4];
+    const size_t N = (size_t)W * H, stride = (size_t)gridDim.x * blockDim.x;
+    const size_t o0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned int gen = 0;
+    double delta[3], dAlpha[3];
+    if (first == 0) {
+        double acc[4] = {0, 0, 0, 0};
+        for (size_t o = o0; o < N; o += stride) {
+            const int y = (int)(o / W), x = (int)(o - (size_t)y * W);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float *u = U + c * N;
+                float lx, ly;
+                if (x == 0) lx = u[o] - u[o + 1] + gX[o];
+                else if (x < W - 1) lx = 2.f * u[o] - u[o - 1] - u[o + 1] + gX[o] - gX[o - 1];
+                else lx = u[o] - u[o - 1] - gX[o - 1];
+                if (y == 0) ly = u[o] - u[o + W] + gY[o];
+                else if (y < H - 1) ly = 2.f * u[o] - u[o - W] - u[o + W] + gY[o] - gY[o - W];
+                else ly = u[o] - u[o - W] - gY[o - W];
+                const float rv = -(lx + ly);
+                r[c * N + o] = rv;
+                d[c * N + o] = rv;
+                acc[c] += (double)rv * rv * (y == H - 1 ? 2.0 : 1.0);
+            }
+        }
+        block_partials(acc, 3, partB, gridDim.x);
+        if (!grid_sync(gb, gen)) return;
+        block_reduce_partials(partB, gridDim.x, 3, sh);
+        for (int c = 0; c < 3; ++c) {
+            delta[c] = sh[c];
+            dAlpha[c] = 0.0;
+        }
+    } else {
+        for (int c = 0; c < 3; ++c) {
+            delta[c] = state[c];
+            dAlpha[c] = state[3 + c];
+        }
+    }
+    for (int it = 0; it < count; ++it) {
+        double acc[4] = {0, 0, 0, 0};
+        for (size_t o = o0; o < N; o += stride) {
+            const int y = (int)(o / W), x = (int)(o - (size_t)y * W);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float qv = ldcg_op(d + c * N, W, H, x, y, o, 1.0f);
+                q[c * N + o] = qv;
+                acc[c] += (double)__ldcg(d + c * N + o) * qv;
+            }
+        }
+        block_partials(acc, 3, partA, gridDim.x);
+        if (!grid_sync(gb, gen)) return;
+        block_reduce_partials(partA, gridDim.x, 3, sh);
+        float alpha[3];
+        for (int c = 0; c < 3; ++c) {
+            dAlpha[c] += sh[c];
+            alpha[c] = (float)delta[c] / (float)dAlpha[c];
+            acc[c] = 0;
+        }
+        for (size_t o = o0; o < N; o += stride) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const size_t i = c * N + o;
+                const float dv = d[i];
+                U[i] += alpha[c] * dv;
+                const float rv = r[i] - alpha[c] * q[i];
+                r[i] = rv;
+                d[i] = rv + dv;
+                acc[c] += (double)rv * rv;
+            }
+        }
+        block_partials(acc, 3, partB, gridDim.x);
+        if (!grid_sync(gb, gen)) return;
+        block_reduce_partials(partB, gridDim.x, 3, sh);
+        for (int c = 0; c < 3; ++c) dAlpha[c] = (double)alpha[c] + sh[c];
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 3) {
+        state[threadIdx.x] = delta[threadIdx.x];
+        state[3 + threadIdx.x] = dAlpha[threadIdx.x];
+    }
 }
 
 // Tiles of the persistent CG: kTileX x kTileY pixels staged with a one-pixel halo.
@@ -1726,6 +1718,18 @@ cudaError_t launch_cg_persistent(int W, int H, const float *gx, const float *gy,
     return cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kPersistThreads), args, smem, st);
 }
 
+cudaError_t launch_cg_faithful(int W, int H, const float *gx, const float *gy, float *U, float *r, float *d, float *q,
+                               double *partA, double *partB, GridBarrier gb, int first, int count, double *state,
+                               cudaStream_t st, LaunchCounter &lc) {
+    ProfScope _ps(lc, "cg_faithful", st);
+    const size_t N = (size_t)W * H;
+    const int want = (int)std::min<size_t>((N + kPersistThreads - 1) / kPersistThreads, 1 << 20);
+    const int blocks = coop_blocks((const void *)k_cg_faithful, want);
+    void *args[] = {&W, &H, (void *)&gx, (void *)&gy, &U, &r, &d, &q, &partA, &partB, &gb, &first, &count, &state};
+    lc.add(1);
+    return cudaLaunchCooperativeKernel((const void *)k_cg_faithful, dim3(blocks), dim3(kPersistThreads), args, 0, st);
+}
+
 int cg_batch_resident_blocks() { return strip_sms(); }
 
 int cg_batch_blocks(int W, int H, int R) { return strip_fits(W, H, R) ? strip_blocks(W, H, R) : 0; }
@@ -1865,39 +1869,6 @@ void launch_hole_fill_iter(int W, int H, const int *holes, int nholes, const flo
     ProfScope _ps(lc, "hole_fill_iter", st);
     if (nholes <= 0) return;
     k_hole_iter<<<(nholes + 255) / 256, 256, 0, st>>>(W, H, holes, nholes, Uin, Uout, partial);
-    lc.add(1);
-}
-
-void launch_cg_init(int W, int H, const float *U, const float *gx, const float *gy, float *r, float *d, bool faithful,
-                    double *partial, cudaStream_t st, LaunchCounter &lc) {
-    ProfScope _ps(lc, "cg_init", st);
-    k_cg_init<<<cg_grid(W, H), dim3(kCgBX, kCgBY), 0, st>>>(W, H, U, gx, gy, r, d, faithful ? 1 : 0, partial);
-    lc.add(1);
-}
-
-void launch_cg_apply(int W, int H, const float *d, float lambda, float *q, double *partial, cudaStream_t st,
-                     LaunchCounter &lc) {
-    k_cg_apply<<<cg_grid(W, H), dim3(kCgBX, kCgBY), 0, st>>>(W, H, d, lambda, q, partial);
-    lc.add(1);
-}
-
-void launch_cg_update(int W, int H, const float alpha[3], const float *d, const float *q, float *U, float *r,
-                      double *partial, cudaStream_t st, LaunchCounter &lc) {
-    ProfScope _ps(lc, "cg_update", st);
-    k_cg_update<<<cg_grid(W, H), dim3(kCgBX, kCgBY), 0, st>>>(W, H, make_float3(alpha[0], alpha[1], alpha[2]), d, q, U,
-                                                             r, partial);
-    lc.add(1);
-}
-
-void launch_cg_dir(int W, int H, const float beta[3], const float *r, float *d, cudaStream_t st, LaunchCounter &lc) {
-    ProfScope _ps(lc, "cg_dir", st);
-    k_cg_dir<<<cg_grid(W, H), dim3(kCgBX, kCgBY), 0, st>>>(W, H, make_float3(beta[0], beta[1], beta[2]), r, d);
-    lc.add(1);
-}
-
-void launch_reduce_segments(int count, int nseg, const double *partial, double *out, cudaStream_t st, LaunchCounter &lc) {
-    ProfScope _ps(lc, "reduce_segments", st);
-    k_reduce_segments<<<nseg, 1024, 0, st>>>(count, partial, out);
     lc.add(1);
 }
 
