@@ -30,7 +30,7 @@ namespace lfrv {
 
 namespace {
 
-constexpr int kBM = 128, kBK = 64, kThreads = 128, kStages = 4, kWgStages = 2;
+constexpr int kBM = 128, kBK = 64, kThreads = 128, kStages = 4;
 
 // Shared-memory matrix descriptor: start >> 4 in bits 0-13, leading byte offset >> 4 in 16-29, stride byte
 // offset >> 4 in 32-45, the fixed version field (1) in 46-47, base offset 0, layout type 0 (no swizzle).
@@ -43,7 +43,8 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo = 128
 }
 
 // Instruction descriptor of kind::f16: D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9 = 1, 10-12 = 1), both
-// K-major (bits 15, 16 = 0), N >> 3 in bits 17-22, M >> 4 in bits 24-28.
+// K-major (bits 15, 16 = 0; kMnMajor sets both), N >> 3 in bits 17-22, M >> 4 in bits 24-28.
+constexpr uint32_t kMnMajor = (1u << 15) | (1u << 16);
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
@@ -616,15 +617,25 @@ __global__ void __launch_bounds__(kThreads) k_conv_tma(const ConvGemm g, const _
 }
 
 // Weight gradient: GEMM rows are the (tap, ci) rows of dW^T (padded to 128), N = the stored output channels, the
-// reduction runs over the output pixels of this split. Both operands are pixel-major in global memory, so each
-// 16-byte load (8 channels of one pixel) is written transposed into a column of a core matrix. Double-buffered:
-// the global loads of stage k overlap the MMAs of stage k - 1. Result: FP32 partial[split][row][co].
+// reduction runs over the output pixels of this split. Both operands are pixel-major in global memory, that is
+// MN-major: eight channels of one pixel are one 16-byte row of a core matrix (8 pixels x 8 channels), so a gather is
+// one 16-byte cp.async and nothing is transposed. Core matrices adjacent in channels lie kWgSbo apart (stride byte
+// offset; 128 B and 32 of padding, which spreads a quarter warp's four chunks of two pixels over all banks), 8-pixel
+// blocks one row of those apart (leading byte offset). Stages of 64 pixels run through a ring of cp.async groups as in
+// k_conv_tc; its depth leaves two CTAs an SM up to 128 columns. Bound by the gather's L1 and L2 traffic (every input
+// pixel is read once a tap). Four 256^2 images, twelve layers: 691 us with 2-byte transposing stores and one stage in
+// flight, 333 us now. Result: FP32 partial[split][row][co].
+constexpr int kWgSbo = 160;
+__host__ __device__ constexpr int wg_stage_bytes(int BN) { return 8 * kWgSbo * (kBM / 8 + BN / 8); }
+__host__ __device__ constexpr int wg_stages(int BN) { return BN <= 32 ? 4 : BN == 64 ? 3 : BN == 128 ? 2 : 3; }
+
 template <int BN>
 __global__ void __launch_bounds__(kThreads) k_wgrad_tc(const WgradGemm g, int *err) {
     extern __shared__ uint8_t dsm[];
-    constexpr int kAB = kBM * kBK * 2, kStage = kAB + BN * kBK * 2;
+    constexpr int kWgStages = wg_stages(BN), kStage = wg_stage_bytes(BN);
+    constexpr int kLboA = kBM / 8 * kWgSbo, kLboB = BN / 8 * kWgSbo, kA = 8 * kLboA;
     constexpr int kCols = BN < 32 ? 32 : BN;
-    constexpr int kBChunks = BN / 16;  // per thread
+    constexpr int kBC = BN < 32 ? 2 : 4;  // dY chunks that adjacent threads take
     __shared__ __align__(8) uint64_t bars[kWgStages];
     __shared__ uint32_t tmem_slot;
     __shared__ int s_fail;
@@ -639,102 +650,90 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_tc(const WgradGemm g, int *e
         s_fail = 0;
         fence_proxy_async_smem();
     }
-    const int pk = tid & 63, grp = tid >> 6;  // this thread's pixel column and first 8-row group
-    // rows of the A chunks: group G = grp + 2 j holds rows m0 + 8 G .. + 7 = 8 channels of one tap
-    int atap[8], aci[8];
+    // this thread's four X chunks (8 channels of one tap each): channel block 4 q + (tid & 3) of the tile
+    int ady[4], adx[4], aci[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int r0 = m0 + (grp + 2 * j) * 8;
-        if (r0 < g.Kf) {
-            atap[j] = r0 / g.Cin;
-            aci[j] = r0 - atap[j] * g.Cin;
-        } else {
-            atap[j] = -1;
-            aci[j] = 0;
-        }
+    for (int q = 0; q < 4; ++q) {
+        const int r0 = m0 + (4 * q + (tid & 3)) * 8;
+        const int tap = r0 / g.Cin;
+        aci[q] = r0 < g.Kf ? r0 - tap * g.Cin : -1;
+        ady[q] = g.ks == 3 ? tap / 3 - 1 : 0;
+        adx[q] = g.ks == 3 ? tap - (tap / 3) * 3 - 1 : 0;
     }
     const __nv_bfloat16 *X = static_cast<const __nv_bfloat16 *>(g.x);
     const __nv_bfloat16 *DY = static_cast<const __nv_bfloat16 *>(g.dy);
     const uint32_t sbase = smem_u32(base);
+    auto load_stage = [&](int kt, int slot) {
+        const uint32_t sa = sbase + slot * kStage, sb = sa + kA;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int pk = (tid >> 2) + 32 * h, p = p0 + kt * kBK + pk;
+            const bool pv = p < p1;
+            const int b = p / HWo, rem = p - b * HWo, oy = rem / g.Wo, ox = rem - oy * g.Wo;
+            const int y0 = oy * g.stride, x0 = ox * g.stride;
+            const size_t img = (size_t)b * g.Hx * g.Wx;
+            const uint32_t dst = sa + (uint32_t)((pk >> 3) * kLboA + (tid & 3) * kWgSbo + ((pk & 7) << 4));
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int iy = y0 + ady[q], ix = x0 + adx[q];
+                const bool ok = pv && aci[q] >= 0 && iy >= 0 && iy < g.Hx && ix >= 0 && ix < g.Wx;
+                const __nv_bfloat16 *src = ok ? X + (img + (size_t)iy * g.Wx + ix) * g.Cin + aci[q] : X;
+                cp_async16(dst + q * 4 * kWgSbo, src, ok ? 16 : 0);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < BN / 16; ++j) {
+            const int i = tid + kThreads * j, c = i % kBC + kBC * (i / (kBC * kBK)), pk = i / kBC % kBK;
+            const int p = p0 + kt * kBK + pk;
+            const bool pv = p < p1;
+            cp_async16(sb + (uint32_t)((pk >> 3) * kLboB + c * kWgSbo + ((pk & 7) << 4)),
+                       pv ? DY + (size_t)p * g.Cout + c * 8 : DY, pv ? 16 : 0);
+        }
+    };
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    const uint32_t idesc = idesc_bf16_f32(kBM, BN);
+    const uint32_t idesc = idesc_bf16_f32(kBM, BN) | kMnMajor;
     const int nk = (p1 - p0 + kBK - 1) / kBK;
+#pragma unroll 1
+    for (int s = 0; s < kWgStages - 1; ++s) {
+        if (s < nk) load_stage(s, s);
+        cp_async_commit();
+    }
     int issued = 0;
 #pragma unroll 1
     for (int kt = 0; kt < nk; ++kt) {
         const int slot = kt % kWgStages;
-        // global loads of this stage (registers)
-        const int p = p0 + kt * kBK + pk;
-        const bool pv = p < p1;
-        int b = 0, oy = 0, ox = 0;
-        if (pv) {
-            b = p / HWo;
-            const int rem = p - b * HWo;
-            oy = rem / g.Wo;
-            ox = rem - oy * g.Wo;
-        }
-        uint4 va[8], vb[kBChunks];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            va[j] = make_uint4(0, 0, 0, 0);
-            if (pv && atap[j] >= 0) {
-                int iy = oy * g.stride, ix = ox * g.stride;
-                if (g.ks == 3) {
-                    const int ky = atap[j] / 3;
-                    iy += ky - 1;
-                    ix += atap[j] - ky * 3 - 1;
-                }
-                if (iy >= 0 && iy < g.Hx && ix >= 0 && ix < g.Wx)
-                    va[j] = __ldg(reinterpret_cast<const uint4 *>(X + ((size_t)b * g.Hx * g.Wx + (size_t)iy * g.Wx + ix) * g.Cin + aci[j]));
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < kBChunks; ++j) {
-            vb[j] = make_uint4(0, 0, 0, 0);
-            if (pv) vb[j] = __ldg(reinterpret_cast<const uint4 *>(DY + (size_t)p * g.Cout + (grp + 2 * j) * 8));
-        }
-        // the slot was last read by the MMAs of stage kt - 2
-        if (kt >= kWgStages) {
-            if (!mbar_wait(&bars[slot], ((kt - kWgStages) / kWgStages) & 1, kSpinLimit)) {
-                s_fail = 1;
-                atomicExch(err, 1);
-            }
-        }
-        tc_fence_before();
-        __syncthreads();
-        if (s_fail) break;
-        uint8_t *sa = base + slot * kStage, *sb = sa + kAB;
-        const int colb = ((pk >> 3) << 7) + ((pk & 7) << 1);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint16_t *h = reinterpret_cast<const uint16_t *>(&va[j]);
-            uint8_t *dst = sa + ((grp + 2 * j) << 10) + colb;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) *reinterpret_cast<uint16_t *>(dst + (i << 4)) = h[i];
-        }
-#pragma unroll
-        for (int j = 0; j < kBChunks; ++j) {
-            const uint16_t *h = reinterpret_cast<const uint16_t *>(&vb[j]);
-            uint8_t *dst = sb + ((grp + 2 * j) << 10) + colb;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) *reinterpret_cast<uint16_t *>(dst + (i << 4)) = h[i];
-        }
+        cp_async_wait<kWgStages - 2>();  // stage kt has landed
         fence_proxy_async_smem();
         tc_fence_before();
         __syncthreads();
         tc_fence_after();
+        if (s_fail) break;
         if (tid == 0) {
-            const uint32_t a = sbase + slot * kStage, bb = a + kAB;
+            const uint32_t a = sbase + slot * kStage, bb = a + kA;
 #pragma unroll
             for (int s = 0; s < kBK / 16; ++s)
-                tc_mma(tmem, smem_desc(a + s * 256), smem_desc(bb + s * 256), idesc, (kt > 0 || s > 0) ? 1 : 0);
+                tc_mma(tmem, smem_desc(a + s * 2 * kLboA, kLboA, kWgSbo), smem_desc(bb + s * 2 * kLboB, kLboB, kWgSbo),
+                       idesc, (kt > 0 || s > 0) ? 1 : 0);
             tc_commit(&bars[slot]);
         }
         issued = kt + 1;
+        const int nxt = kt + kWgStages - 1;
+        if (nxt < nk) {
+            // the slot of stage kt - 1 is free once its MMAs have completed
+            bool ok = true;
+            if (kt >= 1) ok = mbar_wait(&bars[(kt - 1) % kWgStages], ((kt - 1) / kWgStages) & 1, kSpinLimit);
+            if (ok) load_stage(nxt, nxt % kWgStages);
+            else {
+                s_fail = 1;
+                atomicExch(err, 1);
+            }
+        }
+        cp_async_commit();
     }
+    cp_async_wait<0>();
     bool done = true;
     if (issued > 0) done = mbar_wait(&bars[(issued - 1) % kWgStages], ((issued - 1) / kWgStages) & 1, kSpinLimit);
     if (!done) {
@@ -1107,7 +1106,7 @@ cudaError_t launch_conv_tc(const ConvGemm &g, int *err, cudaStream_t st, LaunchC
 
 template <int BN>
 static cudaError_t wgrad_launch(const WgradGemm &g, int splits, int *err, cudaStream_t st) {
-    constexpr int smem = kWgStages * (kBM * kBK * 2 + BN * kBK * 2) + 1024;
+    constexpr int smem = wg_stages(BN) * wg_stage_bytes(BN) + 1024;
     static bool attr = false;
     if (!attr) {
         const cudaError_t e = cudaFuncSetAttribute(k_wgrad_tc<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
