@@ -322,10 +322,9 @@ cudaError_t launch_conv_tc(const ConvGemm &g, int *err, cudaStream_t st, LaunchC
 // Kernel choice of launch_conv_tc: 0 TMA / resident tile / gather as they apply, 1 without the TMA kernel, 2 the
 // gather kernel only (process-wide).
 void set_conv_kernel_pref(int pref);
-cudaError_t launch_wgrad_tc(const WgradGemm &g, int splits, int Cout_real, float *grad, int *err, cudaStream_t st,
-                            LaunchCounter &lc);
-cudaError_t launch_bias_grad(int P, int C, int Creal, const void *dy, float *partial, int blocks, float *out,
-                             cudaStream_t st, LaunchCounter &lc);
+// dW into grad and, unless bias_out is null, db = the column sums of dy (bias_partial: bias_blocks x Cout floats).
+cudaError_t launch_wgrad_tc(const WgradGemm &g, int splits, int Cout_real, float *grad, float *bias_partial,
+                            int bias_blocks, float *bias_out, int *err, cudaStream_t st, LaunchCounter &lc);
 cudaError_t launch_upsample_add_relu(int batch, int Hl, int Wl, int C, const void *t, const void *skip, void *s,
                                      cudaStream_t st, LaunchCounter &lc);
 cudaError_t launch_down_sum(int batch, int Hl, int Wl, int C, const void *ds, void *dt, cudaStream_t st,

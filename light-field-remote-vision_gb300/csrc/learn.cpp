@@ -90,7 +90,7 @@ namespace lfrv {
 
 namespace {
 
-constexpr int kBiasBlocks = 152;
+constexpr int kBiasBlocks = 304;
 constexpr int kLossBlocks = 304;
 constexpr size_t kParamSlack = 256;  // zeros after the last bias: the padded output head reads 16 bias values
 
@@ -245,9 +245,8 @@ void conv_wgrad(lfrv_warmstart *net, int l, const void *x, int level, const void
     net->partial.ensure((size_t)splits * g.Mpad * L.cst * sizeof(float));
     g.partial = net->partial.as<float>();
     float *grad = net->grads.as<float>();
-    LFRV_CUDA(launch_wgrad_tc(g, splits, L.d.cout, grad + L.w_off, net_err(net), c->stream, c->launches));
-    LFRV_CUDA(launch_bias_grad(P, L.cst, L.d.cout, dy, net->bias_part.as<float>(), kBiasBlocks, grad + L.b_off,
-                               c->stream, c->launches));
+    LFRV_CUDA(launch_wgrad_tc(g, splits, L.d.cout, grad + L.w_off, net->bias_part.as<float>(), kBiasBlocks,
+                              grad + L.b_off, net_err(net), c->stream, c->launches));
 }
 
 void forward(lfrv_warmstart *net, const void *in) {
@@ -433,7 +432,7 @@ static void conv_single(lfrv_ctx *c, int mode, int batch, int Hin, int Win, int 
         splits = (P + g.chunk - 1) / g.chunk;
         part.ensure((size_t)splits * g.Mpad * Cout * sizeof(float));
         g.partial = part.as<float>();
-        LFRV_CUDA(launch_wgrad_tc(g, splits, Cout, out, err.as<int>(), c->stream, c->launches));
+        LFRV_CUDA(launch_wgrad_tc(g, splits, Cout, out, nullptr, 0, nullptr, err.as<int>(), c->stream, c->launches));
     }
     int e = 0;
     LFRV_CUDA(cudaMemcpyAsync(&e, err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
