@@ -501,6 +501,11 @@ __global__ void __launch_bounds__(kThreads) k_conv_tile_tc(const ConvGemm g, int
 // stage, issues its four K = 16 MMAs and commits them to the stage's empty mbarrier, which releases the slot to the
 // producer. After the last stage the MMA thread commits to `done`, and the four warps read the accumulator.
 // Forward convolutions of stride 1 or 2 (3 x 3 or 1 x 1) and the data gradient of stride-1 layers (taps mirrored).
+// The data gradient of a stride-2 3 x 3 layer (PARITY) is four convolutions of stride 1 on the output gradient's grid,
+// one for each parity of the input pixel (blockIdx.z, the one with most taps first): of the nine taps an even
+// coordinate meets only the middle one and an odd one the outer two, 1, 2, 2 and 4 taps instead of nine with three
+// quarters zeros. The sums skip exact zeros only, in the order of the taps. Layers 1 to 3 of four 256^2 images: 131, 86
+// and 68 us with the gather kernel, 54, 31 and 21 us now.
 constexpr int kTmaStages = 4;
 
 // K-major operand in the 128-byte swizzle: 128-byte rows (64 bf16), 8-row atoms of 1 KB (stride byte offset),
@@ -514,7 +519,7 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
     return d;
 }
 
-template <int BN>
+template <int BN, bool PARITY>
 __global__ void __launch_bounds__(kThreads) k_conv_tma(const ConvGemm g, const __grid_constant__ CUtensorMap mapA,
                                                        const __grid_constant__ CUtensorMap mapB, int bw, int bh,
                                                        int cblocks, int *err) {
@@ -526,13 +531,15 @@ __global__ void __launch_bounds__(kThreads) k_conv_tma(const ConvGemm g, const _
     __shared__ int s_fail;
     uint8_t *base = align1024(dsm);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int pxn = g.Wo / bw, pyn = g.Ho / bh;
+    const int gw = PARITY ? g.Ws : g.Wo, gh = PARITY ? g.Hs : g.Ho;  // the grid that is cut into patches
+    const int pxn = gw / bw, pyn = gh / bh;
     int blk = blockIdx.x;
     const int pxi = blk % pxn;
     blk /= pxn;
     const int pyi = blk % pyn, b = blk / pyn;
     const int ox0 = pxi * bw, oy0 = pyi * bh, n0 = blockIdx.y * BN;
-    const int nk = g.ks * g.ks * cblocks;
+    const int odd_y = PARITY ? 1 - (int)(blockIdx.z >> 1) : 0, odd_x = PARITY ? 1 - (int)(blockIdx.z & 1) : 0;
+    const int nk = (PARITY ? (1 + odd_y) * (1 + odd_x) : g.ks * g.ks) * cblocks;
     if (warp == 0) tmem_alloc(&tmem_slot, kCols);
     if (tid == 0) {
         for (int s = 0; s < kTmaStages; ++s) {
@@ -556,9 +563,16 @@ __global__ void __launch_bounds__(kThreads) k_conv_tma(const ConvGemm g, const _
                 atomicExch(err, 1);
                 break;
             }
-            const int tap = kt / cblocks, cb = kt - tap * cblocks;
+            int tap = kt / cblocks;
+            const int cb = kt - tap * cblocks;
             int sx = ox0 * g.stride, sy = oy0 * g.stride;
-            if (g.ks == 3) {
+            if constexpr (PARITY) {
+                // tap 0 or 2 along an odd coordinate (source one on, or in place), tap 1 along an even one
+                const int ty = tap >> odd_x, tx = tap & odd_x;
+                sx = ox0 + (odd_x & (tx ^ 1));
+                sy = oy0 + (odd_y & (ty ^ 1));
+                tap = 3 * (odd_y ? 2 * ty : 1) + (odd_x ? 2 * tx : 1);
+            } else if (g.ks == 3) {
                 const int ky = tap / 3, kx = tap - 3 * (tap / 3);
                 if (!g.dgrad) {
                     sx += kx - 1;
@@ -602,7 +616,11 @@ __global__ void __launch_bounds__(kThreads) k_conv_tma(const ConvGemm g, const _
     tc_fence_after();
     if (!s_fail) {
         const int m = warp * 32 + lane;
-        const int oy = oy0 + m / bw, ox = ox0 + m % bw;
+        int oy = oy0 + m / bw, ox = ox0 + m % bw;
+        if constexpr (PARITY) {
+            oy = 2 * oy + odd_y;
+            ox = 2 * ox + odd_x;
+        }
         const size_t row = ((size_t)b * g.Ho + oy) * g.Wo + ox;
 #pragma unroll 1
         for (int c0 = 0; c0 < BN; c0 += 16) {
@@ -1025,21 +1043,30 @@ static cudaError_t launch_tile(const ConvGemm &g, int R, int BN, int smem, int *
     return cudaErrorInvalidValue;
 }
 
-// Patch of the TMA kernel (bw x bh = 128 output pixels), or false when the layer does not tile that way or is a
-// data gradient of stride 2.
+// The data gradient of a stride-2 layer that k_conv_tma takes by parity: an even image, so that every parity has the
+// output gradient's grid, and whole 64-channel blocks, so that a tap's box holds no other tap's weights. Everything
+// else of stride 2 (one row more or less, 1 x 1, 16 or 32 channels) is the gather kernel's.
+static bool tma_parity(const ConvGemm &g) {
+    return g.dgrad && g.stride == 2 && g.ks == 3 && g.C % 64 == 0 && g.Ho == 2 * g.Hs && g.Wo == 2 * g.Ws;
+}
+
+// Patch of the TMA kernel (bw x bh = 128 pixels of the grid it runs over), or false when the layer does not tile that
+// way.
 static bool tma_shape(const ConvGemm &g, int &bw, int &bh) {
     if (g.ks != 1 && g.ks != 3) return false;
-    if (g.dgrad && g.stride != 1) return false;
+    const bool parity = tma_parity(g);
+    if (g.dgrad && g.stride != 1 && !parity) return false;
     if (g.C % 8 || g.C < 8) return false;
-    if (g.Wo >= 128) {
-        if (g.Wo % 128) return false;
+    const int gw = parity ? g.Ws : g.Wo, gh = parity ? g.Hs : g.Ho;
+    if (gw >= 128) {
+        if (gw % 128) return false;
         bw = 128;
         bh = 1;
     } else {
-        if (128 % g.Wo) return false;
-        bw = g.Wo;
-        bh = 128 / g.Wo;
-        if (g.Ho % bh) return false;
+        if (128 % gw) return false;
+        bw = gw;
+        bh = 128 / gw;
+        if (gh % bh) return false;
     }
     const int s = g.dgrad ? 1 : g.stride;
     return bw * s <= 256 && bh * s <= 256;
@@ -1068,20 +1095,33 @@ static bool encode_conv_maps(const ConvGemm &g, int bw, int bh, int BN, CUtensor
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN>
+template <int BN, bool PARITY>
 static cudaError_t tma_launch(const ConvGemm &g, int bw, int bh, const CUtensorMap &mA, const CUtensorMap &mB, int *err,
                               cudaStream_t st) {
     constexpr int smem = kTmaStages * (kBM * 128 + BN * 128) + 1024;
     static bool attr = false;
     if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(k_conv_tma<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaError_t e =
+            cudaFuncSetAttribute(k_conv_tma<BN, PARITY>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    const int cblocks = (g.C + 63) / 64;
-    const dim3 grid(g.batch * (g.Ho / bh) * (g.Wo / bw), g.N / BN);
-    k_conv_tma<BN><<<grid, kThreads, smem, st>>>(g, mA, mB, bw, bh, cblocks, err);
+    const int cblocks = (g.C + 63) / 64, parities = PARITY ? 4 : 1;
+    const dim3 grid(g.batch * (g.Ho * g.Wo / parities) / (bh * bw), g.N / BN, parities);
+    k_conv_tma<BN, PARITY><<<grid, kThreads, smem, st>>>(g, mA, mB, bw, bh, cblocks, err);
     return cudaGetLastError();
+}
+
+template <bool PARITY>
+static cudaError_t launch_tma(const ConvGemm &g, int bn, int bw, int bh, const CUtensorMap &mA, const CUtensorMap &mB,
+                              int *err, cudaStream_t st) {
+    switch (bn) {
+        case 16: return tma_launch<16, PARITY>(g, bw, bh, mA, mB, err, st);
+        case 32: return tma_launch<32, PARITY>(g, bw, bh, mA, mB, err, st);
+        case 64: return tma_launch<64, PARITY>(g, bw, bh, mA, mB, err, st);
+        case 128: return tma_launch<128, PARITY>(g, bw, bh, mA, mB, err, st);
+        default: return tma_launch<256, PARITY>(g, bw, bh, mA, mB, err, st);
+    }
 }
 
 // Which convolution kernel a layer uses: the TMA kernel where its patch tiling applies, else the resident-tile
@@ -1111,19 +1151,13 @@ cudaError_t launch_conv_tc(const ConvGemm &g, int *err, cudaStream_t st, LaunchC
         int bn = g.N;
         const bool tma = pref == 0 && tma_shape(g, bw, bh);
         if (tma) {
-            const int mtiles = g.batch * (g.Ho / bh) * (g.Wo / bw);
+            const int mtiles = g.batch * g.Ho * g.Wo / kBM;
             while (bn > 32 && mtiles * (g.N / bn) < 120) bn >>= 1;
         }
         // a map the driver does not accept sends the layer to the other kernels
         if (tma && encode_conv_maps(g, bw, bh, bn, &mA, &mB)) {
-            cudaError_t e;
-            switch (bn) {
-                case 16: e = tma_launch<16>(g, bw, bh, mA, mB, err, st); break;
-                case 32: e = tma_launch<32>(g, bw, bh, mA, mB, err, st); break;
-                case 64: e = tma_launch<64>(g, bw, bh, mA, mB, err, st); break;
-                case 128: e = tma_launch<128>(g, bw, bh, mA, mB, err, st); break;
-                default: e = tma_launch<256>(g, bw, bh, mA, mB, err, st); break;
-            }
+            const cudaError_t e = tma_parity(g) ? launch_tma<true>(g, bn, bw, bh, mA, mB, err, st)
+                                                : launch_tma<false>(g, bn, bw, bh, mA, mB, err, st);
             lc.add(1);
             return e;
         }
