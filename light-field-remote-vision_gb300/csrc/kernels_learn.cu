@@ -152,69 +152,93 @@ __device__ __forceinline__ bool conv_src(const ConvGemm &g, int y, int x, int ky
     return iy >= 0 && iy < g.Hs && ix >= 0 && ix < g.Ws;
 }
 
+// What the epilogue of 16 columns reads besides the accumulator: the skip values of a 2 x 2 block ([2 d], [2 d + 1] for
+// pixel d) with upskip (UP), else the addend ([0], [1]) and the mask ([2], [3]). Loaded ahead of the accumulator, so that its
+// latency passes during the matrix products.
+template <bool UP>
+struct EpilogueIn {
+    uint4 u[UP ? 8 : 4];
+};
+
+__device__ __forceinline__ size_t upskip_row(const ConvGemm &g, size_t row, int d) {
+    const size_t HW = (size_t)g.Ho * g.Wo, b = row / HW, rem = row - b * HW;
+    const int y = (int)(rem / g.Wo), x = (int)(rem - (size_t)y * g.Wo);
+    return (b * 2 * g.Ho + 2 * y + (d >> 1)) * (size_t)(2 * g.Wo) + 2 * x + (d & 1);
+}
+
+template <bool UP>
+__device__ __forceinline__ void conv_load16(const ConvGemm &g, size_t row, int col, EpilogueIn<UP> &in) {
+    if constexpr (UP) {
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+            const uint4 *sp = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(g.upskip) +
+                                                              upskip_row(g, row, d) * g.N + col);
+            in.u[2 * d] = __ldg(sp);
+            in.u[2 * d + 1] = __ldg(sp + 1);
+        }
+        return;
+    }
+    const size_t o = row * g.N + col;
+    if (g.add) {
+        const uint4 *ap = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(g.add) + o);
+        in.u[0] = __ldg(ap);
+        in.u[1] = __ldg(ap + 1);
+    }
+    if (g.mask) {
+        const uint4 *mp = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(g.mask) + o);
+        in.u[2] = __ldg(mp);
+        in.u[3] = __ldg(mp + 1);
+    }
+}
+
 // Epilogue of 16 accumulator columns (col .. col + 15) of GEMM row `row` (an output pixel, row-major over batch,
-// Ho, Wo): + bias, + add, ReLU, zero where mask <= 0, then the FP32 and / or BF16 stores. With upskip the row's
-// value goes, as relu(v + skip), to its 2 x 2 block of the doubled-resolution BF16 output.
-__device__ __forceinline__ void conv_store16(const ConvGemm &g, size_t row, int col, float v[16]) {
+// Ho, Wo): + bias, + add, ReLU, zero where mask <= 0, then the FP32 and / or BF16 stores. With upskip (and no addend)
+// the row's value goes, as relu(v + skip), to its 2 x 2 block of the doubled-resolution BF16 output.
+template <bool UP>
+__device__ __forceinline__ void conv_store16(const ConvGemm &g, size_t row, int col, float v[16],
+                                             const EpilogueIn<UP> &in) {
     const size_t o = row * g.N + col;
     if (g.bias) {
 #pragma unroll
         for (int k = 0; k < 16; ++k) v[k] += __ldg(g.bias + col + k);
     }
-    if (g.add) {
-        const uint4 *ap = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(g.add) + o);
-        float tt[8];
-        unpack8(ap[0], tt);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] += tt[k];
-        unpack8(ap[1], tt);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) v[8 + k] += tt[k];
-    }
-    if (g.upskip) {
-        const size_t HW = (size_t)g.Ho * g.Wo;
-        const size_t b = row / HW, rem = row - b * HW;
-        const int y = (int)(rem / g.Wo), x = (int)(rem - (size_t)y * g.Wo);
-        const __nv_bfloat16 *sk = static_cast<const __nv_bfloat16 *>(g.upskip);
+    if constexpr (UP) {
         __nv_bfloat16 *out = static_cast<__nv_bfloat16 *>(g.outb);
-        size_t oo[4];
-        uint4 sv[8];
-        // all eight skip loads in flight before the first store
-#pragma unroll
-        for (int d = 0; d < 4; ++d) {
-            const size_t hr = (b * 2 * g.Ho + 2 * y + (d >> 1)) * (size_t)(2 * g.Wo) + 2 * x + (d & 1);
-            oo[d] = hr * g.N + col;
-            const uint4 *sp = reinterpret_cast<const uint4 *>(sk + oo[d]);
-            sv[2 * d] = __ldg(sp);
-            sv[2 * d + 1] = __ldg(sp + 1);
-        }
 #pragma unroll
         for (int d = 0; d < 4; ++d) {
             float a[8], c[8], w0[8], w1[8];
-            unpack8(sv[2 * d], a);
-            unpack8(sv[2 * d + 1], c);
+            unpack8(in.u[2 * d], a);
+            unpack8(in.u[2 * d + 1], c);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
                 w0[k] = fmaxf(v[k] + a[k], 0.f);
                 w1[k] = fmaxf(v[8 + k] + c[k], 0.f);
             }
-            uint4 *bp = reinterpret_cast<uint4 *>(out + oo[d]);
+            uint4 *bp = reinterpret_cast<uint4 *>(out + upskip_row(g, row, d) * g.N + col);
             bp[0] = pack8(w0);
             bp[1] = pack8(w1);
         }
         return;
+    }
+    if (g.add) {
+        float tt[8];
+        unpack8(in.u[0], tt);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] += tt[k];
+        unpack8(in.u[1], tt);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[8 + k] += tt[k];
     }
     if (g.relu) {
 #pragma unroll
         for (int k = 0; k < 16; ++k) v[k] = fmaxf(v[k], 0.f);
     }
     if (g.mask) {
-        const uint4 *mp = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(g.mask) + o);
         float tt[8];
-        unpack8(mp[0], tt);
+        unpack8(in.u[2], tt);
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = tt[k] > 0.f ? v[k] : 0.f;
-        unpack8(mp[1], tt);
+        unpack8(in.u[3], tt);
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[8 + k] = tt[k] > 0.f ? v[8 + k] : 0.f;
     }
@@ -235,7 +259,7 @@ __device__ __forceinline__ void conv_store16(const ConvGemm &g, size_t row, int 
 // One CTA: 128 GEMM rows (pixels) x BN output channels (columns n0 = blockIdx.y * BN ..), K in 64-wide stages through a kStages-deep
 // cp.async ring. Thread 0 issues the four K = 16 MMAs of a stage once the stage has landed and commits them to
 // the stage's mbarrier; a slot is refilled only after the mbarrier shows that the MMAs reading it completed.
-template <int BN>
+template <int BN, bool UP>
 __global__ void __launch_bounds__(kThreads) k_conv_tc(const ConvGemm g, int *err) {
     extern __shared__ uint8_t dsm[];
     constexpr int kAB = kBM * kBK * 2, kStage = kAB + BN * kBK * 2;
@@ -354,9 +378,11 @@ __global__ void __launch_bounds__(kThreads) k_conv_tc(const ConvGemm g, int *err
 #pragma unroll 1
         for (int c0 = 0; c0 < BN; c0 += 16) {
             float v[16];
+            EpilogueIn<UP> in;
+            if (row_ok) conv_load16(g, (size_t)m, n0 + c0, in);
             tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
             if (!row_ok) continue;
-            conv_store16(g, (size_t)m, n0 + c0, v);
+            conv_store16(g, (size_t)m, n0 + c0, v, in);
         }
     }
     tc_fence_before();
@@ -372,11 +398,12 @@ __global__ void __launch_bounds__(kThreads) k_conv_tc(const ConvGemm g, int *err
 // instead of nine gathers. The weights stream per tap through a 3-slot cp.async ring. TMEM: R accumulators of BN
 // columns. Needs W % 128 == 0, H % R == 0, C % 16 == 0.
 constexpr int kTileW = 130, kTapStages = 3;
+constexpr int kEpiThreads = 256;  // two groups of four warps share an epilogue (a warp reads TMEM lanes 32 (w % 4) ..)
 
 __host__ __device__ constexpr int tile_lbo_px(int R) { return ((R + 2) * kTileW) | 1; }  // odd: spreads the banks
 
 template <int BN, int R>
-__global__ void __launch_bounds__(kThreads) k_conv_tile_tc(const ConvGemm g, int *err) {
+__global__ void __launch_bounds__(kEpiThreads) k_conv_tile_tc(const ConvGemm g, int *err) {
     extern __shared__ uint8_t dsm[];
     constexpr int kCols = (R * BN) < 32 ? 32 : (R * BN);
     constexpr int npix = (R + 2) * kTileW, lbo_px = tile_lbo_px(R);
@@ -404,8 +431,15 @@ __global__ void __launch_bounds__(kThreads) k_conv_tile_tc(const ConvGemm g, int
     const __nv_bfloat16 *src = static_cast<const __nv_bfloat16 *>(g.src);
     const __nv_bfloat16 *wt = static_cast<const __nv_bfloat16 *>(g.wt);
     // the input tile (zero outside the image): thread q -> pixel q / chunks, chunk q % chunks (coalesced reads)
+    // unit u of the epilogue: 16 columns of one row; the two groups of four warps take every other one
+    const int m = (warp & 3) * 32 + lane;
+    constexpr int kUnits = R * (BN / 16);
+    auto unit_row = [&](int u) { return ((size_t)b * g.Ho + y0 + u / (BN / 16)) * g.Wo + x0 + m; };
+    auto unit_col = [&](int u) { return n0 + u % (BN / 16) * 16; };
+    EpilogueIn<false> in;
+    if ((warp >> 2) < kUnits) conv_load16(g, unit_row(warp >> 2), unit_col(warp >> 2), in);
     const size_t img = (size_t)b * g.Hs * g.Ws;
-    for (int q = tid; q < npix * chunks; q += kThreads) {
+    for (int q = tid; q < npix * chunks; q += kEpiThreads) {
         const int p = q / chunks, j = q - p * chunks;
         const int rr = p / kTileW, cc = p - rr * kTileW;
         const int iy = y0 - 1 + rr, ix = x0 - 1 + cc;
@@ -417,7 +451,7 @@ __global__ void __launch_bounds__(kThreads) k_conv_tile_tc(const ConvGemm g, int
     // one tap's weights: B[n][c] = wt[n0 + n][tap * C + c], chunk-major (chunk j at j * BN * 16, row n at n * 16)
     auto load_tap = [&](int t, int slot) {
         const uint32_t dst = sB + (uint32_t)slot * bstage;
-        for (int q = tid; q < BN * chunks; q += kThreads) {
+        for (int q = tid; q < BN * chunks; q += kEpiThreads) {
             const int n = q % BN, j = q / BN;
             cp_async16(dst + (uint32_t)(j * BN + n) * 16u, wt + (size_t)(n0 + n) * g.ldw + t * C + j * 8, 16);
         }
@@ -476,16 +510,12 @@ __global__ void __launch_bounds__(kThreads) k_conv_tile_tc(const ConvGemm g, int
     __syncthreads();
     tc_fence_after();
     if (!s_fail && issued == 9) {
-        const int m = warp * 32 + lane;
 #pragma unroll 1
-        for (int i = 0; i < R; ++i) {
-            const size_t row = ((size_t)b * g.Ho + y0 + i) * g.Wo + x0 + m;
-#pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 16) {
-                float v[16];
-                tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(i * BN + c0), v);
-                conv_store16(g, row, n0 + c0, v);
-            }
+        for (int u = warp >> 2; u < kUnits; u += 2) {
+            float v[16];
+            tc_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(u * 16), v);
+            conv_store16(g, unit_row(u), unit_col(u), v, in);
+            if (u + 2 < kUnits) conv_load16(g, unit_row(u + 2), unit_col(u + 2), in);
         }
     }
     tc_fence_before();
@@ -505,8 +535,8 @@ __global__ void __launch_bounds__(kThreads) k_conv_tile_tc(const ConvGemm g, int
 // one for each parity of the input pixel (blockIdx.z, the one with most taps first): of the nine taps an even
 // coordinate meets only the middle one and an odd one the outer two, 1, 2, 2 and 4 taps instead of nine with three
 // quarters zeros. The sums skip exact zeros only, in the order of the taps. Layers 1 to 3 of four 256^2 images: 131, 86
-// and 68 us with the gather kernel, 54, 31 and 21 us now.
-constexpr int kTmaStages = 4;
+// and 68 us with the gather kernel, 27, 16 and 14 us now.
+constexpr int kTmaMaxStages = 4;
 
 // K-major operand in the 128-byte swizzle: 128-byte rows (64 bf16), 8-row atoms of 1 KB (stride byte offset),
 // layout type 2 in bits 61-63; successive K = 16 slices start 32 B apart inside the atom.
@@ -519,14 +549,14 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
     return d;
 }
 
-template <int BN, bool PARITY>
-__global__ void __launch_bounds__(kThreads) k_conv_tma(const ConvGemm g, const __grid_constant__ CUtensorMap mapA,
+template <int BN, bool PARITY, bool UP>
+__global__ void __launch_bounds__(kEpiThreads) k_conv_tma(const ConvGemm g, const __grid_constant__ CUtensorMap mapA,
                                                        const __grid_constant__ CUtensorMap mapB, int bw, int bh,
-                                                       int cblocks, int *err) {
+                                                       int cblocks, int stages, int *err) {
     extern __shared__ uint8_t dsm[];
     constexpr int kA = kBM * 128, kStage = kA + BN * 128;
     constexpr int kCols = BN < 32 ? 32 : BN;
-    __shared__ __align__(8) uint64_t full[kTmaStages], empty[kTmaStages], done;
+    __shared__ __align__(8) uint64_t full[kTmaMaxStages], empty[kTmaMaxStages], done;
     __shared__ uint32_t tmem_slot;
     __shared__ int s_fail;
     uint8_t *base = align1024(dsm);
@@ -540,9 +570,18 @@ __global__ void __launch_bounds__(kThreads) k_conv_tma(const ConvGemm g, const _
     const int ox0 = pxi * bw, oy0 = pyi * bh, n0 = blockIdx.y * BN;
     const int odd_y = PARITY ? 1 - (int)(blockIdx.z >> 1) : 0, odd_x = PARITY ? 1 - (int)(blockIdx.z & 1) : 0;
     const int nk = (PARITY ? (1 + odd_y) * (1 + odd_x) : g.ks * g.ks) * cblocks;
+    const int m = (warp & 3) * 32 + lane;
+    int oy = oy0 + m / bw, ox = ox0 + m % bw;
+    if constexpr (PARITY) {
+        oy = 2 * oy + odd_y;
+        ox = 2 * ox + odd_x;
+    }
+    const size_t row = ((size_t)b * g.Ho + oy) * g.Wo + ox;
+    EpilogueIn<UP> in;
+    if ((warp >> 2) * 16 < BN) conv_load16(g, row, n0 + (warp >> 2) * 16, in);
     if (warp == 0) tmem_alloc(&tmem_slot, kCols);
     if (tid == 0) {
-        for (int s = 0; s < kTmaStages; ++s) {
+        for (int s = 0; s < stages; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
@@ -557,8 +596,8 @@ __global__ void __launch_bounds__(kThreads) k_conv_tma(const ConvGemm g, const _
     if (warp == 0 && lane == 0) {
         // producer
         for (int kt = 0; kt < nk; ++kt) {
-            const int slot = kt % kTmaStages, use = kt / kTmaStages;
-            if (kt >= kTmaStages && !mbar_wait(&empty[slot], (use - 1) & 1, kSpinLimit)) {
+            const int use = kt / stages, slot = kt - use * stages;
+            if (kt >= stages && !mbar_wait(&empty[slot], (use - 1) & 1, kSpinLimit)) {
                 s_fail = 1;
                 atomicExch(err, 1);
                 break;
@@ -591,7 +630,7 @@ __global__ void __launch_bounds__(kThreads) k_conv_tma(const ConvGemm g, const _
         // MMA issuer
         const uint32_t idesc = idesc_bf16_f32(kBM, BN);
         for (int kt = 0; kt < nk; ++kt) {
-            const int slot = kt % kTmaStages, use = kt / kTmaStages;
+            const int use = kt / stages, slot = kt - use * stages;
             if (!mbar_wait(&full[slot], use & 1, kSpinLimit)) {
                 s_fail = 1;
                 atomicExch(err, 1);
@@ -615,18 +654,12 @@ __global__ void __launch_bounds__(kThreads) k_conv_tma(const ConvGemm g, const _
     __syncthreads();
     tc_fence_after();
     if (!s_fail) {
-        const int m = warp * 32 + lane;
-        int oy = oy0 + m / bw, ox = ox0 + m % bw;
-        if constexpr (PARITY) {
-            oy = 2 * oy + odd_y;
-            ox = 2 * ox + odd_x;
-        }
-        const size_t row = ((size_t)b * g.Ho + oy) * g.Wo + ox;
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 16) {
+        for (int c0 = (warp >> 2) * 16; c0 < BN; c0 += 32) {
             float v[16];
-            tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-            conv_store16(g, row, n0 + c0, v);
+            tc_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
+            conv_store16(g, row, n0 + c0, v, in);
+            if (c0 + 32 < BN) conv_load16(g, row, n0 + c0 + 32, in);
         }
     }
     tc_fence_before();
@@ -979,18 +1012,30 @@ __global__ void k_pack_weights(int Cout, int Cst, int Cin, int taps, int Kpad, i
 }
 
 // ------------------------------------------------------------------ launchers
-template <int BN>
+template <int BN, bool UP>
 static cudaError_t conv_launch(const ConvGemm &g, int *err, cudaStream_t st) {
     constexpr int smem = kStages * (kBM * kBK * 2 + BN * kBK * 2) + 1024;
     static bool attr = false;
     if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(k_conv_tc<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaError_t e = cudaFuncSetAttribute(k_conv_tc<BN, UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
         attr = true;
     }
     const int M = g.batch * g.Ho * g.Wo;
-    k_conv_tc<BN><<<dim3((M + kBM - 1) / kBM, g.N / BN), kThreads, smem, st>>>(g, err);
+    k_conv_tc<BN, UP><<<dim3((M + kBM - 1) / kBM, g.N / BN), kThreads, smem, st>>>(g, err);
     return cudaGetLastError();
+}
+
+template <bool UP>
+static cudaError_t launch_gather(const ConvGemm &g, int bn, int *err, cudaStream_t st) {
+    switch (bn) {
+        case 16: return conv_launch<16, UP>(g, err, st);
+        case 32: return conv_launch<32, UP>(g, err, st);
+        case 64: return conv_launch<64, UP>(g, err, st);
+        case 128: return conv_launch<128, UP>(g, err, st);
+        case 256: return conv_launch<256, UP>(g, err, st);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 template <int BN, int R>
@@ -1003,7 +1048,7 @@ static cudaError_t tile_launch(const ConvGemm &g, int smem, int *err, cudaStream
         attr = smem;
     }
     const dim3 grid(g.batch * (g.Ho / R) * (g.Wo >> 7), g.N / BN);
-    k_conv_tile_tc<BN, R><<<grid, kThreads, smem, st>>>(g, err);
+    k_conv_tile_tc<BN, R><<<grid, kEpiThreads, smem, st>>>(g, err);
     return cudaGetLastError();
 }
 
@@ -1095,32 +1140,37 @@ static bool encode_conv_maps(const ConvGemm &g, int bw, int bh, int BN, CUtensor
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, bool PARITY>
+template <int BN, bool PARITY, bool UP>
 static cudaError_t tma_launch(const ConvGemm &g, int bw, int bh, const CUtensorMap &mA, const CUtensorMap &mB, int *err,
                               cudaStream_t st) {
-    constexpr int smem = kTmaStages * (kBM * 128 + BN * 128) + 1024;
+    constexpr int stage = kBM * 128 + BN * 128, limit = 200 * 1024;
     static bool attr = false;
     if (!attr) {
         const cudaError_t e =
-            cudaFuncSetAttribute(k_conv_tma<BN, PARITY>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            cudaFuncSetAttribute(k_conv_tma<BN, PARITY, UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit + 1024);
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    const int cblocks = (g.C + 63) / 64, parities = PARITY ? 4 : 1;
+    const int cblocks = (g.C + 63) / 64, parities = PARITY ? 4 : 1, nk = (PARITY ? 4 : g.ks * g.ks) * cblocks;
     const dim3 grid(g.batch * (g.Ho * g.Wo / parities) / (bh * bw), g.N / BN, parities);
-    k_conv_tma<BN, PARITY><<<grid, kThreads, smem, st>>>(g, mA, mB, bw, bh, cblocks, err);
+    // four stages (what fits of them) when the grid leaves each SM one or two CTAs; two when there are more, which then
+    // hide each other's latency: with four the layers of four 256^2 images took 260 us forward, with two 243, and rings
+    // of six or eight gave the one-CTA layers nothing
+    const int per_sm = ((int)(grid.x * grid.y * grid.z) + 151) / 152;
+    const int stages = std::min({nk, kTmaMaxStages, per_sm > 2 ? 2 : limit / per_sm / stage});
+    k_conv_tma<BN, PARITY, UP><<<grid, kEpiThreads, stages * stage + 1024, st>>>(g, mA, mB, bw, bh, cblocks, stages, err);
     return cudaGetLastError();
 }
 
-template <bool PARITY>
+template <bool PARITY, bool UP>
 static cudaError_t launch_tma(const ConvGemm &g, int bn, int bw, int bh, const CUtensorMap &mA, const CUtensorMap &mB,
                               int *err, cudaStream_t st) {
     switch (bn) {
-        case 16: return tma_launch<16, PARITY>(g, bw, bh, mA, mB, err, st);
-        case 32: return tma_launch<32, PARITY>(g, bw, bh, mA, mB, err, st);
-        case 64: return tma_launch<64, PARITY>(g, bw, bh, mA, mB, err, st);
-        case 128: return tma_launch<128, PARITY>(g, bw, bh, mA, mB, err, st);
-        default: return tma_launch<256, PARITY>(g, bw, bh, mA, mB, err, st);
+        case 16: return tma_launch<16, PARITY, UP>(g, bw, bh, mA, mB, err, st);
+        case 32: return tma_launch<32, PARITY, UP>(g, bw, bh, mA, mB, err, st);
+        case 64: return tma_launch<64, PARITY, UP>(g, bw, bh, mA, mB, err, st);
+        case 128: return tma_launch<128, PARITY, UP>(g, bw, bh, mA, mB, err, st);
+        default: return tma_launch<256, PARITY, UP>(g, bw, bh, mA, mB, err, st);
     }
 }
 
@@ -1156,8 +1206,9 @@ cudaError_t launch_conv_tc(const ConvGemm &g, int *err, cudaStream_t st, LaunchC
         }
         // a map the driver does not accept sends the layer to the other kernels
         if (tma && encode_conv_maps(g, bw, bh, bn, &mA, &mB)) {
-            const cudaError_t e = tma_parity(g) ? launch_tma<true>(g, bn, bw, bh, mA, mB, err, st)
-                                                : launch_tma<false>(g, bn, bw, bh, mA, mB, err, st);
+            const cudaError_t e = tma_parity(g) ? launch_tma<true, false>(g, bn, bw, bh, mA, mB, err, st)
+                                  : g.upskip    ? launch_tma<false, true>(g, bn, bw, bh, mA, mB, err, st)
+                                                : launch_tma<false, false>(g, bn, bw, bh, mA, mB, err, st);
             lc.add(1);
             return e;
         }
@@ -1177,15 +1228,7 @@ cudaError_t launch_conv_tc(const ConvGemm &g, int *err, cudaStream_t st, LaunchC
     const int mtiles = (g.batch * g.Ho * g.Wo + kBM - 1) / kBM;
     int bn = g.N;
     while (bn > 32 && mtiles * (g.N / bn) < 120) bn >>= 1;
-    cudaError_t e;
-    switch (bn) {
-        case 16: e = conv_launch<16>(g, err, st); break;
-        case 32: e = conv_launch<32>(g, err, st); break;
-        case 64: e = conv_launch<64>(g, err, st); break;
-        case 128: e = conv_launch<128>(g, err, st); break;
-        case 256: e = conv_launch<256>(g, err, st); break;
-        default: return cudaErrorInvalidValue;
-    }
+    const cudaError_t e = g.upskip ? launch_gather<true>(g, bn, err, st) : launch_gather<false>(g, bn, err, st);
     lc.add(1);
     return e;
 }
