@@ -681,7 +681,7 @@ __host__ __device__ constexpr int wg_stage_bytes(int BN) { return 8 * kWgSbo * (
 __host__ __device__ constexpr int wg_stages(int BN) { return BN <= 32 ? 4 : BN == 64 ? 3 : BN == 128 ? 2 : 3; }
 
 template <int BN>
-__global__ void __launch_bounds__(kThreads) k_wgrad_tc(const WgradGemm g, int *err) {
+__global__ void __launch_bounds__(kEpiThreads) k_wgrad_tc(const WgradGemm g, int *err) {
     extern __shared__ uint8_t dsm[];
     constexpr int kWgStages = wg_stages(BN), kStage = wg_stage_bytes(BN);
     constexpr int kLboA = kBM / 8 * kWgSbo, kLboB = BN / 8 * kWgSbo, kA = 8 * kLboA;
@@ -701,43 +701,44 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_tc(const WgradGemm g, int *e
         s_fail = 0;
         fence_proxy_async_smem();
     }
-    // this thread's four X chunks (8 channels of one tap each): channel block 4 q + (tid & 3) of the tile
-    int ady[4], adx[4], aci[4];
+    // this thread's four X chunks (8 channels of one tap each), channel blocks 4 q + (tid & 3) of the tile, all of pixel
+    // tid / 4 of a stage: the tap's step, and the chunk's offset from the pixel's first channel
+    int ady[4], adx[4], aoff[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int r0 = m0 + (4 * q + (tid & 3)) * 8;
         const int tap = r0 / g.Cin;
-        aci[q] = r0 < g.Kf ? r0 - tap * g.Cin : -1;
         ady[q] = g.ks == 3 ? tap / 3 - 1 : 0;
         adx[q] = g.ks == 3 ? tap - (tap / 3) * 3 - 1 : 0;
+        aoff[q] = (ady[q] * g.Wx + adx[q]) * g.Cin + r0 - tap * g.Cin;
+        if (r0 >= g.Kf) ady[q] = -(1 << 28);  // past the last row: outside every image
     }
     const __nv_bfloat16 *X = static_cast<const __nv_bfloat16 *>(g.x);
     const __nv_bfloat16 *DY = static_cast<const __nv_bfloat16 *>(g.dy);
     const uint32_t sbase = smem_u32(base);
+    const int pk = tid >> 2;
     auto load_stage = [&](int kt, int slot) {
         const uint32_t sa = sbase + slot * kStage, sb = sa + kA;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int pk = (tid >> 2) + 32 * h, p = p0 + kt * kBK + pk;
+        {
+            const int p = p0 + kt * kBK + pk;
             const bool pv = p < p1;
             const int b = p / HWo, rem = p - b * HWo, oy = rem / g.Wo, ox = rem - oy * g.Wo;
             const int y0 = oy * g.stride, x0 = ox * g.stride;
-            const size_t img = (size_t)b * g.Hx * g.Wx;
+            const __nv_bfloat16 *px = X + ((size_t)b * g.Hx * g.Wx + (size_t)y0 * g.Wx + x0) * g.Cin;
             const uint32_t dst = sa + (uint32_t)((pk >> 3) * kLboA + (tid & 3) * kWgSbo + ((pk & 7) << 4));
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int iy = y0 + ady[q], ix = x0 + adx[q];
-                const bool ok = pv && aci[q] >= 0 && iy >= 0 && iy < g.Hx && ix >= 0 && ix < g.Wx;
-                const __nv_bfloat16 *src = ok ? X + (img + (size_t)iy * g.Wx + ix) * g.Cin + aci[q] : X;
-                cp_async16(dst + q * 4 * kWgSbo, src, ok ? 16 : 0);
+                const bool ok = pv && (unsigned)(y0 + ady[q]) < (unsigned)g.Hx && (unsigned)(x0 + adx[q]) < (unsigned)g.Wx;
+                cp_async16(dst + q * 4 * kWgSbo, ok ? px + aoff[q] : X, ok ? 16 : 0);
             }
         }
 #pragma unroll
-        for (int j = 0; j < BN / 16; ++j) {
-            const int i = tid + kThreads * j, c = i % kBC + kBC * (i / (kBC * kBK)), pk = i / kBC % kBK;
-            const int p = p0 + kt * kBK + pk;
+        for (int j = 0; j < (BN * 8 + kEpiThreads - 1) / kEpiThreads; ++j) {
+            const int i = tid + kEpiThreads * j, c = i % kBC + kBC * (i / (kBC * kBK)), k = i / kBC % kBK;
+            if (BN * 8 < kEpiThreads && i >= BN * 8) break;
+            const int p = p0 + kt * kBK + k;
             const bool pv = p < p1;
-            cp_async16(sb + (uint32_t)((pk >> 3) * kLboB + c * kWgSbo + ((pk & 7) << 4)),
+            cp_async16(sb + (uint32_t)((k >> 3) * kLboB + c * kWgSbo + ((k & 7) << 4)),
                        pv ? DY + (size_t)p * g.Cout + c * 8 : DY, pv ? 16 : 0);
         }
     };
@@ -795,12 +796,12 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_tc(const WgradGemm g, int *e
     __syncthreads();
     tc_fence_after();
     if (!s_fail) {
-        const int r = warp * 32 + lane;
+        const int r = (warp & 3) * 32 + lane;
         float *out = g.partial + ((size_t)blockIdx.y * g.Mpad + m0 + r) * BN;
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 16) {
+        for (int c0 = (warp >> 2) * 16; c0 < BN; c0 += 32) {
             float v[16];
-            if (issued > 0) tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+            if (issued > 0) tc_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
             else {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) v[i] = 0.f;
@@ -970,8 +971,10 @@ __global__ void __launch_bounds__(256) k_output_head(int batch, int HW, int Cy, 
             acc += (double)d[c] * d[c];
         }
         if (dy) {
-            for (int c = 0; c < Cy; ++c)
-                dy[p * Cy + c] = __float2bfloat16_rn(c < 3 ? d[c] * scale : 0.f);
+            const float f[8] = {d[0] * scale, d[1] * scale, d[2] * scale, 0.f, 0.f, 0.f, 0.f, 0.f};
+            uint4 *row = reinterpret_cast<uint4 *>(dy + p * Cy);
+            row[0] = pack8(f);
+            for (int c = 1; c < Cy / 8; ++c) row[c] = make_uint4(0, 0, 0, 0);
         }
     }
     acc = block_sum<256>(acc, sh);
@@ -1242,7 +1245,7 @@ static cudaError_t wgrad_launch(const WgradGemm &g, int splits, int *err, cudaSt
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    k_wgrad_tc<BN><<<dim3(g.Mpad / kBM, splits), kThreads, smem, st>>>(g, err);
+    k_wgrad_tc<BN><<<dim3(g.Mpad / kBM, splits), kEpiThreads, smem, st>>>(g, err);
     return cudaGetLastError();
 }
 
