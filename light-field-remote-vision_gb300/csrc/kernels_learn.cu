@@ -430,7 +430,8 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tile_tc(const ConvGemm g, 
     }
     const __nv_bfloat16 *src = static_cast<const __nv_bfloat16 *>(g.src);
     const __nv_bfloat16 *wt = static_cast<const __nv_bfloat16 *>(g.wt);
-    // the input tile (zero outside the image): thread q -> pixel q / chunks, chunk q % chunks (coalesced reads)
+    // the input tile (zero outside the image): thread q -> pixel q / chunks of a row, chunk q % chunks (coalesced reads), in
+    // every row of the tile
     // unit u of the epilogue: 16 columns of one row; the two groups of four warps take every other one
     const int m = (warp & 3) * 32 + lane;
     constexpr int kUnits = R * (BN / 16);
@@ -439,13 +440,18 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tile_tc(const ConvGemm g, 
     EpilogueIn<false> in;
     if ((warp >> 2) < kUnits) conv_load16(g, unit_row(warp >> 2), unit_col(warp >> 2), in);
     const size_t img = (size_t)b * g.Hs * g.Ws;
-    for (int q = tid; q < npix * chunks; q += kEpiThreads) {
-        const int p = q / chunks, j = q - p * chunks;
-        const int rr = p / kTileW, cc = p - rr * kTileW;
-        const int iy = y0 - 1 + rr, ix = x0 - 1 + cc;
-        const bool ok = iy >= 0 && iy < g.Hs && ix >= 0 && ix < g.Ws;
-        const __nv_bfloat16 *gp = ok ? src + (img + (size_t)iy * g.Ws + ix) * C + j * 8 : src;
-        cp_async16(sA + (uint32_t)j * lboA + (uint32_t)p * 16u, gp, ok ? 16 : 0);
+    for (int q = tid; q < kTileW * chunks; q += kEpiThreads) {
+        const int cc = q / chunks, j = q - cc * chunks;
+        const int ix = x0 - 1 + cc;
+        const bool okx = ix >= 0 && ix < g.Ws;
+        const __nv_bfloat16 *col = src + (img + (size_t)(okx ? ix : 0)) * C + j * 8;
+        const uint32_t dst = sA + (uint32_t)j * lboA + (uint32_t)cc * 16u;
+#pragma unroll
+        for (int rr = 0; rr < R + 2; ++rr) {
+            const int iy = y0 - 1 + rr;
+            const bool ok = okx && iy >= 0 && iy < g.Hs;
+            cp_async16(dst + (uint32_t)(rr * kTileW) * 16u, ok ? col + (size_t)iy * g.Ws * C : src, ok ? 16 : 0);
+        }
     }
     cp_async_commit();
     // one tap's weights: B[n][c] = wt[n0 + n][tap * C + c], chunk-major (chunk j at j * BN * 16, row n at n * 16)
@@ -716,30 +722,42 @@ __global__ void __launch_bounds__(kEpiThreads) k_wgrad_tc(const WgradGemm g, int
     const __nv_bfloat16 *X = static_cast<const __nv_bfloat16 *>(g.x);
     const __nv_bfloat16 *DY = static_cast<const __nv_bfloat16 *>(g.dy);
     const uint32_t sbase = smem_u32(base);
-    const int pk = tid >> 2;
+    const int pk = tid >> 2, yk = tid / kBC;  // this thread's pixel of a stage for X and for dY
+    int p = p0 + pk, b = p / HWo, oy = (p - b * HWo) / g.Wo, ox = p - b * HWo - oy * g.Wo;
+    // stages are loaded in order: the pixel moves on by one stage a call, without a division where a row holds a stage
     auto load_stage = [&](int kt, int slot) {
         const uint32_t sa = sbase + slot * kStage, sb = sa + kA;
-        {
-            const int p = p0 + kt * kBK + pk;
-            const bool pv = p < p1;
-            const int b = p / HWo, rem = p - b * HWo, oy = rem / g.Wo, ox = rem - oy * g.Wo;
-            const int y0 = oy * g.stride, x0 = ox * g.stride;
-            const __nv_bfloat16 *px = X + ((size_t)b * g.Hx * g.Wx + (size_t)y0 * g.Wx + x0) * g.Cin;
-            const uint32_t dst = sa + (uint32_t)((pk >> 3) * kLboA + (tid & 3) * kWgSbo + ((pk & 7) << 4));
+        const bool pv = p < p1;
+        const int y0 = oy * g.stride, x0 = ox * g.stride;
+        const __nv_bfloat16 *px = X + (size_t)((b * g.Hx + y0) * g.Wx + x0) * g.Cin;
+        const uint32_t dst = sa + (uint32_t)((pk >> 3) * kLboA + (tid & 3) * kWgSbo + ((pk & 7) << 4));
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const bool ok = pv && (unsigned)(y0 + ady[q]) < (unsigned)g.Hx && (unsigned)(x0 + adx[q]) < (unsigned)g.Wx;
-                cp_async16(dst + q * 4 * kWgSbo, ok ? px + aoff[q] : X, ok ? 16 : 0);
-            }
+        for (int q = 0; q < 4; ++q) {
+            const bool ok = pv && (unsigned)(y0 + ady[q]) < (unsigned)g.Hx && (unsigned)(x0 + adx[q]) < (unsigned)g.Wx;
+            cp_async16(dst + q * 4 * kWgSbo, ok ? px + aoff[q] : X, ok ? 16 : 0);
         }
+        if (yk < kBK) {
+            const int py = p0 + kt * kBK + yk;
+            const bool yv = py < p1;
+            const __nv_bfloat16 *src = yv ? DY + (size_t)py * BN + tid % kBC * 8 : DY;
+            const uint32_t ydst = sb + (uint32_t)((yk >> 3) * kLboB + tid % kBC * kWgSbo + ((yk & 7) << 4));
 #pragma unroll
-        for (int j = 0; j < (BN * 8 + kEpiThreads - 1) / kEpiThreads; ++j) {
-            const int i = tid + kEpiThreads * j, c = i % kBC + kBC * (i / (kBC * kBK)), k = i / kBC % kBK;
-            if (BN * 8 < kEpiThreads && i >= BN * 8) break;
-            const int p = p0 + kt * kBK + k;
-            const bool pv = p < p1;
-            cp_async16(sb + (uint32_t)((k >> 3) * kLboB + c * kWgSbo + ((k & 7) << 4)),
-                       pv ? DY + (size_t)p * g.Cout + c * 8 : DY, pv ? 16 : 0);
+            for (int c = 0; c < BN / 8; c += kBC) cp_async16(ydst + c * kWgSbo, yv ? src + c * 8 : DY, yv ? 16 : 0);
+        }
+        p += kBK;
+        if (g.Wo >= kBK) {
+            ox += kBK;
+            if (ox >= g.Wo) {
+                ox -= g.Wo;
+                if (++oy == g.Ho) {
+                    oy = 0;
+                    ++b;
+                }
+            }
+        } else {
+            b = p / HWo;
+            oy = (p - b * HWo) / g.Wo;
+            ox = p - b * HWo - oy * g.Wo;
         }
     };
     tc_fence_before();
