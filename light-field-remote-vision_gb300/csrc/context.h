@@ -159,3 +159,9 @@ struct lfrv_ctx {
     // contexts of the corrected IBR_color jobs of a batched call (one per job, own stream and workspace)
     std::vector<lfrv_ctx *> tv_jobs;
 };
+
+namespace lfrv {
+// The side stream: work of a call that depends only on its inputs (or whose results only the call's end reads) runs there,
+// between events recorded on the context stream (fork) and one the context stream waits for (join). Created on first use.
+cudaStream_t side_stream(lfrv_ctx *c);
+}  // namespace lfrv

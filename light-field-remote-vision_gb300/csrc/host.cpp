@@ -121,9 +121,7 @@ static double *host_sums(lfrv_ctx *c) {
     return c->host_sums;
 }
 
-// The side stream: work of a call that depends only on its inputs runs there, between an event recorded on the
-// context stream (fork) and one the context stream waits for (join). Created on first use.
-static cudaStream_t side_stream(lfrv_ctx *c) {
+cudaStream_t side_stream(lfrv_ctx *c) {
     if (!c->side_stream) {
         LFRV_CUDA(cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking));
         LFRV_CUDA(cudaEventCreateWithFlags(&c->side_fork, cudaEventDisableTiming));

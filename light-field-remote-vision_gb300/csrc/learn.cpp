@@ -218,20 +218,16 @@ void conv_dgrad(lfrv_warmstart *net, int l, const void *dy, int level, const voi
     LFRV_CUDA(launch_conv_tc(g, net_err(net), net->ctx->stream, net->ctx->launches));
 }
 
-// dW and db of layer l (input x at `level`, output gradient dy) into the flat gradient.
-void conv_wgrad(lfrv_warmstart *net, int l, const void *x, int level, const void *dy) {
+// Weight gradient of layer l, whose input lies at `level`: shapes and the split of its pixels.
+WgradGemm wgrad_gemm(const lfrv_warmstart *net, int l, int level, int &splits) {
     const Layer &L = net->L[l];
-    lfrv_ctx *c = net->ctx;
-    const int Hin = net->H >> level, Win = net->W >> level;
     WgradGemm g{};
-    g.x = x;
     g.Cin = L.d.cin;
-    g.Hx = Hin;
-    g.Wx = Win;
-    g.dy = dy;
+    g.Hx = net->H >> level;
+    g.Wx = net->W >> level;
     g.Cout = L.cst;
-    g.Ho = Hin / L.d.stride;
-    g.Wo = Win / L.d.stride;
+    g.Ho = g.Hx / L.d.stride;
+    g.Wo = g.Wx / L.d.stride;
     g.batch = net->batch;
     g.ks = L.d.ks;
     g.stride = L.d.stride;
@@ -239,14 +235,29 @@ void conv_wgrad(lfrv_warmstart *net, int l, const void *x, int level, const void
     g.Mpad = round_up(L.Kf, 128);
     const int P = net->batch * g.Ho * g.Wo;
     const int mt = g.Mpad / 128, max_splits = (P + 63) / 64;
-    int splits = std::min(max_splits, std::max(1, (2 * 152 + mt - 1) / mt));
+    splits = std::min(max_splits, std::max(1, (2 * 152 + mt - 1) / mt));
     g.chunk = round_up((P + splits - 1) / splits, 64);
     splits = (P + g.chunk - 1) / g.chunk;
-    net->partial.ensure((size_t)splits * g.Mpad * L.cst * sizeof(float));
+    return g;
+}
+
+// dW and db of layer l (input x at `level`, output gradient dy) into the flat gradient, on the side stream once the
+// context stream has dy: nothing of the backward pass reads them, so they run beside the data gradients of the layers
+// below, whose grids leave half the chip idle. backward() sizes the shared partials before the first of them and joins.
+void conv_wgrad(lfrv_warmstart *net, int l, const void *x, int level, const void *dy) {
+    const Layer &L = net->L[l];
+    lfrv_ctx *c = net->ctx;
+    int splits = 0;
+    WgradGemm g = wgrad_gemm(net, l, level, splits);
+    g.x = x;
+    g.dy = dy;
     g.partial = net->partial.as<float>();
     float *grad = net->grads.as<float>();
+    cudaStream_t side = side_stream(c);
+    LFRV_CUDA(cudaEventRecord(c->side_fork, c->stream));
+    LFRV_CUDA(cudaStreamWaitEvent(side, c->side_fork, 0));
     LFRV_CUDA(launch_wgrad_tc(g, splits, L.d.cout, grad + L.w_off, net->bias_part.as<float>(), kBiasBlocks,
-                              grad + L.b_off, net_err(net), c->stream, c->launches));
+                              grad + L.b_off, net_err(net), side, c->launches));
 }
 
 void forward(lfrv_warmstart *net, const void *in) {
@@ -271,32 +282,42 @@ void backward(lfrv_warmstart *net, const void *in) {
     lfrv_ctx *c = net->ctx;
     auto b = [&](int i) { return net->t[i].p; };
     const int B = net->batch, H = net->H, W = net->W;
-    conv_wgrad(net, 11, b(A10), 0, b(DY11));
+    constexpr int level_of[kLayers] = {0, 0, 1, 2, 3, 3, 2, 2, 1, 1, 0, 0};  // of each layer's input
+    size_t partial = 0;
+    for (int l = 0; l < kLayers; ++l) {
+        int splits = 0;
+        const WgradGemm g = wgrad_gemm(net, l, level_of[l], splits);
+        partial = std::max(partial, (size_t)splits * g.Mpad * g.Cout * sizeof(float));
+    }
+    net->partial.ensure(partial);
+    conv_wgrad(net, 11, b(A10), level_of[11], b(DY11));
     conv_dgrad(net, 11, b(DY11), 0, nullptr, b(A10), b(G10));
-    conv_wgrad(net, 10, b(S9), 0, b(G10));
+    conv_wgrad(net, 10, b(S9), level_of[10], b(G10));
     conv_dgrad(net, 10, b(G10), 0, nullptr, b(S9), b(GS9));
     LFRV_CUDA(launch_down_sum(B, H >> 1, W >> 1, 32, b(GS9), b(DT9), c->stream, c->launches));
-    conv_wgrad(net, 9, b(A8), 1, b(DT9));
+    conv_wgrad(net, 9, b(A8), level_of[9], b(DT9));
     conv_dgrad(net, 9, b(DT9), 1, nullptr, b(A8), b(G8));
-    conv_wgrad(net, 8, b(S7), 1, b(G8));
+    conv_wgrad(net, 8, b(S7), level_of[8], b(G8));
     conv_dgrad(net, 8, b(G8), 1, nullptr, b(S7), b(GS7));
     LFRV_CUDA(launch_down_sum(B, H >> 2, W >> 2, 64, b(GS7), b(DT7), c->stream, c->launches));
-    conv_wgrad(net, 7, b(A6), 2, b(DT7));
+    conv_wgrad(net, 7, b(A6), level_of[7], b(DT7));
     conv_dgrad(net, 7, b(DT7), 2, nullptr, b(A6), b(G6));
-    conv_wgrad(net, 6, b(S5), 2, b(G6));
+    conv_wgrad(net, 6, b(S5), level_of[6], b(G6));
     conv_dgrad(net, 6, b(G6), 2, nullptr, b(S5), b(GS5));
     LFRV_CUDA(launch_down_sum(B, H >> 3, W >> 3, 128, b(GS5), b(DT5), c->stream, c->launches));
-    conv_wgrad(net, 5, b(A4), 3, b(DT5));
+    conv_wgrad(net, 5, b(A4), level_of[5], b(DT5));
     conv_dgrad(net, 5, b(DT5), 3, nullptr, b(A4), b(G4));
-    conv_wgrad(net, 4, b(A3), 3, b(G4));
+    conv_wgrad(net, 4, b(A3), level_of[4], b(G4));
     conv_dgrad(net, 4, b(G4), 3, nullptr, b(A3), b(G3));
-    conv_wgrad(net, 3, b(A2), 2, b(G3));
+    conv_wgrad(net, 3, b(A2), level_of[3], b(G3));
     conv_dgrad(net, 3, b(G3), 2, b(GS5), b(A2), b(G2));
-    conv_wgrad(net, 2, b(A1), 1, b(G2));
+    conv_wgrad(net, 2, b(A1), level_of[2], b(G2));
     conv_dgrad(net, 2, b(G2), 1, b(GS7), b(A1), b(G1));
-    conv_wgrad(net, 1, b(A0), 0, b(G1));
+    conv_wgrad(net, 1, b(A0), level_of[1], b(G1));
     conv_dgrad(net, 1, b(G1), 0, b(GS9), b(A0), b(G0));
-    conv_wgrad(net, 0, in, 0, b(G0));
+    conv_wgrad(net, 0, in, level_of[0], b(G0));
+    LFRV_CUDA(cudaEventRecord(c->side_join, c->side_stream));
+    LFRV_CUDA(cudaStreamWaitEvent(c->stream, c->side_join, 0));
 }
 
 // Output head: prediction and/or the loss partials + dY of the last layer (asynchronous).
