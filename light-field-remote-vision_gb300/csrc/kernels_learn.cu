@@ -173,21 +173,21 @@ __device__ __forceinline__ void conv_load16(const ConvGemm &g, size_t row, int c
         for (int d = 0; d < 4; ++d) {
             const uint4 *sp = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(g.upskip) +
                                                               upskip_row(g, row, d) * g.N + col);
-            in.u[2 * d] = __ldg(sp);
-            in.u[2 * d + 1] = __ldg(sp + 1);
+            in.u[2 * d] = sp[0];
+            in.u[2 * d + 1] = sp[1];
         }
         return;
     }
     const size_t o = row * g.N + col;
     if (g.add) {
         const uint4 *ap = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(g.add) + o);
-        in.u[0] = __ldg(ap);
-        in.u[1] = __ldg(ap + 1);
+        in.u[0] = ap[0];
+        in.u[1] = ap[1];
     }
     if (g.mask) {
         const uint4 *mp = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(g.mask) + o);
-        in.u[2] = __ldg(mp);
-        in.u[3] = __ldg(mp + 1);
+        in.u[2] = mp[0];
+        in.u[3] = mp[1];
     }
 }
 
@@ -323,6 +323,8 @@ __global__ void __launch_bounds__(kThreads) k_conv_tc(const ConvGemm g, int *err
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_trigger();
+    pdl_wait();
     const uint32_t tmem = tmem_slot;
     const uint32_t idesc = idesc_bf16_f32(kBM, BN);
     const int nk = (g.K + kBK - 1) / kBK;
@@ -428,6 +430,11 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tile_tc(const ConvGemm g, 
         s_fail = 0;
         fence_proxy_async_smem();
     }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    pdl_trigger();
+    pdl_wait();
     const __nv_bfloat16 *src = static_cast<const __nv_bfloat16 *>(g.src);
     const __nv_bfloat16 *wt = static_cast<const __nv_bfloat16 *>(g.wt);
     // the input tile (zero outside the image): thread q -> pixel q / chunks of a row, chunk q % chunks (coalesced reads), in
@@ -466,9 +473,6 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tile_tc(const ConvGemm g, 
     cp_async_commit();
     load_tap(1, 1);
     cp_async_commit();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
     const uint32_t tmem = tmem_slot;
     const uint32_t idesc = idesc_bf16_f32(kBM, BN);
     int issued = 0;
@@ -583,8 +587,6 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tma(const ConvGemm g, cons
         ox = 2 * ox + odd_x;
     }
     const size_t row = ((size_t)b * g.Ho + oy) * g.Wo + ox;
-    EpilogueIn<UP> in;
-    if ((warp >> 2) * 16 < BN) conv_load16(g, row, n0 + (warp >> 2) * 16, in);
     if (warp == 0) tmem_alloc(&tmem_slot, kCols);
     if (tid == 0) {
         for (int s = 0; s < stages; ++s) {
@@ -598,6 +600,10 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tma(const ConvGemm g, cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_trigger();
+    pdl_wait();
+    EpilogueIn<UP> in;
+    if ((warp >> 2) * 16 < BN) conv_load16(g, row, n0 + (warp >> 2) * 16, in);
     const uint32_t tmem = tmem_slot;
     if (warp == 0 && lane == 0) {
         // producer
@@ -831,6 +837,7 @@ __global__ void __launch_bounds__(kEpiThreads) k_wgrad_tc(const WgradGemm g, int
     }
     tc_fence_before();
     __syncthreads();
+    pdl_wait();  // the column sums this kernel ran beside
     if (warp == 0) tmem_free(tmem, kCols);
 }
 
@@ -839,6 +846,7 @@ __global__ void __launch_bounds__(kEpiThreads) k_wgrad_tc(const WgradGemm g, int
 constexpr int kColsumUnroll = 4;
 __global__ void __launch_bounds__(256) k_colsum(int P, int C, const __nv_bfloat16 *__restrict__ dy,
                                                 float *__restrict__ partial) {
+    pdl_trigger();
     __shared__ float sh[256 * 9];  // nine floats a thread: eight and one of padding
     const int chunks = C >> 3, lanes = 256 / chunks, j = threadIdx.x % chunks, l = threadIdx.x / chunks;
     float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -973,6 +981,7 @@ __global__ void __launch_bounds__(256) k_output_head(int batch, int HW, int Cy, 
                                                      const float *__restrict__ u0, const float *__restrict__ target,
                                                      float *__restrict__ pred, __nv_bfloat16 *__restrict__ dy,
                                                      double *__restrict__ loss_partial) {
+    pdl_wait();
     __shared__ double sh[8];
     const size_t P = (size_t)batch * HW;
     const float scale = 2.0f / (3.0f * (float)P);
@@ -1033,6 +1042,17 @@ __global__ void k_pack_weights(int Cout, int Cst, int Cin, int taps, int Kpad, i
 }
 
 // ------------------------------------------------------------------ launchers
+// A forward layer starts setting up (tensor memory, barriers, indices) while the layer before it ends: twelve layers of one
+// 512^2 image 239 -> 222 us. The data gradients don't: their early blocks would hold shared memory that the weight
+// gradients beside them use (4 images of 256^2, the call without its copy: 690 us with, 665 without).
+template <typename... Params, typename... Args>
+static cudaError_t launch_layer(const ConvGemm &g, void (*kernel)(Params...), dim3 grid, int threads, int smem,
+                                cudaStream_t st, Args... args) {
+    if (!g.dgrad) return launch_pdl(kernel, grid, dim3(threads), (size_t)smem, st, args...);
+    kernel<<<grid, threads, smem, st>>>(args...);
+    return cudaGetLastError();
+}
+
 template <int BN, bool UP>
 static cudaError_t conv_launch(const ConvGemm &g, int *err, cudaStream_t st) {
     constexpr int smem = kStages * (kBM * kBK * 2 + BN * kBK * 2) + 1024;
@@ -1043,8 +1063,7 @@ static cudaError_t conv_launch(const ConvGemm &g, int *err, cudaStream_t st) {
         attr = true;
     }
     const int M = g.batch * g.Ho * g.Wo;
-    k_conv_tc<BN, UP><<<dim3((M + kBM - 1) / kBM, g.N / BN), kThreads, smem, st>>>(g, err);
-    return cudaGetLastError();
+    return launch_layer(g, k_conv_tc<BN, UP>, dim3((M + kBM - 1) / kBM, g.N / BN), kThreads, smem, st, g, err);
 }
 
 template <bool UP>
@@ -1069,8 +1088,7 @@ static cudaError_t tile_launch(const ConvGemm &g, int smem, int *err, cudaStream
         attr = smem;
     }
     const dim3 grid(g.batch * (g.Ho / R) * (g.Wo >> 7), g.N / BN);
-    k_conv_tile_tc<BN, R><<<grid, kEpiThreads, smem, st>>>(g, err);
-    return cudaGetLastError();
+    return launch_layer(g, k_conv_tile_tc<BN, R>, grid, kEpiThreads, smem, st, g, err);
 }
 
 // The resident-tile kernel's shape for a stride-1 3 x 3 layer (forward, or data gradient of a stride-1 layer), or
@@ -1179,8 +1197,8 @@ static cudaError_t tma_launch(const ConvGemm &g, int bw, int bh, const CUtensorM
     // of six or eight gave the one-CTA layers nothing
     const int per_sm = ((int)(grid.x * grid.y * grid.z) + 151) / 152;
     const int stages = std::min({nk, kTmaMaxStages, per_sm > 2 ? 2 : limit / per_sm / stage});
-    k_conv_tma<BN, PARITY, UP><<<grid, kEpiThreads, stages * stage + 1024, st>>>(g, mA, mB, bw, bh, cblocks, stages, err);
-    return cudaGetLastError();
+    return launch_layer(g, k_conv_tma<BN, PARITY, UP>, grid, kEpiThreads, stages * stage + 1024, st, g, mA, mB, bw, bh,
+                        cblocks, stages, err);
 }
 
 template <bool PARITY, bool UP>
@@ -1255,7 +1273,7 @@ cudaError_t launch_conv_tc(const ConvGemm &g, int *err, cudaStream_t st, LaunchC
 }
 
 template <int BN>
-static cudaError_t wgrad_launch(const WgradGemm &g, int splits, int *err, cudaStream_t st) {
+static cudaError_t wgrad_launch(const WgradGemm &g, int splits, bool beside, int *err, cudaStream_t st) {
     constexpr int smem = wg_stages(BN) * wg_stage_bytes(BN) + 1024;
     static bool attr = false;
     if (!attr) {
@@ -1263,27 +1281,17 @@ static cudaError_t wgrad_launch(const WgradGemm &g, int splits, int *err, cudaSt
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    k_wgrad_tc<BN><<<dim3(g.Mpad / kBM, splits), kEpiThreads, smem, st>>>(g, err);
+    const dim3 grid(g.Mpad / kBM, splits);
+    // beside: the launch before it is this layer's column sums, which started after all that this kernel reads was written
+    if (beside) return launch_pdl(k_wgrad_tc<BN>, grid, dim3(kEpiThreads), smem, st, g, err);
+    k_wgrad_tc<BN><<<grid, kEpiThreads, smem, st>>>(g, err);
     return cudaGetLastError();
 }
 
 cudaError_t launch_wgrad_tc(const WgradGemm &g, int splits, int Cout_real, float *grad, float *bias_partial,
                             int bias_blocks, float *bias_out, int *err, cudaStream_t st, LaunchCounter &lc) {
-    {
-        ProfScope _ps(lc, "conv_wgrad_tc", st);
-        if (g.Cin % 8 || g.Mpad % kBM || g.Mpad < g.Kf || g.chunk % kBK) return cudaErrorInvalidValue;
-        cudaError_t e;
-        switch (g.Cout) {
-            case 16: e = wgrad_launch<16>(g, splits, err, st); break;
-            case 32: e = wgrad_launch<32>(g, splits, err, st); break;
-            case 64: e = wgrad_launch<64>(g, splits, err, st); break;
-            case 128: e = wgrad_launch<128>(g, splits, err, st); break;
-            case 256: e = wgrad_launch<256>(g, splits, err, st); break;
-            default: return cudaErrorInvalidValue;
-        }
-        lc.add(1);
-        if (e != cudaSuccess) return e;
-    }
+    if (g.Cin % 8 || g.Mpad % kBM || g.Mpad < g.Kf || g.chunk % kBK) return cudaErrorInvalidValue;
+    if (g.Cout != 16 && g.Cout != 32 && g.Cout != 64 && g.Cout != 128 && g.Cout != 256) return cudaErrorInvalidValue;
     ReducePart w{}, bias{};
     auto part = [](ReducePart &r, const float *partial, float *out, size_t stride, int count, int Cst, int Kf, int Cout) {
         // threads per element: enough to fill the chip where the elements alone do not, at most one a partial
@@ -1294,13 +1302,27 @@ cudaError_t launch_wgrad_tc(const WgradGemm &g, int splits, int Cout_real, float
         r = ReducePart{partial, out, stride, count, Cst, Kf, Cout, lanes, (int)((vecs + width - 1) / width)};
     };
     part(w, g.partial, grad, (size_t)g.Mpad * g.Cout, splits, g.Cout, g.Kf, Cout_real);
-    if (bias_out) {
+    if (bias_out) {  // before the products, which start while it runs
         ProfScope _ps(lc, "bias_grad", st);
         const int P = g.batch * g.Ho * g.Wo, lanes = 256 / (g.Cout / 8);
         const int blocks = std::min(bias_blocks, std::max(1, P / (lanes * kColsumUnroll)));
         k_colsum<<<blocks, 256, 0, st>>>(P, g.Cout, static_cast<const __nv_bfloat16 *>(g.dy), bias_partial);
         lc.add(1);
         part(bias, bias_partial, bias_out, (size_t)g.Cout, blocks, g.Cout, 1, Cout_real);
+    }
+    {
+        ProfScope _ps(lc, "conv_wgrad_tc", st);
+        const bool beside = bias_out != nullptr;
+        cudaError_t e;
+        switch (g.Cout) {
+            case 16: e = wgrad_launch<16>(g, splits, beside, err, st); break;
+            case 32: e = wgrad_launch<32>(g, splits, beside, err, st); break;
+            case 64: e = wgrad_launch<64>(g, splits, beside, err, st); break;
+            case 128: e = wgrad_launch<128>(g, splits, beside, err, st); break;
+            default: e = wgrad_launch<256>(g, splits, beside, err, st); break;
+        }
+        lc.add(1);
+        if (e != cudaSuccess) return e;
     }
     ProfScope _ps(lc, "wgrad_reduce", st);
     k_wgrad_reduce<<<w.blocks + bias.blocks, 256, 0, st>>>(w, bias);
@@ -1335,10 +1357,10 @@ cudaError_t launch_output_head(int batch, int HW, int Cy, const float *y, const 
                                float *pred, void *dy, double *loss_partial, int blocks, cudaStream_t st,
                                LaunchCounter &lc) {
     ProfScope _ps(lc, "output_head", st);
-    k_output_head<<<blocks, 256, 0, st>>>(batch, HW, Cy, y, u0, target, pred, static_cast<__nv_bfloat16 *>(dy),
-                                         loss_partial);
+    const cudaError_t e = launch_pdl(k_output_head, dim3(blocks), dim3(256), 0, st, batch, HW, Cy, y, u0, target, pred,
+                                     static_cast<__nv_bfloat16 *>(dy), loss_partial);
     lc.add(1);
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_adam(size_t n, float *w, const float *grad, float *m, float *v, float lr_t, float b1, float b2,

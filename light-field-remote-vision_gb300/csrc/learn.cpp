@@ -83,7 +83,7 @@ struct lfrv_warmstart {
     long long step = 0;
     int batch = 0, H = 0, W = 0;
     lfrv::DevBuf t[lfrv::kTensors];
-    lfrv::DevBuf y, partial, bias_part, loss_part, err;
+    lfrv::DevBuf y, partial[2], bias_part[2], loss_part, err;  // [0] context stream, [1] side stream
 };
 
 namespace lfrv {
@@ -241,23 +241,34 @@ WgradGemm wgrad_gemm(const lfrv_warmstart *net, int l, int level, int &splits) {
     return g;
 }
 
-// dW and db of layer l (input x at `level`, output gradient dy) into the flat gradient, on the side stream once the
-// context stream has dy: nothing of the backward pass reads them, so they run beside the data gradients of the layers
-// below, whose grids leave half the chip idle. backward() sizes the shared partials before the first of them and joins.
+// Layers whose weight gradients the context stream computes after the last data gradient; the side stream takes the
+// others. The data gradients take about half as long as the weight gradients, so the last layers, the first's with its
+// 48 channels at full resolution the longest of all, balance the two (4 images of 256^2, the call without its copy:
+// 715 us with none, 696 with one, 678 with two, 683 with three, 694 with four).
+constexpr int kMainWgradLayers = 2;
+
+// dW and db of layer l (input x at `level`, output gradient dy) into the flat gradient, on the context stream or on the
+// side stream once the context stream has dy: nothing of the backward pass reads them, so they run beside the data
+// gradients of the layers below, whose grids leave half the chip idle. backward() sizes each stream's partials before the
+// first launch and joins.
 void conv_wgrad(lfrv_warmstart *net, int l, const void *x, int level, const void *dy) {
     const Layer &L = net->L[l];
     lfrv_ctx *c = net->ctx;
+    const int lane = l < kMainWgradLayers ? 0 : 1;
     int splits = 0;
     WgradGemm g = wgrad_gemm(net, l, level, splits);
     g.x = x;
     g.dy = dy;
-    g.partial = net->partial.as<float>();
+    g.partial = net->partial[lane].as<float>();
     float *grad = net->grads.as<float>();
-    cudaStream_t side = side_stream(c);
-    LFRV_CUDA(cudaEventRecord(c->side_fork, c->stream));
-    LFRV_CUDA(cudaStreamWaitEvent(side, c->side_fork, 0));
-    LFRV_CUDA(launch_wgrad_tc(g, splits, L.d.cout, grad + L.w_off, net->bias_part.as<float>(), kBiasBlocks,
-                              grad + L.b_off, net_err(net), side, c->launches));
+    cudaStream_t st = c->stream;
+    if (lane) {
+        st = side_stream(c);
+        LFRV_CUDA(cudaEventRecord(c->side_fork, c->stream));
+        LFRV_CUDA(cudaStreamWaitEvent(st, c->side_fork, 0));
+    }
+    LFRV_CUDA(launch_wgrad_tc(g, splits, L.d.cout, grad + L.w_off, net->bias_part[lane].as<float>(), kBiasBlocks,
+                              grad + L.b_off, net_err(net), st, c->launches));
 }
 
 void forward(lfrv_warmstart *net, const void *in) {
@@ -283,13 +294,14 @@ void backward(lfrv_warmstart *net, const void *in) {
     auto b = [&](int i) { return net->t[i].p; };
     const int B = net->batch, H = net->H, W = net->W;
     constexpr int level_of[kLayers] = {0, 0, 1, 2, 3, 3, 2, 2, 1, 1, 0, 0};  // of each layer's input
-    size_t partial = 0;
+    size_t partial[2] = {0, 0};
     for (int l = 0; l < kLayers; ++l) {
         int splits = 0;
         const WgradGemm g = wgrad_gemm(net, l, level_of[l], splits);
-        partial = std::max(partial, (size_t)splits * g.Mpad * g.Cout * sizeof(float));
+        size_t &lane = partial[l < kMainWgradLayers ? 0 : 1];
+        lane = std::max(lane, (size_t)splits * g.Mpad * g.Cout * sizeof(float));
     }
-    net->partial.ensure(partial);
+    for (int i = 0; i < 2; ++i) net->partial[i].ensure(partial[i]);
     conv_wgrad(net, 11, b(A10), level_of[11], b(DY11));
     conv_dgrad(net, 11, b(DY11), 0, nullptr, b(A10), b(G10));
     conv_wgrad(net, 10, b(S9), level_of[10], b(G10));
@@ -484,7 +496,7 @@ extern "C" int lfrv_warmstart_create(lfrv_ctx *ctx, unsigned long long seed, lfr
         net->grads.ensure(net->nparams * sizeof(float));
         net->adam_m.ensure(net->nparams * sizeof(float));
         net->adam_v.ensure(net->nparams * sizeof(float));
-        net->bias_part.ensure((size_t)kBiasBlocks * 256 * sizeof(float));
+        for (auto &buf : net->bias_part) buf.ensure((size_t)kBiasBlocks * 256 * sizeof(float));
         net->loss_part.ensure(kLossBlocks * sizeof(double));
         net->err.ensure(sizeof(int));
         LFRV_CUDA(cudaMemsetAsync(net->err.p, 0, sizeof(int), ctx->stream));
