@@ -301,6 +301,7 @@ struct ConvGemm {
     int relu;
     const void *add, *mask;
     float *outf;
+    int outf_head;  // outf holds the first four channels alone, four floats a pixel
     void *outb;
     // nearest-upsampling fusion (1 x 1 decoder layers): with upskip set, each output pixel's value v is written as
     // relu(v + upskip) to its 2 x 2 block of outb at (2 Ho) x (2 Wo), upskip being a BF16 tensor of that size

@@ -193,14 +193,21 @@ __device__ __forceinline__ void conv_load16(const ConvGemm &g, size_t row, int c
 
 // Epilogue of 16 accumulator columns (col .. col + 15) of GEMM row `row` (an output pixel, row-major over batch,
 // Ho, Wo): + bias, + add, ReLU, zero where mask <= 0, then the FP32 and / or BF16 stores. With upskip (and no addend)
-// the row's value goes, as relu(v + skip), to its 2 x 2 block of the doubled-resolution BF16 output.
+// the row's value goes, as relu(v + skip), to its 2 x 2 block of the doubled-resolution BF16 output. `bias`: the 16
+// columns' biases in shared memory.
 template <bool UP>
 __device__ __forceinline__ void conv_store16(const ConvGemm &g, size_t row, int col, float v[16],
-                                             const EpilogueIn<UP> &in) {
+                                             const EpilogueIn<UP> &in, const float *bias) {
     const size_t o = row * g.N + col;
     if (g.bias) {
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] += __ldg(g.bias + col + k);
+        for (int k = 0; k < 4; ++k) {
+            const float4 b = reinterpret_cast<const float4 *>(bias)[k];
+            v[4 * k] += b.x;
+            v[4 * k + 1] += b.y;
+            v[4 * k + 2] += b.z;
+            v[4 * k + 3] += b.w;
+        }
     }
     if constexpr (UP) {
         __nv_bfloat16 *out = static_cast<__nv_bfloat16 *>(g.outb);
@@ -242,7 +249,9 @@ __device__ __forceinline__ void conv_store16(const ConvGemm &g, size_t row, int 
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[8 + k] = tt[k] > 0.f ? v[8 + k] : 0.f;
     }
-    if (g.outf) {
+    if (g.outf && g.outf_head) {
+        if (col == 0) *reinterpret_cast<float4 *>(g.outf + row * 4) = make_float4(v[0], v[1], v[2], v[3]);
+    } else if (g.outf) {
         float4 *fp = reinterpret_cast<float4 *>(g.outf + o);
 #pragma unroll
         for (int k = 0; k < 4; ++k) fp[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
@@ -267,6 +276,7 @@ __global__ void __launch_bounds__(kThreads) k_conv_tc(const ConvGemm g, int *err
     __shared__ __align__(8) uint64_t bars[kStages];
     __shared__ uint32_t tmem_slot;
     __shared__ int s_fail;
+    __shared__ __align__(16) float s_bias[BN];
     uint8_t *base = align1024(dsm);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int M = g.batch * g.Ho * g.Wo, HWo = g.Ho * g.Wo;
@@ -325,6 +335,7 @@ __global__ void __launch_bounds__(kThreads) k_conv_tc(const ConvGemm g, int *err
     tc_fence_after();
     pdl_trigger();
     pdl_wait();
+    for (int c = tid; g.bias && c < BN; c += kThreads) s_bias[c] = __ldcg(g.bias + n0 + c);  // read after the loop's barriers
     const uint32_t tmem = tmem_slot;
     const uint32_t idesc = idesc_bf16_f32(kBM, BN);
     const int nk = (g.K + kBK - 1) / kBK;
@@ -384,7 +395,7 @@ __global__ void __launch_bounds__(kThreads) k_conv_tc(const ConvGemm g, int *err
             if (row_ok) conv_load16(g, (size_t)m, n0 + c0, in);
             tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
             if (!row_ok) continue;
-            conv_store16(g, (size_t)m, n0 + c0, v, in);
+            conv_store16(g, (size_t)m, n0 + c0, v, in, s_bias + c0);
         }
     }
     tc_fence_before();
@@ -398,7 +409,10 @@ __global__ void __launch_bounds__(kThreads) k_conv_tc(const ConvGemm g, int *err
 // (stride byte offset 128) and the 8-channel chunks are kLboA apart (leading byte offset), so the A operand of
 // tap (ky, kx) for output row i is the same tile read from pixel (i + ky) * 130 + kx on: nine shifted descriptors
 // instead of nine gathers. The weights stream per tap through a 3-slot cp.async ring. TMEM: R accumulators of BN
-// columns. Needs W % 128 == 0, H % R == 0, C % 16 == 0.
+// columns. Needs W % 128 == 0, H % R == 0, C % 16 == 0. Bound by the latency of a CTA's phases and by shared-memory
+// wavefronts: with 64 registers and 57 KB, four CTAs of 256 threads share an SM at 32 channels (one 1024^2 image, the 32 ->
+// 32 and 32 -> 16 layers: 75 and 69 us with the weights' rows 16 bytes a lane and the biases read a column at a time, 69
+// and 57 now).
 constexpr int kTileW = 130, kTapStages = 3;
 constexpr int kEpiThreads = 256;  // two groups of four warps share an epilogue (a warp reads TMEM lanes 32 (w % 4) ..)
 
@@ -412,7 +426,8 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tile_tc(const ConvGemm g, 
     __shared__ __align__(8) uint64_t bars[kTapStages];
     __shared__ uint32_t tmem_slot;
     __shared__ int s_fail;
-    uint8_t *base = align1024(dsm);
+    __shared__ __align__(16) float s_bias[BN];
+    uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(dsm) + 127) & ~(uintptr_t)127);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int C = g.C, chunks = C >> 3;
     const int strips = g.Wo >> 7, yblocks = g.Ho / R;
@@ -423,7 +438,8 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tile_tc(const ConvGemm g, 
     const int x0 = strip << 7, y0 = yb * R, n0 = blockIdx.y * BN;
     const uint32_t lboA = (uint32_t)lbo_px * 16u;
     const uint32_t sA = smem_u32(base), sB = sA + (uint32_t)chunks * lboA;
-    const uint32_t bstage = (uint32_t)BN * (uint32_t)C * 2u;  // bytes of one tap's weights
+    constexpr uint32_t kLboB = (BN + 2) * 16;
+    const uint32_t bstage = (uint32_t)chunks * kLboB;  // one tap's weights
     if (warp == 0) tmem_alloc(&tmem_slot, kCols);
     if (tid == 0) {
         for (int s = 0; s < kTapStages; ++s) mbar_init(&bars[s], 1);
@@ -435,6 +451,7 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tile_tc(const ConvGemm g, 
     tc_fence_after();
     pdl_trigger();
     pdl_wait();
+    if (g.bias && tid < BN) s_bias[tid] = __ldcg(g.bias + n0 + tid);  // read after the loop's barriers
     const __nv_bfloat16 *src = static_cast<const __nv_bfloat16 *>(g.src);
     const __nv_bfloat16 *wt = static_cast<const __nv_bfloat16 *>(g.wt);
     // the input tile (zero outside the image): thread q -> pixel q / chunks of a row, chunk q % chunks (coalesced reads), in
@@ -461,12 +478,19 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tile_tc(const ConvGemm g, 
         }
     }
     cp_async_commit();
-    // one tap's weights: B[n][c] = wt[n0 + n][tap * C + c], chunk-major (chunk j at j * BN * 16, row n at n * 16)
+    // one tap's weights: B[n][c] = wt[n0 + n][tap * C + c], chunk-major (chunk j at j * kLboB, row n at n * 16). Adjacent
+    // threads take adjacent chunks of a row; the two rows of padding of a plane put four chunks of two rows, a quarter
+    // warp's, in different banks
+    const int wn = tid / chunks, wj = tid - wn * chunks;
     auto load_tap = [&](int t, int slot) {
         const uint32_t dst = sB + (uint32_t)slot * bstage;
+        int n = wn, j = wj;
         for (int q = tid; q < BN * chunks; q += kEpiThreads) {
-            const int n = q % BN, j = q / BN;
-            cp_async16(dst + (uint32_t)(j * BN + n) * 16u, wt + (size_t)(n0 + n) * g.ldw + t * C + j * 8, 16);
+            cp_async16(dst + (uint32_t)j * kLboB + (uint32_t)n * 16u, wt + (size_t)(n0 + n) * g.ldw + t * C + j * 8, 16);
+            if (BN * chunks > kEpiThreads) {
+                n = (q + kEpiThreads) / chunks;
+                j = q + kEpiThreads - n * chunks;
+            }
         }
     };
     load_tap(0, 0);
@@ -492,7 +516,7 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tile_tc(const ConvGemm g, 
                 const uint32_t a0 = sA + (uint32_t)((i + sy) * kTileW + sx) * 16u;
                 for (int s = 0; s < C / 16; ++s)
                     tc_mma(tmem + (uint32_t)(i * BN), smem_desc(a0 + (uint32_t)(2 * s) * lboA, lboA, 128),
-                           smem_desc(bb + (uint32_t)(2 * s) * (uint32_t)BN * 16u, (uint32_t)BN * 16u, 128), idesc,
+                           smem_desc(bb + (uint32_t)(2 * s) * kLboB, kLboB, 128), idesc,
                            (t > 0 || s > 0) ? 1 : 0);
             }
             tc_commit(&bars[t % kTapStages]);
@@ -524,7 +548,7 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tile_tc(const ConvGemm g, 
         for (int u = warp >> 2; u < kUnits; u += 2) {
             float v[16];
             tc_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(u * 16), v);
-            conv_store16(g, unit_row(u), unit_col(u), v, in);
+            conv_store16(g, unit_row(u), unit_col(u), v, in, s_bias + u % (BN / 16) * 16);
             if (u + 2 < kUnits) conv_load16(g, unit_row(u + 2), unit_col(u + 2), in);
         }
     }
@@ -569,6 +593,7 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tma(const ConvGemm g, cons
     __shared__ __align__(8) uint64_t full[kTmaMaxStages], empty[kTmaMaxStages], done;
     __shared__ uint32_t tmem_slot;
     __shared__ int s_fail;
+    __shared__ __align__(16) float s_bias[BN];
     uint8_t *base = align1024(dsm);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gw = PARITY ? g.Ws : g.Wo, gh = PARITY ? g.Hs : g.Ho;  // the grid that is cut into patches
@@ -602,6 +627,7 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tma(const ConvGemm g, cons
     tc_fence_after();
     pdl_trigger();
     pdl_wait();
+    if (g.bias && tid < BN) s_bias[tid] = __ldcg(g.bias + n0 + tid);  // read after the loop's barriers
     EpilogueIn<UP> in;
     if ((warp >> 2) * 16 < BN) conv_load16(g, row, n0 + (warp >> 2) * 16, in);
     const uint32_t tmem = tmem_slot;
@@ -670,7 +696,7 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tma(const ConvGemm g, cons
         for (int c0 = (warp >> 2) * 16; c0 < BN; c0 += 32) {
             float v[16];
             tc_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
-            conv_store16(g, row, n0 + c0, v, in);
+            conv_store16(g, row, n0 + c0, v, in, s_bias + c0);
             if (c0 + 32 < BN) conv_load16(g, row, n0 + c0 + 32, in);
         }
     }
@@ -974,10 +1000,11 @@ __global__ void k_down_sum(int batch, int Hl, int Wl, int C, const __nv_bfloat16
     }
 }
 
-// Output head: pred = u0 + y[:, 0:3] (planar per image), and with a target the loss 1/(3 P) sum (pred - target)^2,
+// Output head: pred = u0 + y[:, 0:3] (y: four floats a pixel; pred planar per image), and with a target the loss 1/(3 P) sum (pred - target)^2,
 // its gradient dy = 2 (pred - target) / (3 P) as BF16 [P][Cy] (zero in the padding channels), per-block loss
 // partials in FP64.
-__global__ void __launch_bounds__(256) k_output_head(int batch, int HW, int Cy, const float *__restrict__ y,
+template <bool LOSS>
+__global__ void __launch_bounds__(256) k_output_head(int batch, int HW, int Cy, const float4 *__restrict__ y,
                                                      const float *__restrict__ u0, const float *__restrict__ target,
                                                      float *__restrict__ pred, __nv_bfloat16 *__restrict__ dy,
                                                      double *__restrict__ loss_partial) {
@@ -988,24 +1015,28 @@ __global__ void __launch_bounds__(256) k_output_head(int batch, int HW, int Cy, 
     double acc = 0.0;
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < P; p += (size_t)gridDim.x * blockDim.x) {
         const size_t b = p / HW, o = p - b * HW;
+        const float4 yp = __ldcg(y + p);
+        const float yc[3] = {yp.x, yp.y, yp.z};
         float d[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const size_t q = (b * 3 + c) * HW + o;
-            const float v = u0[q] + y[p * Cy + c];
+            const float v = u0[q] + yc[c];
             if (pred) pred[q] = v;
-            d[c] = target ? v - target[q] : 0.f;
-            acc += (double)d[c] * d[c];
+            if constexpr (LOSS) {
+                d[c] = v - target[q];
+                acc += (double)d[c] * d[c];
+            }
         }
-        if (dy) {
+        if constexpr (LOSS) {
             const float f[8] = {d[0] * scale, d[1] * scale, d[2] * scale, 0.f, 0.f, 0.f, 0.f, 0.f};
             uint4 *row = reinterpret_cast<uint4 *>(dy + p * Cy);
             row[0] = pack8(f);
             for (int c = 1; c < Cy / 8; ++c) row[c] = make_uint4(0, 0, 0, 0);
         }
     }
-    acc = block_sum<256>(acc, sh);
-    if (threadIdx.x == 0 && loss_partial) loss_partial[blockIdx.x] = acc;
+    if constexpr (LOSS) acc = block_sum<256>(acc, sh);
+    if (LOSS && threadIdx.x == 0) loss_partial[blockIdx.x] = acc;
 }
 
 // Adam on the flat FP32 parameters (bias-corrected step sizes computed on the host).
@@ -1101,7 +1132,7 @@ static bool tile_shape(const ConvGemm &g, int &R, int &BN, int &smem) {
         if (g.Ho % r) continue;
         for (int bn = g.N; bn >= 16 && bn >= g.N / 2; bn >>= 1) {
             if (r * bn > 256 || bn > 128) continue;
-            const int sm = (g.C / 8) * tile_lbo_px(r) * 16 + kTapStages * bn * g.C * 2 + 1024;
+            const int sm = (g.C / 8) * tile_lbo_px(r) * 16 + kTapStages * (g.C / 8) * (bn + 2) * 16 + 128;
             if (sm > 200 * 1024) continue;
             const int ctas = g.batch * (g.Ho / r) * (g.Wo / 128) * (g.N / bn);
             const int score = std::min(ctas, 2 * 148);
@@ -1357,8 +1388,12 @@ cudaError_t launch_output_head(int batch, int HW, int Cy, const float *y, const 
                                float *pred, void *dy, double *loss_partial, int blocks, cudaStream_t st,
                                LaunchCounter &lc) {
     ProfScope _ps(lc, "output_head", st);
-    const cudaError_t e = launch_pdl(k_output_head, dim3(blocks), dim3(256), 0, st, batch, HW, Cy, y, u0, target, pred,
-                                     static_cast<__nv_bfloat16 *>(dy), loss_partial);
+    // `blocks` loss partials; without a target there is no FP64 sum and a thread takes one pixel (1024^2: 20 us with the
+    // sum of zeros and 304 blocks, 10 now)
+    const float4 *y4 = reinterpret_cast<const float4 *>(y);
+    const int nb = target ? blocks : (int)(((size_t)batch * HW + 255) / 256);
+    const cudaError_t e = launch_pdl(target ? k_output_head<true> : k_output_head<false>, dim3(nb), dim3(256), 0, st, batch,
+                                     HW, Cy, y4, u0, target, pred, static_cast<__nv_bfloat16 *>(dy), loss_partial);
     lc.add(1);
     return e;
 }

@@ -157,7 +157,7 @@ void net_shape(lfrv_warmstart *net, int batch, int H, int W) {
         const size_t px = (size_t)batch * (H >> kTensorL[i]) * (W >> kTensorL[i]);
         net->t[i].ensure(px * kTensorC[i] * 2);
     }
-    net->y.ensure((size_t)batch * H * W * 16 * sizeof(float));
+    net->y.ensure((size_t)batch * H * W * 4 * sizeof(float));
     net->batch = batch;
     net->H = H;
     net->W = W;
@@ -189,6 +189,7 @@ void conv_forward(lfrv_warmstart *net, int l, const void *x, int level, void *ou
     g.relu = L.d.relu;
     g.outb = outb;
     g.outf = outf;
+    g.outf_head = 1;  // the last layer's three channels
     g.upskip = upskip;
     LFRV_CUDA(launch_conv_tc(g, net_err(net), net->ctx->stream, net->ctx->launches));
 }
