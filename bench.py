@@ -101,7 +101,6 @@ def algorithmic_bytes(kernel: str, V: int, n: int, N: int, ks: int, cg_iters: in
         "vis_any": 4 * N + 8 * V * n + 4 * V * n + 1 * N,
         "initial_image": 24 * V * n + 4 * V * n + 4 * N + 16 * N,
         "hole_list": 1 * N,
-        "hole_fill_iter": None,
         "sobel": 12 * V * n + 8 * V * n,
         "u_gradient": (8 + 4 + 8) * V * n + 4 * V * n + 4 * N + 12 * N,
         # start: U, g read, r and d written; five iterations: d read, q written; U, r, d, q read, U, r, d written
@@ -111,9 +110,9 @@ def algorithmic_bytes(kernel: str, V: int, n: int, N: int, ks: int, cg_iters: in
         # all inner iterations of one ISTA step in one launch: 88 B per target pixel per iteration
         "rof_persistent": 88 * N * rof_iters,
         "residual": 12 * N + 24 * V * n + 12 * V * n,
-        # the FGP iterations of one FISTA step in one launch; per iteration the FP64 dual p and momentum q (48 B
-        # each), F (12), lam, 1/L, g (4 each) read and p, q written (96): 216 B per target pixel (FP32 and
-        # double-float arithmetic of the dual both keep FP64 storage)
+        # the FGP iterations of one FISTA step in one launch; per iteration the dual p and momentum q as float pairs
+        # (48 B each), F (12), lam, 1/L, g (4 each) read and p, q written (96): 216 B per target pixel (FP32 and
+        # double-float arithmetic of the dual both keep the pairs)
         "tv_fgp": 200 * 216 * N,
         "tv_fgp_df": 200 * 216 * N,
         "dataterm_F": 12 * V * n + 8 * V * n + 4 * V * n + 12 * N + 12 * N,
@@ -127,8 +126,8 @@ def algorithmic_bytes(kernel: str, V: int, n: int, N: int, ks: int, cg_iters: in
 # bytes (at C2 its traffic is 1.03 x its algorithmic bytes: depth maps read once, keys in L2).
 NCU_TRAFFIC_BYTES = {
     ("zbuffer_splat", 1024 * 1024): 83.942912e6 + 2.418432e6 + 0.335616e6,
-    ("gradient_setup", 1024 * 1024): 223.959296e6 + 18.378240e6,
-    ("cg_persistent", 1024 * 1024): 21.045248e6 + 0.000512e6,
+    ("gradient_setup", 1024 * 1024): 221.8e6 + 15.8e6,
+    ("cg_persistent", 1024 * 1024): 21.1e6 + 0.1e6,
     ("zbuffer_splat", 2048 * 2048): 1.03 * (12 * 80 * 1024 * 1024 + 8 * 2048 * 2048),
     ("rof_persistent", 256 * 256): 3.427584e6 + 0.028928e6,
 }
@@ -792,12 +791,12 @@ def roofline_of(prof: dict, V: int, n: int, N: int, ks: int, stats, rof_iters, t
             roof["dram_frac"] = roof["traffic"] / avg_s / 1e9 / peak
         # what bounds the kernel instead of HBM, from its ncu capture
         roof["limiter"] = {
-            "cg_persistent": "two grid barriers per iteration and the FP64 block sums before them; r and d stay in "
-                             "shared memory, so DRAM moves only the one-time read of g and u",
+            "cg_persistent": "one grid barrier per iteration with the block sums and the FP64 scalars beside it; r, s, x "
+                             "and d stay on chip, so DRAM moves only the one-time read of g and u",
             "zbuffer_splat": "instruction issue (75% issue active): per source pixel four projected corners, a "
                              "two-triangle set-up and the coverage and depth of its pixel centres; DRAM traffic is "
                              "the algorithmic bytes",
-            "gradient_setup": "latency of dependent gathers at 24% occupancy (63 register partials per lane)",
+            "gradient_setup": "latency of the gathers in flight (28 register partials per lane)",
             "rof_persistent": "block barriers between the dual and primal phases and the grid barrier per super-step; "
                               "the working set is L2-resident",
         }.get(dom)

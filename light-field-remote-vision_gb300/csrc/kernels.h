@@ -165,8 +165,6 @@ void launch_push_pull(int W, int H, bool faithful, const uint8_t *vis, float *U,
                       LaunchCounter &lc);
 
 // ---- IBR_gradient: hole filling and CG (kernels_cg.cu)
-void launch_hole_fill_iter(int W, int H, const int *holes, int nholes, const float *Uin, float *Uout,
-                           double *partial, cudaStream_t st, LaunchCounter &lc);
 int hole_fill_partials(int nholes);
 void launch_hole_list(int W, int H, const uint8_t *vis, int *holes, int *count, cudaStream_t st, LaunchCounter &lc);
 int cg_partials(int W, int H);
@@ -326,8 +324,6 @@ void set_conv_kernel_pref(int pref);
 // dW into grad and, unless bias_out is null, db = the column sums of dy (bias_partial: bias_blocks x Cout floats).
 cudaError_t launch_wgrad_tc(const WgradGemm &g, int splits, int Cout_real, float *grad, float *bias_partial,
                             int bias_blocks, float *bias_out, int *err, cudaStream_t st, LaunchCounter &lc);
-cudaError_t launch_upsample_add_relu(int batch, int Hl, int Wl, int C, const void *t, const void *skip, void *s,
-                                     cudaStream_t st, LaunchCounter &lc);
 cudaError_t launch_down_sum(int batch, int Hl, int Wl, int C, const void *ds, void *dt, cudaStream_t st,
                             LaunchCounter &lc);
 cudaError_t launch_output_head(int batch, int HW, int Cy, const float *y, const float *u0, const float *target,

@@ -134,37 +134,6 @@ __global__ void k_hole_write(int W, int H, const uint8_t *__restrict__ vis, cons
     }
 }
 
-// One Jacobi step on the holes; partial = sum over holes of lap * U_new for channel 2 (the reference keeps
-// the energy of the last channel).
-__global__ void __launch_bounds__(256) k_hole_iter(int W, int H, const int *__restrict__ holes, int nholes,
-                                                   const float *__restrict__ Uin, float *__restrict__ Uout,
-                                                   double *__restrict__ partial) {
-    __shared__ double red[8];
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t N = (size_t)W * H;
-    double e = 0.0;
-    if (k < nholes) {
-        const int o = holes[k];
-        const int ox = o % W, oy = o / W;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const float *u = Uin + c * N;
-            float v = 0.f, wt = 0.f;
-            if (ox > 0) { v += u[o - 1]; wt += 1.f; }
-            if (oy > 0) { v += u[o - W]; wt += 1.f; }
-            if (ox < W - 1) { v += u[o + 1]; wt += 1.f; }
-            if (oy < H - 1) { v += u[o + W]; wt += 1.f; }
-            v /= wt;
-            const float lap = v - u[o];
-            const float un = u[o] + lap;
-            Uout[c * N + o] = un;
-            if (c == 2) e = (double)(lap * un);
-        }
-    }
-    const double s = block_sum<256>(e, red);
-    if (threadIdx.x == 0) partial[blockIdx.x] = s;
-}
-
 // ------------------------------------------------------------------ conjugate gradient
 constexpr int kCgBX = 32, kCgBY = 8;
 
@@ -380,7 +349,7 @@ __device__ __forceinline__ float ldcg_op(const float *d, int W, int H, int x, in
 // alpha + r . r after each, r0 . r0 counting the last row twice. Two grid barriers an iteration: after q = A d with d . q,
 // and after the update of u, r and d with r . r. state: [0..2] r0 . r0, [3..5] dAlpha, carried from launch to launch.
 // Bound by the barriers at small images and by the streams of r, d, q and U at large ones; the scalars stay on the device
-// because a copy back for each (11 of them) cost more than the arithmetic: a whole call with host arrays, 9 views of 256^2,
+// because a copy back for each (11 of them) cost more than the arithmetic: a whole call with host arrays, 8 views of 256^2,
 // took 607 us with host-stepped kernels and takes 375 us.
 __global__ void __launch_bounds__(kPersistThreads) k_cg_faithful(int W, int H, const float *__restrict__ gX,
                                                                  const float *__restrict__ gY, float *U, float *r,
@@ -1862,14 +1831,6 @@ cudaError_t launch_hole_fill_persistent(int W, int H, const int *holes, const in
     lc.add(1);
     return cudaLaunchCooperativeKernel((const void *)k_hole_fill_persistent, dim3(blocks), dim3(kPersistThreads), args,
                                        0, st);
-}
-
-void launch_hole_fill_iter(int W, int H, const int *holes, int nholes, const float *Uin, float *Uout, double *partial,
-                           cudaStream_t st, LaunchCounter &lc) {
-    ProfScope _ps(lc, "hole_fill_iter", st);
-    if (nholes <= 0) return;
-    k_hole_iter<<<(nholes + 255) / 256, 256, 0, st>>>(W, H, holes, nholes, Uin, Uout, partial);
-    lc.add(1);
 }
 
 void launch_cg_energy(int W, int H, const float *U, const float *U0, const float *gx, const float *gy, double *partial,

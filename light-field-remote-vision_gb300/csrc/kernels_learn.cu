@@ -956,27 +956,6 @@ __global__ void __launch_bounds__(256) k_wgrad_reduce(const ReducePart w, const 
     }
 }
 
-// s = relu(up2(t) + skip): t at (Hl, Wl), skip and s at (2 Hl, 2 Wl), C channels (8 per thread).
-__global__ void k_upsample_add_relu(int batch, int Hl, int Wl, int C, const __nv_bfloat16 *__restrict__ t,
-                                    const __nv_bfloat16 *__restrict__ skip, __nv_bfloat16 *__restrict__ s) {
-    const int C8 = C >> 3, W = 2 * Wl, H = 2 * Hl;
-    const size_t total = (size_t)batch * H * W * C8;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int c8 = (int)(i % C8);
-        const size_t pix = i / C8;
-        const int x = (int)(pix % W);
-        const size_t r = pix / W;
-        const int y = (int)(r % H), b = (int)(r / H);
-        const size_t lo = (((size_t)b * Hl + (y >> 1)) * Wl + (x >> 1)) * C + c8 * 8;
-        float a[8], k[8];
-        unpack8(*reinterpret_cast<const uint4 *>(t + lo), a);
-        unpack8(*reinterpret_cast<const uint4 *>(skip + pix * C + c8 * 8), k);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = fmaxf(a[j] + k[j], 0.f);
-        *reinterpret_cast<uint4 *>(s + pix * C + c8 * 8) = pack8(a);
-    }
-}
-
 // dt = sum of the 2 x 2 block of ds (the adjoint of nearest upsampling).
 __global__ void k_down_sum(int batch, int Hl, int Wl, int C, const __nv_bfloat16 *__restrict__ ds,
                            __nv_bfloat16 *__restrict__ dt) {
@@ -1362,17 +1341,6 @@ cudaError_t launch_wgrad_tc(const WgradGemm &g, int splits, int Cout_real, float
 }
 
 static int ew_blocks(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 152 * 16); }
-
-cudaError_t launch_upsample_add_relu(int batch, int Hl, int Wl, int C, const void *t, const void *skip, void *s,
-                                     cudaStream_t st, LaunchCounter &lc) {
-    ProfScope _ps(lc, "upsample_add", st);
-    const size_t n = (size_t)batch * 4 * Hl * Wl * (C / 8);
-    k_upsample_add_relu<<<ew_blocks(n), 256, 0, st>>>(batch, Hl, Wl, C, static_cast<const __nv_bfloat16 *>(t),
-                                                     static_cast<const __nv_bfloat16 *>(skip),
-                                                     static_cast<__nv_bfloat16 *>(s));
-    lc.add(1);
-    return cudaGetLastError();
-}
 
 cudaError_t launch_down_sum(int batch, int Hl, int Wl, int C, const void *ds, void *dt, cudaStream_t st,
                             LaunchCounter &lc) {

@@ -1354,12 +1354,6 @@ __global__ void k_trace_energy(const double *__restrict__ sums, float lambda, fl
     *dst = (double)e;
 }
 
-// Elementwise helpers.
-__global__ void k_fill_u8(size_t n, uint8_t *p, uint8_t v) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
-}
-
 __global__ void k_premultiply_dpart(int V, int n, const float *__restrict__ dpart3, int dpart_channels,
                                     float *__restrict__ dp) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
