@@ -1120,21 +1120,23 @@ constexpr int kSmallHoles = 2048, kSmallThreads = 1024, kHoleCluster = 8;
 static_assert(kSmallHoles == 1 << 11 && kHoleCluster * kSmallHoles <= 32767, "hole references are 16-bit");
 constexpr size_t kSmallHoleSmem = (size_t)kSmallHoles * (6 * 4 + 12 * 4 + 4 * 2 + 4);
 
+// Shared arrays of a block besides the dynamic ones.
+struct HoleShared {
+    float rws[kSmallHoles];  // 1 / wts
+    float wsum[2][kSmallThreads / 32];
+    int holes[kSmallHoles];
+};
+
 template <int C>
-__global__ void __launch_bounds__(kSmallThreads) k_hole_fill_small(int W, int H, const int *__restrict__ holes,
-                                                                   const int *__restrict__ count, float *A,
-                                                                   int max_iter, double *state) {
-    const int nh = *count;
-    // the sizes this form takes (every block of a cluster returns together, before any cluster barrier)
-    if (nh > C * kSmallHoles || (C > 1 && nh <= kSmallHoles)) return;
-    extern __shared__ __align__(16) float hsm[];
+__device__ __forceinline__ void hole_fill_small(int W, int H, const int *__restrict__ holes, int nh, float *A, int max_iter,
+                                                double *state, float *hsm, HoleShared &sh) {
     float *cur = hsm, *nxt = hsm + 3 * kSmallHoles;            // [3][kSmallHoles] each
     float *fixedv = hsm + 6 * kSmallHoles;                      // [4 dirs][3][kSmallHoles]
     float *wts = hsm + 18 * kSmallHoles;                        // [kSmallHoles]
-    __shared__ float rws[kSmallHoles];                          // 1 / wts
     short *nb = reinterpret_cast<short *>(hsm + 19 * kSmallHoles);  // [4][kSmallHoles]: reference, -1 fixed, -2 none
-    __shared__ float wsum[2][kSmallThreads / 32];
-    __shared__ int s_holes[kSmallHoles];
+    float *rws = sh.rws;
+    float(&wsum)[2][kSmallThreads / 32] = sh.wsum;
+    int *s_holes = sh.holes;
     const int rank = C > 1 ? (int)cg::this_cluster().block_rank() : 0;
     const int chunk = (nh + C - 1) / C, h0 = rank * chunk, nloc = max(0, min(nh - h0, chunk));
     const size_t N = (size_t)W * H;
@@ -1277,6 +1279,22 @@ __global__ void __launch_bounds__(kSmallThreads) k_hole_fill_small(int W, int H,
     if (rank == 0 && threadIdx.x == 0) state[0] = (double)k;
     // no block leaves while another may still read its shared memory
     if constexpr (C > 1) cg::this_cluster().sync();
+}
+
+// C = 1: at most kSmallHoles holes. C > 1: at most C times as many; the first block alone fills what one block holds (its
+// barrier is the cheaper one), so that one launch serves both ranges: a second one that finds nothing to do took 2 to 5 us
+// of a render (64^2 137 -> 135 us, 24 views of 301 x 203 241 -> 236).
+template <int C>
+__global__ void __launch_bounds__(kSmallThreads) k_hole_fill_small(int W, int H, const int *__restrict__ holes,
+                                                                   const int *__restrict__ count, float *A,
+                                                                   int max_iter, double *state) {
+    extern __shared__ __align__(16) float hsm[];
+    __shared__ HoleShared sh;
+    const int nh = *count;
+    // every block of a cluster returns together, before any cluster barrier
+    if (nh > C * kSmallHoles) return;
+    if (C > 1 && nh > kSmallHoles) hole_fill_small<C>(W, H, holes, nh, A, max_iter, state, hsm, sh);
+    else if (blockIdx.x == 0) hole_fill_small<1>(W, H, holes, nh, A, max_iter, state, hsm, sh);
 }
 
 // Hole filling with the whole iteration loop in one launch (hole_filling, sources/gradientIBR.cu:87-152).
@@ -1756,9 +1774,9 @@ bool encode_tensor_map_3d(CUtensorMap *map, const float *base, int cols, int row
 cudaError_t launch_hole_fill_persistent(int W, int H, const int *holes, const int *count, float *A, float *B,
                                         double *part, GridBarrier gb, int max_iter, double *state, cudaStream_t st,
                                         LaunchCounter &lc) {
-    // The hole count is on the device: the three forms are queued, and each returns at once unless the count is
-    // in its range (one block up to kSmallHoles, one cluster of kHoleCluster blocks up to kHoleCluster times that
-    // where the device can place such a cluster, the grid-wide kernel above).
+    // The hole count is on the device: the shared-memory form (one cluster of kHoleCluster blocks, where the device can
+    // place one, whose first block alone fills what one block holds; else one block) and the grid-wide kernel are both
+    // queued, and each returns at once unless the count is in its range.
     int handled = kSmallHoles;
     {
         ProfScope _ps(lc, "hole_fill_small", st);
@@ -1800,10 +1818,7 @@ cudaError_t launch_hole_fill_persistent(int W, int H, const int *holes, const in
             }
             use_cluster = cluster_ok[slot] > 0;
         }
-        k_hole_fill_small<1><<<1, kSmallThreads, kSmallHoleSmem, st>>>(W, H, holes, count, A, max_iter, state);
-        lc.add(1);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+        cudaError_t e;
         if (use_cluster) {
             cudaLaunchConfig_t q = {};
             cudaLaunchAttribute at[1];
@@ -1818,10 +1833,13 @@ cudaError_t launch_hole_fill_persistent(int W, int H, const int *holes, const in
             q.attrs = at;
             q.numAttrs = 1;
             e = cudaLaunchKernelEx(&q, k_hole_fill_small<kHoleCluster>, W, H, holes, count, A, max_iter, state);
-            if (e != cudaSuccess) return e;
-            lc.add(1);
             handled = kHoleCluster * kSmallHoles;
+        } else {
+            k_hole_fill_small<1><<<1, kSmallThreads, kSmallHoleSmem, st>>>(W, H, holes, count, A, max_iter, state);
+            e = cudaGetLastError();
         }
+        if (e != cudaSuccess) return e;
+        lc.add(1);
     }
     ProfScope _ps(lc, "hole_fill", st);
     const size_t N = (size_t)W * H;
