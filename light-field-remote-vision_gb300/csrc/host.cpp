@@ -13,6 +13,7 @@
 //   D1 the CG loop of possion_conj_grad (beta == 1, alpha accumulator never cleared, 5 iterations).
 // D2 (the FISTA extrapolation is overwritten by the next step, optimization.cu:1765-1767) never changes
 // the result, so the extrapolation is not computed; the iterate simply advances.
+#include "batch_layout.h"
 #include "context.h"
 
 #include <algorithm>
@@ -1963,8 +1964,8 @@ extern "C" int lfrv_render_view_warm_dev(lfrv_ctx *ctx, lfrv_warmstart *net, con
 
 // ====================================================================== batched targets
 // IBR_gradient jobs with the corrected CG share k_cg_strip launches (each as many jobs as fit on chip together); every
-// other job runs on its own. Per gradient job the batch pool holds U, gx, gy, r, dA, dB (14 N
-// floats) and 8 doubles of state.
+// other job runs on its own. batch_layout.h says what the pool holds per gradient
+// job.
 // Host-buffer calls pass host_out (per job: a pinned host destination, or nullptr) and sent (per job, zeroed): an
 // IBR_gradient job's output is then copied to host_out as soon as its CG is done, on the copy stream, while the next
 // jobs run, and sent[job] is set. views_ready (or nullptr): an event the jobs wait for before they read their colour
@@ -1978,7 +1979,8 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
         int job;
         Geometry G;
         size_t off;  // float offset of the job's buffers in the pool
-        bool seeded;  // the learned warm start seeds its CG (seed at 14 N + 16, network input after it)
+        bool seeded;  // the learned warm start seeds its CG
+        BatchLayout at;
     };
     if (net && warmstart_ctx(net) != c) raise(LFRV_E_ARG, "the warm-start network belongs to another context");
     std::vector<Slot> batched;
@@ -1997,9 +1999,8 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
             check_solver_options(*J.cfg);
             if (G.W < 2 || G.H < 2) raise(LFRV_E_ARG, "job %d: target smaller than 2 x 2", j);
             const bool seeded = net && G.W % 8 == 0 && G.H % 8 == 0;
-            batched.push_back({j, G, pool, seeded});
-            pool += 14 * G.N + 16;  // + 8 doubles of state, kept 64-byte aligned by the 16-float pad
-            if (seeded) pool += 3 * G.N + (G.N * kLearnChannels * 2 + 63) / 64 * 16;  // seed + BF16 input
+            batched.push_back({j, G, pool, seeded, batch_layout(G.N, seeded, kLearnChannels)});
+            pool += batched.back().at.size;
         }
     }
     ws.batch.ensure(sizeof(float) * std::max<size_t>(pool, 16));
@@ -2112,13 +2113,13 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
         // k_tau counts the inverse map's buckets as it writes tau (no separate count pass)
         warp(l, G.V, G.w, G.h, J.d_depth, J.cams, J.target, nullptr, nullptr, lw.tau.as<float>(), nullptr, nullptr,
              nullptr, &G);
-        float *U = base + sl.off;
+        float *job = base + sl.off, *U = job + sl.at.U;
         // the shared view gradients are written (and so the views are uploaded, which the context stream waited for)
         LFRV_CUDA(cudaStreamWaitEvent(l->stream, c->vg_ready, 0));
-        gradient_prepare(l, *J.cfg, G, J.d_views, lw.tau.as<float>(), nullptr, nullptr, U, U + 3 * G.N, U + 4 * G.N,
-                         sl.seeded ? U + 17 * G.N + 16 : nullptr, nullptr, ws.vg_pool.as<char>() + vg_off[q]);
+        gradient_prepare(l, *J.cfg, G, J.d_views, lw.tau.as<float>(), nullptr, nullptr, U, job + sl.at.gx, job + sl.at.gy,
+                         sl.seeded ? job + sl.at.input : nullptr, nullptr, ws.vg_pool.as<char>() + vg_off[q]);
         // keep this job's hole-fill iteration count (state slot 8) beside its CG state
-        double *st = reinterpret_cast<double *>(U + 14 * G.N);
+        double *st = reinterpret_cast<double *>(job + sl.at.state);
         LFRV_CUDA(cudaMemcpyAsync(st + 6, lw.state.as<double>() + 8, sizeof(double), cudaMemcpyDeviceToDevice,
                                   l->stream));
     }
@@ -2155,8 +2156,8 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
     // seeds of the warm-started jobs: the network, one target after another on the context stream
     for (const Slot &sl : batched)
         if (sl.seeded) {
-            float *U = base + sl.off;
-            warmstart_predict_async(net, sl.G.H, sl.G.W, U + 17 * sl.G.N + 16, U, U + 14 * sl.G.N + 16);
+            float *job = base + sl.off;
+            warmstart_predict_async(net, sl.G.H, sl.G.W, job + sl.at.input, job + sl.at.U, job + sl.at.seed);
         }
     // energy traces of the batched jobs: one region of ws.trace per job that asks for one
     std::vector<size_t> trace_off(batched.size(), 0);
@@ -2171,13 +2172,15 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
     // too large for it): it runs the single-target CG on its pool buffers, one after another on the context stream.
     // The others share launches of as many jobs as fit the GPU together.
     const int resident = cg_batch_resident_blocks();
+    // the CG's iterate, which holds a job's output: the seed's buffer, or U
+    auto result = [](const Slot &sl) { return sl.seeded ? sl.at.seed : sl.at.U; };
     // a job's final output (the CG's iterate) to its host destination, after what the context stream has queued
     auto send = [&](const Slot &sl) {
         if (!host_out || !host_out[sl.job] || !sent) return;
         cudaStream_t cs = copy_stream(c);
         LFRV_CUDA(cudaEventRecord(c->out_ready, s));
         LFRV_CUDA(cudaStreamWaitEvent(cs, c->out_ready, 0));
-        LFRV_CUDA(cudaMemcpyAsync(host_out[sl.job], base + sl.off + (sl.seeded ? 14 * sl.G.N + 16 : 0),
+        LFRV_CUDA(cudaMemcpyAsync(host_out[sl.job], base + sl.off + result(sl),
                                   sizeof(float) * 3 * sl.G.N, cudaMemcpyDeviceToHost, cs));
         sent[sl.job] = 1;
     };
@@ -2192,15 +2195,14 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
         const lfrv_config &cfg = *jobs[sl.job].cfg;
         const lfrv_stats *jst = jobs[sl.job].stats;
         const bool traced = jst && jst->energy_trace && jst->trace_capacity > 0;
-        float *U = base + sl.off;
-        const size_t N = sl.G.N;
+        float *job = base + sl.off;
         const size_t np = (size_t)persistent_partials();
         double *part = partial_buf(c, 8 * np);
         const GridBarrier gb = fresh_barrier(c);
-        LFRV_CUDA(launch_cg_persistent(sl.G.W, sl.G.H, U + 3 * N, U + 4 * N, sl.seeded ? U + 14 * N + 16 : U,
-                                       U + 5 * N, U + 8 * N, U + 11 * N, part, part + 4 * np, gb, cfg.cg_max_iter,
-                                       cfg.cg_gap_tol, reinterpret_cast<double *>(U + 14 * N), s, c->launches,
-                                       sl.seeded ? U : nullptr, traced ? ws.trace.as<double>() + trace_off[q] : nullptr,
+        LFRV_CUDA(launch_cg_persistent(sl.G.W, sl.G.H, job + sl.at.gx, job + sl.at.gy, job + result(sl), job + sl.at.r,
+                                       job + sl.at.dA, job + sl.at.dB, part, part + 4 * np, gb, cfg.cg_max_iter,
+                                       cfg.cg_gap_tol, reinterpret_cast<double *>(job + sl.at.state), s, c->launches,
+                                       sl.seeded ? job + sl.at.U : nullptr, traced ? ws.trace.as<double>() + trace_off[q] : nullptr,
                                        traced ? jst->trace_capacity : 0));
         check_launch("batched job CG");
         send(sl);
@@ -2216,20 +2218,20 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
     for (size_t q = 0; q < grouped.size(); ++q) {
         const Slot &sl = batched[grouped[q]];
         const lfrv_config &cfg = *jobs[sl.job].cfg;
-        float *U = base + sl.off;
+        float *job = base + sl.off;
         CgProblem &P = probs[q];
         P = CgProblem{};
         P.W = sl.G.W;
         P.H = sl.G.H;
         P.max_iter = cfg.cg_max_iter;
         P.gap_tol = cfg.cg_gap_tol;
-        P.gx = U + 3 * sl.G.N;
-        P.gy = U + 4 * sl.G.N;
-        P.U = sl.seeded ? U + 14 * sl.G.N + 16 : U;
-        P.dA = U + 8 * sl.G.N;
-        P.dB = U + 11 * sl.G.N;
-        P.state = reinterpret_cast<double *>(U + 14 * sl.G.N);
-        P.U0 = sl.seeded ? U : nullptr;
+        P.gx = job + sl.at.gx;
+        P.gy = job + sl.at.gy;
+        P.U = job + result(sl);
+        P.dA = job + sl.at.dA;
+        P.dB = job + sl.at.dB;
+        P.state = reinterpret_cast<double *>(job + sl.at.state);
+        P.U0 = sl.seeded ? job + sl.at.U : nullptr;
         const lfrv_stats *jst = jobs[sl.job].stats;
         const bool traced = jst && jst->energy_trace && jst->trace_capacity > 0;
         P.trace = traced ? ws.trace.as<double>() + trace_off[grouped[q]] : nullptr;
@@ -2280,7 +2282,8 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
         double *part = partial_buf(c, (size_t)14 * resident);
         for (const Group &g : groups) {
             gb.count = reinterpret_cast<unsigned int *>(d_meta + g.off_bars);
-            LFRV_CUDA(launch_cg_batch(reinterpret_cast<const CgProblem *>(d_meta + g.off_probs),
+            LFRV_CUDA(launch_cg_batch(&probs[g.first], (int)g.cnt,
+                                      reinterpret_cast<const CgProblem *>(d_meta + g.off_probs),
                                       reinterpret_cast<const int *>(d_meta + g.off_blocks), g.R, g.used, part,
                                       part + (size_t)7 * resident, gb, s, c->launches));
             for (size_t q = 0; q < g.cnt; ++q) send(batched[grouped[g.first + q]]);
@@ -2327,7 +2330,7 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
     }
     for (const Slot &sl : batched)
         if (!(sent && sent[sl.job]))
-            LFRV_CUDA(cudaMemcpyAsync(jobs[sl.job].d_out, base + sl.off + (sl.seeded ? 14 * sl.G.N + 16 : 0),
+            LFRV_CUDA(cudaMemcpyAsync(jobs[sl.job].d_out, base + sl.off + result(sl),
                                       sizeof(float) * 3 * sl.G.N, cudaMemcpyDeviceToDevice, s));
     sync(c);
     for (lfrv_ctx *l : c->lanes) {
@@ -2338,7 +2341,7 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
         lfrv_stats *st = jobs[sl.job].stats;
         if (!st) continue;
         double state[8];
-        LFRV_CUDA(cudaMemcpy(state, base + sl.off + 14 * sl.G.N, sizeof(state), cudaMemcpyDeviceToHost));
+        LFRV_CUDA(cudaMemcpy(state, base + sl.off + sl.at.state, sizeof(state), cudaMemcpyDeviceToHost));
         st->outer_iterations = (int)state[5];
         st->gap = state[4];
         st->energy = state[3];

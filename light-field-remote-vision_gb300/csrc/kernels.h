@@ -229,7 +229,8 @@ int tv_fgp_default_variant(bool extended);
 constexpr double kTvExtendedBelow = 2e-3;
 
 // One target of an on-chip CG launch (k_cg_strip): its image, buffers and, in a batched launch, the contiguous range of
-// blocks that work on it. dA, dB: 3 N floats each (the exchanged borders). state: [0..2] gamma = |r|^2, [3] E, [4] gap,
+// blocks that work on it. dA, dB: 3 N floats each (the exchanged borders), on 8-byte boundaries (the launchers refuse
+// others). state: [0..2] gamma = |r|^2, [3] E, [4] gap,
 // [5] iterations (written by the problem's first block).
 struct CgProblem {
     int W, H;
@@ -250,9 +251,9 @@ int cg_batch_resident_blocks();
 int cg_batch_rows(const CgProblem *probs, int count);
 int cg_batch_blocks(int W, int H, int R);
 constexpr int kCgBatchMaxRows = 28;
-// gb.count: 8 zeroed words per problem. partA, partB: 7 doubles per block each.
-cudaError_t launch_cg_batch(const CgProblem *d_probs, const int *d_block_prob, int R, int blocks, double *partA,
-                            double *partB, GridBarrier gb, cudaStream_t st, LaunchCounter &lc);
+// gb.count: 8 zeroed words per problem. partA, partB: 7 doubles per block each. d_probs: the `count` problems of probs.
+cudaError_t launch_cg_batch(const CgProblem *probs, int count, const CgProblem *d_probs, const int *d_block_prob, int R,
+                            int blocks, double *partA, double *partB, GridBarrier gb, cudaStream_t st, LaunchCounter &lc);
 
 // Persistent ROF instantiations (iterations per super-step x block size), chosen per image size by the host's
 // autotuner; v indexes them.

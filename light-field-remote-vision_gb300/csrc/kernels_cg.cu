@@ -15,6 +15,7 @@
 #include <cooperative_groups.h>
 #include <cudaTypedefs.h>
 
+#include "batch_layout.h"
 #include "device_common.cuh"
 #include "tma.cuh"
 #include "kernels.h"
@@ -1674,6 +1675,7 @@ cudaError_t launch_cg_persistent(int W, int H, const float *gx, const float *gy,
         one.trace_cap = trace_cap;
         const int R = strip_rows(W, H, strip_sms());
         if (R > 0) {
+            if (!cg_borders_aligned(dA, dB)) return cudaErrorMisalignedAddress;
             one.nb = strip_blocks(W, H, R);
             lc.add(1);
             return launch_strip(R, one.nb, one, nullptr, nullptr, partA, partB, gb, st);
@@ -1735,8 +1737,11 @@ int cg_batch_rows(const CgProblem *probs, int count) {
     return 0;
 }
 
-cudaError_t launch_cg_batch(const CgProblem *d_probs, const int *d_block_prob, int R, int blocks, double *partA,
-                            double *partB, GridBarrier gb, cudaStream_t st, LaunchCounter &lc) {
+cudaError_t launch_cg_batch(const CgProblem *probs, int count, const CgProblem *d_probs, const int *d_block_prob, int R,
+                            int blocks, double *partA, double *partB, GridBarrier gb, cudaStream_t st,
+                            LaunchCounter &lc) {
+    for (int i = 0; i < count; ++i)
+        if (!cg_borders_aligned(probs[i].dA, probs[i].dB)) return cudaErrorMisalignedAddress;
     ProfScope _ps(lc, "cg_batch", st);
     lc.add(1);
     return launch_strip(R, blocks, CgProblem{}, d_probs, d_block_prob, partA, partB, gb, st);
