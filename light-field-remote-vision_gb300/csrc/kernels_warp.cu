@@ -581,12 +581,15 @@ void launch_zbuffer_splat(int V, int w, int h, const float *depth, const WarpCam
     k_zsplat<<<dim3((n + per_block - 1) / per_block, V), 256, 0, st>>>(V, w, h, depth, cams, W, H, zkey, defer);
     lc.add(1);
     if (defer_q) {
-        // as many warps as three blocks per SM hold (the counts are read on the device), fewer for few quads: a block's
-        // launch costs more there than a longer loop
+        // As many warps as three blocks per SM hold (the counts are read on the device), fewer only where even a warp per
+        // eight input quads needs fewer: with dsf 4, or a target camera much closer than the views, every quad is queued
+        // (8 views of 48 x 40, dsf 4, the whole render: 197 us with all blocks, 200 with a warp per 8 quads, 235 with one
+        // per 32, 325 with one per 128; 64^2 and dsf 1, where hardly any is, 155 us with each).
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        launch_pdl(k_zsplat_defer, dim3((unsigned)std::min<long long>(3 * std::max(sms, 1), (long long)V * n / 1024 + 8)), dim3(256), 0, st, w, h, depth, cams, W, H, zkey, defer);
+        const unsigned int blocks = (unsigned)std::min<long long>(3 * std::max(sms, 1), (long long)V * n / 64 + 8);
+        launch_pdl(k_zsplat_defer, dim3(blocks), dim3(256), 0, st, w, h, depth, cams, W, H, zkey, defer);
         lc.add(1);
     }
 }
