@@ -270,8 +270,11 @@ struct SplatSrc {
 };
 
 // Accumulates sum_entries A * payload and sum_entries A (times the optional scale) for target (x, y), entry after entry
-// in the buckets' order. The loads are a chain (bucket bounds, entry, the view's data), so all bounds are read first and
-// the entries four at a time, their data in flight together (8 views of 256^2, dsf 1: the data term 25 -> 17 us).
+// in the buckets' order. The loads are a chain (bucket bounds, entry, the view's data), so up to KS 3 all bounds are read
+// first and the entries four at a time, their data in flight together (8 views of 256^2, dsf 1: the data term 25 -> 17 us).
+// Beyond, KS^2 buckets share the same entries: most are empty, and the registers of the bounds and of four entries take
+// warps away, so bucket and entry are read one after the other (8 views of 129 x 97, faithful IBR_color with dt_beta, six
+// iterations: dsf 4 3278 us by fours, 2195 one by one; dsf 3 1444 and 1285).
 template <int KS, int NCH>
 __device__ __forceinline__ void splat_accumulate(int x, int y, int W, int H, int n, int dsf, int BW,
                                                  const unsigned int *__restrict__ start,
@@ -281,21 +284,30 @@ __device__ __forceinline__ void splat_accumulate(int x, int y, int W, int H, int
 #pragma unroll
     for (int c = 0; c < 3; ++c) acc[c] = 0.f;
     norm = 0.f;
+    constexpr bool kAhead = KS <= 3;
+    constexpr int B = kAhead ? 4 : 1;
     // anchors x - KS + 1 .. x of anchor row y - i are consecutive buckets: tap (j, i)'s is KS - 1 - j of them
     unsigned int bound[KS][KS + 1];
 #pragma unroll
-    for (int i = 0; i < KS; ++i) {
+    for (int i = 0; kAhead && i < KS; ++i) {
         const size_t r = (size_t)(y - i + KS - 1) * BW + x;
 #pragma unroll
         for (int q = 0; q <= KS; ++q) bound[i][q] = __ldg(start + r + q);
     }
-    constexpr int B = 4;
 #pragma unroll
     for (int i = 0; i < KS; ++i) {
 #pragma unroll
         for (int j = 0; j < KS; ++j) {
             const int ax = x - j, ay = y - i;  // anchor whose tap (j, i) lands on (x, y)
-            const unsigned int s = bound[i][KS - 1 - j], e = bound[i][KS - j];
+            unsigned int s, e;
+            if constexpr (kAhead) {
+                s = bound[i][KS - 1 - j];
+                e = bound[i][KS - j];
+            } else {
+                const unsigned int *b = start + (size_t)(ay + KS - 1) * BW + (ax + KS - 1);
+                s = __ldg(b);
+                e = __ldg(b + 1);
+            }
             for (unsigned int k = s; k < e; k += B) {
                 unsigned int ent[B];
                 float tx[B], ty[B], w[B], v[B][NCH > 0 ? NCH : 1];
