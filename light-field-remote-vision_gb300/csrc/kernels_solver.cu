@@ -133,7 +133,9 @@ __global__ void __launch_bounds__(256) k_bucket_fill(int V, int n, int W, int H,
 // from a view's puts two of its pixels into one bucket) and hold an entry of nearly every view, so eight lanes sort each
 // such bucket: its entries in shared memory, every lane counts the entries smaller than its own (they are distinct, so
 // the count is the entry's place). One thread's insertion sort per bucket, which stood here before, made this pass 5.2
-// of the 6.3 ms of a 384^2 target of 80 views; it remains for buckets beyond kSortCap entries.
+// of the 6.3 ms of a 384^2 target of 80 views. It remains for buckets beyond kSortCap entries (80 views with four pixels
+// each in a bucket fit; 320 entries a bucket are 40 KB of shared memory a block), one such bucket per lane, so that a warp
+// sorts 32 of them beside each other and not one per group of eight lanes.
 constexpr int kSortBuckets = 256, kSortLanes = 8, kSortCap = 320;
 
 __device__ __forceinline__ void insertion_sort(unsigned int *a, unsigned int s, unsigned int e) {
@@ -157,19 +159,16 @@ __global__ void __launch_bounds__(kSortBuckets) k_bucket_sort(int nb, const unsi
     unsigned int *own = buf[threadIdx.x / kSortLanes];
     const bool dup = b < nb && bucket_dup(start, mask, mw, nb, b);
     const unsigned int s0 = dup ? start[b] : 0u, n0 = dup ? start[b + 1] - s0 : 0u;
-    unsigned int todo = __ballot_sync(0xffffffffu, dup);
+    if (n0 > (unsigned int)kSortCap) insertion_sort(entries, s0, s0 + n0);
+    unsigned int todo = __ballot_sync(0xffffffffu, dup && n0 <= (unsigned int)kSortCap);
     while (todo) {
         // the next buckets, one per group of lanes
         unsigned int rest = todo;
         for (int g = lane / kSortLanes; g > 0; --g) rest &= rest - 1;
         const int l = rest ? __ffs(rest) - 1 : 0;
         const unsigned int s = __shfl_sync(0xffffffffu, s0, l), have = __shfl_sync(0xffffffffu, n0, l);
-        const unsigned int n = rest ? have : 0u;
+        const unsigned int m = rest ? have : 0u;
         for (int g = 0; g < 32 / kSortLanes; ++g) todo &= todo - 1;
-        if (n > (unsigned int)kSortCap) {
-            if (sub == 0) insertion_sort(entries, s, s + n);
-        }
-        const unsigned int m = n > (unsigned int)kSortCap ? 0u : n;
         const unsigned int padded = (m + 3u) & ~3u;  // the last group of four is filled with the largest key
         for (unsigned int i = sub; i < padded; i += kSortLanes) own[i] = i < m ? entries[s + i] : 0xFFFFFFFFu;
         __syncwarp();
