@@ -306,7 +306,10 @@ __device__ __forceinline__ bool zsplat_vertices(const ViewCam &c, int m, int w, 
 // 0, and of larger ones from word kZdeferHead on, counted in word 1. Those quads are few, but one lane rasterising one
 // of them would hold its whole warp; k_zsplat_defer gives each small box a warp and each large one kZbigParts. When the
 // queue is full the quad is rasterised where it is.
-constexpr int kZdeferHead = 32, kZbigCap = 8192, kZbigBox = 96, kZbigParts = 16;
+// The line between them is where each part has a full pass of its 32 lanes: below, sixteen warps would compute the corners
+// for the work of a few (target cameras ten times closer, splat and queue: 3 x 3 views of 256^2 at dsf 1, boxes of some 100
+// centres, 23 us a warp each, 59 split from 96 centres on, 22 now; 24 views of 128^2 at dsf 2, 400 centres: 32, 57 and 32).
+constexpr int kZdeferHead = 32, kZbigCap = 8192, kZbigParts = 16, kZbigBox = 32 * kZbigParts;
 struct ZDefer {
     unsigned int *q;
     unsigned int cap;
