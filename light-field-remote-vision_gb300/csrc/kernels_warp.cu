@@ -584,14 +584,17 @@ void launch_zbuffer_splat(int V, int w, int h, const float *depth, const WarpCam
     k_zsplat<<<dim3((n + per_block - 1) / per_block, V), 256, 0, st>>>(V, w, h, depth, cams, W, H, zkey, defer);
     lc.add(1);
     if (defer_q) {
-        // As many warps as three blocks per SM hold (the counts are read on the device), fewer only where even a warp per
-        // eight input quads needs fewer: with dsf 4, or a target camera much closer than the views, every quad is queued
-        // (8 views of 48 x 40, dsf 4, the whole render: 197 us with all blocks, 200 with a warp per 8 quads, 235 with one
-        // per 32, 325 with one per 128; 64^2 and dsf 1, where hardly any is, 155 us with each).
+        // As many warps as three blocks per SM hold (the counts are read on the device) where the target has nine pixels or
+        // more per source pixel: there every quad of a surface at the views' distance is queued (8 views of 48 x 40, dsf 4,
+        // the whole render: 197 us with all blocks, 235 with a warp per 32 input quads, 325 with one per 128). Else no more
+        // than a warp per 32 input quads, which also serves target cameras several times closer, while a launch of
+        // hundreds of blocks that find nothing shows in a small render (8 views of 64^2: 136 us, 138 with all blocks).
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const unsigned int blocks = (unsigned)std::min<long long>(3 * std::max(sms, 1), (long long)V * n / 64 + 8);
+        const bool all = (size_t)W * H >= 9 * (size_t)n;
+        const unsigned int blocks =
+            (unsigned)std::min<long long>(3 * std::max(sms, 1), all ? (1 << 20) : (long long)V * n / 256 + 8);
         launch_pdl(k_zsplat_defer, dim3(blocks), dim3(256), 0, st, w, h, depth, cams, W, H, zkey, defer);
         lc.add(1);
     }
