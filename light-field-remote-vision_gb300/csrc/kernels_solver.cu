@@ -1113,12 +1113,12 @@ __global__ void k_sobel(int W, int H, const float *__restrict__ rgb, size_t in_s
 // A thread owns V vertically adjacent pixels: their U, p, tau F and g stay in registers, the neighbours above and
 // below come from registers too except at the ends, and shared memory carries U and the x duals (which the left and
 // right neighbours read) and the y duals of each thread's last pixel. The code of a pixel has no branch for the image:
-//   - a dual whose forward difference does not exist (the last column / row, pixels outside the image) keeps its value;
-//     outside the image it starts at 0, which is what the divergence of the first column / row subtracts;
+//   - a dual whose forward difference does not exist (the last column / row, pixels outside the image) has step 0 and
+//     keeps its value; outside the image it starts at 0, which is what the divergence of the first column / row subtracts;
 //   - what other pixels outside the image hold is in no difference.
-// The difference is left out by a select, not multiplied by 0, and the projection and the prox give what a square root
-// and divisions give also beyond FP32's range (|p| infinite scales by 0, an infinite numerator stays infinite), so that
-// infinite, not-a-number and overflowing values spread as in the reference's loop.
+// Infinite, not-a-number and overflowing values spread as in the reference's loop: a dual whose squared norm is not finite
+// is worked out again, leaving out differences that do not exist (the step of 0 gives 0 times infinity) and scaling by
+// r / inf = 0, off the common path; an infinite numerator of the prox stays infinite.
 // Threads whose pixels the tile no longer depends on skip the iteration; what the rest computes beyond that is stale
 // and stays outside the tile.
 // The projection scales by g / |p| only beyond the ball, as g times a reciprocal square root with one Newton step; the
@@ -1176,8 +1176,7 @@ __global__ void __launch_bounds__((rof_threads<K, TY, V>())) k_rof_persistent(in
     // shared memory that no thread writes (pads) is read too: finite from here on
     for (int i = threadIdx.x; i < 6 * PL + 3 * PY; i += blockDim.x) sm[i] = 0.f;
     __syncthreads();
-    float u[V][3], p[V][6], tf[V][3], r[V];
-    bool fx = false, fy[V];  // the forward differences exist
+    float u[V][3], p[V][6], tf[V][3], r[V], sy[V], sx = 0.f;
     for (int done = 0; done < niter; done += K, ++step) {
         const int iters = min(K, niter - done);
         const float *Ui = (step & 1) ? U1 : U0, *Pi = (step & 1) ? P1 : P0;
@@ -1185,14 +1184,14 @@ __global__ void __launch_bounds__((rof_threads<K, TY, V>())) k_rof_persistent(in
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
             const int gx = (t % tiles_x) * kRofTX - K + lx, gy0 = (t / tiles_x) * TY - K + ly0;
             const bool inx = mine && gx >= 0 && gx < W;
-            fx = inx && gx < W - 1;
+            sx = inx && gx < W - 1 ? sigma : 0.f;
 #pragma unroll
             for (int k = 0; k < V; ++k) {
                 const int gy = gy0 + k;
                 const bool in = inx && gy >= 0 && gy < H;
                 const bool own = tile_x && ly0 + k >= K && ly0 + k < K + TY;
                 const size_t o = in ? (size_t)gy * W + gx : 0;
-                fy[k] = gy >= 0 && gy < H - 1;
+                sy[k] = gy >= 0 && gy < H - 1 ? sigma : 0.f;
                 if (step == 0 || !resident) {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) tf[k][c] = in ? tau * __ldg(F + c * N + o) : 0.f;
@@ -1226,25 +1225,35 @@ __global__ void __launch_bounds__((rof_threads<K, TY, V>())) k_rof_persistent(in
                     for (int c = 0; c < 3; ++c) below[c] = sU[c * PL + V * RX];
 #pragma unroll
                     for (int k = 0; k < V; ++k) {
-                        float n2 = 0.f;
+                        float n2 = 0.f, v[6], scale = 1.f;
 #pragma unroll
                         for (int c = 0; c < 3; ++c) {
                             const float uc = u[k][c];
-                            const float ur = sU[c * PL + k * RX + 1], ud = k + 1 < V ? u[k + 1 < V ? k + 1 : k][c] : below[c];
-                            const float a = fx ? fmaf(sigma, ur - uc, p[k][2 * c]) : p[k][2 * c];
-                            const float b = fy[k] ? fmaf(sigma, ud - uc, p[k][2 * c + 1]) : p[k][2 * c + 1];
-                            p[k][2 * c] = a;
-                            p[k][2 * c + 1] = b;
-                            n2 = fmaf(b, b, fmaf(a, a, n2));
+                            const float ur = sU[c * PL + k * RX + 1];
+                            const float ud = k + 1 < V ? u[k + 1 < V ? k + 1 : k][c] : below[c];
+                            v[2 * c] = fmaf(sx, ur - uc, p[k][2 * c]);
+                            v[2 * c + 1] = fmaf(sy[k], ud - uc, p[k][2 * c + 1]);
+                            n2 = fmaf(v[2 * c + 1], v[2 * c + 1], fmaf(v[2 * c], v[2 * c], n2));
                         }
                         // beyond the ball: p *= g / |p| (a negative radius scales always, as |p| > g does)
                         const float r2 = r[k] < 0.f ? -1.f : r[k] * r[k];
-                        if (n2 > r2) {
-                            const float e = rsqrtf(n2);
-                            const float q = n2 < kInf ? r[k] * fmaf(e * 0.5f, fmaf(-n2 * e, e, 1.f), e) : 0.f;
+                        if (!(n2 <= r2)) {
+                            if (n2 > r2 && n2 < kInf) {
+                                const float e = rsqrtf(n2);
+                                scale = r[k] * fmaf(e * 0.5f, fmaf(-n2 * e, e, 1.f), e);
+                            } else {
+                                n2 = 0.f;
 #pragma unroll
-                            for (int c = 0; c < 6; ++c) p[k][c] *= q;
+                                for (int c = 0; c < 3; ++c) {
+                                    if (!(inx && gx < W - 1)) v[2 * c] = p[k][2 * c];
+                                    if (!(gy0 + k >= 0 && gy0 + k < H - 1)) v[2 * c + 1] = p[k][2 * c + 1];
+                                    n2 = fmaf(v[2 * c + 1], v[2 * c + 1], fmaf(v[2 * c], v[2 * c], n2));
+                                }
+                                if (n2 > r2) scale = n2 < kInf ? r[k] / sqrtf(n2) : 0.f;
+                            }
                         }
+#pragma unroll
+                        for (int c = 0; c < 6; ++c) p[k][c] = v[c] * scale;
 #pragma unroll
                         for (int c = 0; c < 3; ++c) sPx[c * PL + k * RX] = p[k][2 * c];
                     }
