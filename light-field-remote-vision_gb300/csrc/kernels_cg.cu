@@ -16,6 +16,7 @@
 #include <cudaTypedefs.h>
 
 #include "batch_layout.h"
+#include "cg_scalars.h"
 #include "device_common.cuh"
 #include "tma.cuh"
 #include "kernels.h"
@@ -993,8 +994,8 @@ __global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem o
     };
     dots(0, partA, true);
     // The FP64 scalars. An FP64 operation has a latency of some dozens of cycles, so the path every warp waits for
-    // holds only beta, the denominator and an FP32 quotient (warp 0, one channel per lane) beside the stop test (warp
-    // 1); the quotients that the next iteration needs (1 / gamma, 1 / alpha, the energy's decrease) follow on nine
+    // holds only beta, the denominator and the step length (warp 0, one channel per lane; cg_quotient) beside the stop test
+    // (warp 1); the quotients that the next iteration needs (1 / gamma, 1 / alpha, the energy's decrease) follow on nine
     // lanes of the last warp while the others go on (an FP64 instruction holds the SM's pipe as long for one lane as
     // for 32).
     double E = 0.0;  // warp 1's copy is the one in use
@@ -1017,10 +1018,7 @@ __global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem o
                 beta = 0.0;
                 den = del;
             }
-            const float fd = (float)den;
-            float alpha = 0.f;
-            if (den > 0.0) alpha = fd > 1e-30f && fd < 1e30f ? __fdiv_rn((float)gam, fd) : (float)(gam / den);
-            s_coef[threadIdx.x] = alpha;
+            s_coef[threadIdx.x] = den > 0.0 ? cg_quotient(gam, den) : 0.f;
             s_coef[3 + threadIdx.x] = (float)beta;
             s_den[threadIdx.x] = den;
         }
