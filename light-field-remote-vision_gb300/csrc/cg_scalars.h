@@ -23,4 +23,14 @@ LFRV_HD float cg_quotient(double a, double b) {
     return fmaf(fmaf(-q, bl, fmaf(-q, bh, ah) + al), 1.0f / bh, q);
 }
 
+// An unevaluated sum of two floats, and their addition (Knuth's two-sum; the low part holds the rounding errors).
+struct CgSum {
+    float hi, lo;
+};
+LFRV_HD CgSum cg_add(CgSum a, CgSum b) {
+    const float s = a.hi + b.hi, t = s - a.hi;
+    const float err = (a.hi - (s - t)) + (b.hi - t);
+    return {s, (a.lo + b.lo) + err};
+}
+
 }  // namespace lfrv

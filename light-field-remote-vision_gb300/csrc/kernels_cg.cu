@@ -768,7 +768,9 @@ __global__ void __launch_bounds__(kPersistThreads) k_cg_persistent(int W, int H,
 // second exchange. Borders and block partials are double-buffered by iteration parity: a block that has passed the
 // barrier writes the next set while a slower one still reads this one. A step whose denominator is not positive
 // (rounding at FP32's floor, long after the certified gap) restarts from the residual (beta = 0).
-// Dot products: FP32 per lane and warp, FP64 across warps and blocks, as in the streamed form.
+// Dot products: FP32 over the 8 rows of two columns that a lane adds, pairs of floats (CgSum, some 42 bits) across those
+// chunks and a warp's lanes, FP64 across warps and blocks. The streamed form adds fewer pixels a lane, but the lanes of a
+// warp in FP32; with FP32 up to the warp here too, 1792 products would be added before FP64.
 //
 // Measured against the shared-memory form with two barriers an iteration that stood here before: 1024^2 (152 blocks,
 // R = 28) 154 -> 100 us for 7 iterations, 512^2 12.1 -> 5.0 us an iteration, 64^2 9.3 -> 3.4 us. Bound at 1024^2 by the
@@ -779,6 +781,7 @@ constexpr int kStripWarps = kStripUnits * 3, kStripThreads = kStripWarps * 32;
 constexpr int kStripCols = 64;
 constexpr int kStripClusterBlocks = 16, kStripClusterR = 8;
 constexpr int kStripSlots = 7;                               // gamma x 3, delta x 3, the starting energy
+constexpr int kStripChunk = 8;                               // rows that a lane adds in FP32
 
 constexpr int kStripRow = kStripCols + 4;                    // a row of r: 2 words (ghost in the second), 64 columns, ghost
 
@@ -853,7 +856,8 @@ __global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem o
     static_assert(R <= 32, "a ghost column is one value per lane");
     extern __shared__ __align__(16) float strip_mem[];
     __shared__ double sh[8], s_dE[3], s_den[3], s_ig[3], s_ia[3];
-    __shared__ float s_coef[6], red[kStripWarps][3];
+    __shared__ float s_coef[6];
+    __shared__ CgSum red[kStripWarps][3];
     __shared__ int s_stop;
     const int pid = probs ? block_prob[blockIdx.x] : 0;
     const CgProblem P = probs ? probs[pid] : one;
@@ -884,13 +888,13 @@ __global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem o
     float2 X[R], D[R];
     float2 st = {}, sb = {};     // s on the ghost rows
     float sl = 0.f, sr = 0.f;    // s on the ghost columns (row = lane)
-    float e = 0.f;
+    CgSum e = {0.f, 0.f};
     // ---- start: r = b - A x on the unit and its ghost ring (outside the image: the border pixel), F(x)
     if (active) {
         auto start = [&](int px, int py, float &en) {
             return strip_start(W, H, min(max(px, 0), W - 1), min(max(py, 0), H - 1), P.gx, P.gy, U, U0, en);
         };
-        float e0, e1, none;
+        float e0, e1, es = 0.f, none;
         {
             // the ghost ring
             const float2 gt = make_float2(start(x, y0 - 1, none), start(x + 1, y0 - 1, none));
@@ -907,7 +911,11 @@ __global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem o
 #pragma unroll 4
         for (int j = 0; j < nrows; ++j) {
             pair(Rl + j * kStripRow) = make_float2(start(x, y0 + j, e0), start(x + 1, y0 + j, e1));
-            e += (ina ? e0 : 0.f) + (inb ? e1 : 0.f);
+            es += (ina ? e0 : 0.f) + (inb ? e1 : 0.f);
+            if ((j & (kStripChunk - 1)) == kStripChunk - 1 || j == nrows - 1) {
+                e = cg_add(e, {es, 0.f});
+                es = 0.f;
+            }
             Ss[j * 32] = make_float2(0.f, 0.f);
         }
         __syncwarp();
@@ -942,10 +950,16 @@ __global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem o
     // dot products of the current r, w's border into set `set`, block partials into part
     auto dots = [&](int set, double *part, bool energy) {
         float g0 = 0.f, g1 = 0.f, d0 = 0.f, d1 = 0.f;
+        CgSum g = {0.f, 0.f}, d = {0.f, 0.f};
         float *B = border(set, active ? u : 0);
         float2 *Brow = reinterpret_cast<float2 *>(B) + lane;
         float *col = edgeL ? B + 2 * kStripCols : B + 2 * kStripCols + R;
-        if (active)
+        auto fold = [&]() {
+            g = cg_add(g, {(ina ? g0 : 0.f) + (inb ? g1 : 0.f), 0.f});
+            d = cg_add(d, {(ina ? d0 : 0.f) + (inb ? d1 : 0.f), 0.f});
+            g0 = g1 = d0 = d1 = 0.f;
+        };
+        if (active) {
             walk([&](int j, float2 v, float2 w) {
                 if (j == 0) Brow[0] = w;
                 if (j == nrows - 1) Brow[32] = w;
@@ -955,29 +969,34 @@ __global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem o
                 g1 = fmaf(v.y, v.y, g1);
                 d0 = fmaf(v.x, w.x, d0);
                 d1 = fmaf(v.y, w.y, d1);
+                if (R > kStripChunk && (j & (kStripChunk - 1)) == kStripChunk - 1) fold();
             });
-        float g = (ina ? g0 : 0.f) + (inb ? g1 : 0.f), d = (ina ? d0 : 0.f) + (inb ? d1 : 0.f), q = energy ? e : 0.f;
+            fold();
+        }
+        // lanes 0 to 15 go on with g, the others with d
+        auto from = [&](CgSum v, int o) {
+            return CgSum{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
+        };
+        const bool upper = lane >= 16;
+        CgSum h = cg_add(upper ? d : g, from(upper ? g : d, 16));
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            g += __shfl_down_sync(0xffffffffu, g, o);
-            d += __shfl_down_sync(0xffffffffu, d, o);
-            if (energy) q += __shfl_down_sync(0xffffffffu, q, o);
+        for (int o = 8; o > 0; o >>= 1) h = cg_add(h, from(h, o));
+        if (energy) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) e = cg_add(e, from(e, o));
+            if (lane == 0) red[warp][2] = e;
         }
-        if (lane == 0) {
-            red[warp][0] = g;
-            red[warp][1] = d;
-            red[warp][2] = q;
-        }
+        if ((lane & 15) == 0) red[warp][lane >> 4] = h;
         __syncthreads();
         if (threadIdx.x < 6) {
-            const float *v = &red[threadIdx.x % 3][threadIdx.x / 3];
+            const CgSum *v = &red[threadIdx.x % 3][threadIdx.x / 3];
             static_assert(kStripUnits == 4, "four units per channel");
-            part[(size_t)threadIdx.x * G + blockIdx.x] =
-                ((double)v[0] + (double)v[9]) + ((double)v[18] + (double)v[27]);
+            const double hi = ((double)v[0].hi + (double)v[9].hi) + ((double)v[18].hi + (double)v[27].hi);
+            part[(size_t)threadIdx.x * G + blockIdx.x] = hi + (double)((v[0].lo + v[9].lo) + (v[18].lo + v[27].lo));
         } else if (threadIdx.x == 6 && energy) {
             double t = 0.0;
 #pragma unroll
-            for (int k = 0; k < kStripWarps; ++k) t += (double)red[k][2];
+            for (int k = 0; k < kStripWarps; ++k) t += (double)red[k][2].hi + (double)red[k][2].lo;
             part[(size_t)6 * G + blockIdx.x] = t;
         }
     };
