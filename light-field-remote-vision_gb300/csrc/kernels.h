@@ -1,6 +1,7 @@
 // kernels.h -- host-side declarations of the lfrv kernel launchers (internal to liblfrv).
 #pragma once
 
+#include "cg_strip_rule.h"
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -250,7 +251,6 @@ int cg_batch_resident_blocks();
 // one of them at R (0: its borders do not fit dA and dB).
 int cg_batch_rows(const CgProblem *probs, int count);
 int cg_batch_blocks(int W, int H, int R);
-constexpr int kCgBatchMaxRows = 28;
 // gb.count: 8 zeroed words per problem. partA, partB: 7 doubles per block each. d_probs: the `count` problems of probs.
 cudaError_t launch_cg_batch(const CgProblem *probs, int count, const CgProblem *d_probs, const int *d_block_prob, int R,
                             int blocks, double *partA, double *partB, GridBarrier gb, cudaStream_t st, LaunchCounter &lc);

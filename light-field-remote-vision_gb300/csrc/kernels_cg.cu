@@ -776,10 +776,7 @@ __global__ void __launch_bounds__(kPersistThreads) k_cg_persistent(int W, int H,
 // R = 28) 154 -> 100 us for 7 iterations, 512^2 12.1 -> 5.0 us an iteration, 64^2 9.3 -> 3.4 us. Bound at 1024^2 by the
 // walks (about 160 cycles a row of a warp, three warps a scheduler), below 512^2 by the reduction, the barrier and the
 // FP64 scalars between two iterations.
-constexpr int kStripUnits = 4;                               // spatial units per block
 constexpr int kStripWarps = kStripUnits * 3, kStripThreads = kStripWarps * 32;
-constexpr int kStripCols = 64;
-constexpr int kStripClusterBlocks = 16, kStripClusterR = 8;
 constexpr int kStripSlots = 7;                               // gamma x 3, delta x 3, the starting energy
 constexpr int kStripChunk = 8;                               // rows that a lane adds in FP32
 
@@ -788,8 +785,6 @@ constexpr int kStripRow = kStripCols + 4;                    // a row of r: 2 wo
 // per warp: r with its ghost rows (and one row read ahead of need), s
 __host__ __device__ constexpr int strip_warp_floats(int R) { return (R + 3) * kStripRow + R * kStripCols; }
 constexpr size_t strip_smem(int R) { return sizeof(float) * kStripWarps * (size_t)strip_warp_floats(R); }
-// top row, bottom row, left column, right column
-__host__ __device__ constexpr int strip_border(int R) { return 2 * kStripCols + 2 * R; }
 
 // a / b in FP64 for the solver's scalars: an FP32 reciprocal refined by Newton steps in FP64 (a few dependent
 // FMAs instead of the full division sequence, whose latency sits on the path every block waits for). The
@@ -1574,35 +1569,27 @@ cudaError_t launch_poisson_jacobi(int W, int H, int iters, const float *gx, cons
 }
 
 // ------------------------------------------------------------------ strip CG: rule and launch
-static int strip_sms() {
+// Whether a block of k_cg_strip<R> fits an SM of the current device. The attribute belongs to the device's context, which
+// a program may reset, so it is set every time, as the other launchers do, and the occupancy asked with it.
+template <int R>
+static bool strip_ready() {
+    const void *kern = (const void *)k_cg_strip<R>;
+    int per_sm = 0;
+    const bool ok =
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)strip_smem(R)) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kStripThreads, strip_smem(R)) == cudaSuccess &&
+        per_sm >= 1;
+    if (!ok) cudaGetLastError();  // a refused query leaves no error behind
+    return ok;
+}
+
+// Blocks of a strip launch that can be resident at once: one per SM, 0 (every image runs the streamed form) where the
+// largest does not fit.
+static int strip_capacity() {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
-static int strip_blocks(int W, int H, int R) {
-    const int units = ((W + kStripCols - 1) / kStripCols) * ((H + R - 1) / R);
-    return (units + kStripUnits - 1) / kStripUnits;
-}
-
-static constexpr int kStripRows[] = {4, 8, 16, kCgBatchMaxRows};
-
-// Whether the borders of the units fit in dA and in dB (3 N floats each); very thin images do not.
-static bool strip_fits(int W, int H, int R) {
-    return (size_t)((W + kStripCols - 1) / kStripCols) * ((H + R - 1) / R) * 3 * strip_border(R) <= (size_t)3 * W * H;
-}
-
-// Rows per unit for a W x H image on at most `blocks` blocks (one per SM): the smallest R of one cluster while R is
-// at most kStripClusterR, else the smallest R that fits the grid (an iteration's arithmetic is proportional to R,
-// its barrier is not); 0: the image does not fit on chip.
-static int strip_rows(int W, int H, int blocks) {
-    for (int R : kStripRows)
-        if (R <= kStripClusterR && strip_fits(W, H, R) && strip_blocks(W, H, R) <= std::min(kStripClusterBlocks, blocks))
-            return R;
-    for (int R : kStripRows)
-        if (strip_fits(W, H, R) && strip_blocks(W, H, R) <= blocks) return R;
-    return 0;
+    return strip_ready<kCgBatchMaxRows>() ? sms : 0;
 }
 
 template <int R>
@@ -1610,20 +1597,17 @@ static cudaError_t launch_strip_r(int blocks, const CgProblem &one, const CgProb
                                   double *partA, double *partB, GridBarrier gb, cudaStream_t st) {
     const void *kern = (const void *)k_cg_strip<R>;
     const size_t smem = strip_smem(R);
+    if (!strip_ready<R>()) return cudaErrorInvalidConfiguration;
     int dev = 0;
     cudaGetDevice(&dev);
-    // the attributes are per device: set the first time each device launches here
+    // per device: whether one cluster of kStripClusterBlocks can be placed
     static std::mutex mu;
-    static int state[64] = {};  // 1: set, 2: set and one cluster of kStripClusterBlocks can be placed
-    int have = 0;
-    if (dev >= 0 && dev < 64) {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!state[dev]) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-            state[dev] = 1;
-            if (R <= kStripClusterR &&
-                cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+    static int placed[64] = {};  // 0 unknown, 1 yes, -1 no
+    bool fits = false;
+    if (R <= kStripClusterR && dev >= 0 && dev < 64) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+            std::lock_guard<std::mutex> lock(mu);
+            if (placed[dev] == 0) {
                 cudaLaunchConfig_t cfg = {};
                 cfg.gridDim = dim3(kStripClusterBlocks);
                 cfg.blockDim = dim3(kStripThreads);
@@ -1634,13 +1618,13 @@ static cudaError_t launch_strip_r(int blocks, const CgProblem &one, const CgProb
                 cfg.attrs = at;
                 cfg.numAttrs = 1;
                 int n = 0;
-                if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1) state[dev] = 2;
+                placed[dev] = cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1 ? 1 : -1;
             }
-            cudaGetLastError();
+            fits = placed[dev] > 0;
         }
-        have = state[dev];
+        if (!fits) cudaGetLastError();
     }
-    int cluster = (!probs && blocks > 1 && blocks <= kStripClusterBlocks && have == 2) ? 1 : 0;
+    int cluster = (!probs && blocks > 1 && blocks <= kStripClusterBlocks && fits) ? 1 : 0;
     void *args[] = {(void *)&one, (void *)&probs, (void *)&block_prob, &partA, &partB, &gb, &cluster};
     if (cluster) {
         cudaLaunchConfig_t cfg = {};
@@ -1690,7 +1674,7 @@ cudaError_t launch_cg_persistent(int W, int H, const float *gx, const float *gy,
         one.U0 = U0;
         one.trace = trace;
         one.trace_cap = trace_cap;
-        const int R = strip_rows(W, H, strip_sms());
+        const int R = strip_rows(W, H, strip_capacity());
         if (R > 0) {
             if (!cg_borders_aligned(dA, dB)) return cudaErrorMisalignedAddress;
             one.nb = strip_blocks(W, H, R);
@@ -1736,20 +1720,20 @@ cudaError_t launch_cg_faithful(int W, int H, const float *gx, const float *gy, f
     return cudaLaunchCooperativeKernel((const void *)k_cg_faithful, dim3(blocks), dim3(kPersistThreads), args, 0, st);
 }
 
-int cg_batch_resident_blocks() { return strip_sms(); }
+int cg_batch_resident_blocks() { return strip_capacity(); }
 
 int cg_batch_blocks(int W, int H, int R) { return strip_fits(W, H, R) ? strip_blocks(W, H, R) : 0; }
 
 // The smallest R whose blocks of all the images fit the GPU together (as strip_rows for one image); 0: none.
 int cg_batch_rows(const CgProblem *probs, int count) {
-    const int sms = strip_sms();
+    const int capacity = strip_capacity();
     for (int R : kStripRows) {
         long long blocks = 0;
-        for (int i = 0; i < count && blocks <= sms; ++i) {
+        for (int i = 0; i < count && blocks <= capacity; ++i) {
             const int b = cg_batch_blocks(probs[i].W, probs[i].H, R);
-            blocks += b > 0 ? b : sms + 1;
+            blocks += b > 0 ? b : capacity + 1;
         }
-        if (blocks <= sms) return R;
+        if (blocks <= capacity) return R;
     }
     return 0;
 }
