@@ -248,6 +248,12 @@ WgradGemm wgrad_gemm(const lfrv_warmstart *net, int l, int level, int &splits) {
 // 715 us with none, 696 with one, 678 with two, 683 with three, 694 with four).
 constexpr int kMainWgradLayers = 2;
 
+// The stream of layer l's weight gradient: 0 the context stream, 1 the side stream. With per-kernel profiling on, everything
+// stays on the context stream, so that each kernel's event time is its own and not shared with a concurrent one.
+int wgrad_lane(const lfrv_warmstart *net, int l) {
+    return net->ctx->launches.prof || l < kMainWgradLayers ? 0 : 1;
+}
+
 // dW and db of layer l (input x at `level`, output gradient dy) into the flat gradient, on the context stream or on the
 // side stream once the context stream has dy: nothing of the backward pass reads them, so they run beside the data
 // gradients of the layers below, whose grids leave half the chip idle. backward() sizes each stream's partials before the
@@ -255,7 +261,7 @@ constexpr int kMainWgradLayers = 2;
 void conv_wgrad(lfrv_warmstart *net, int l, const void *x, int level, const void *dy) {
     const Layer &L = net->L[l];
     lfrv_ctx *c = net->ctx;
-    const int lane = l < kMainWgradLayers ? 0 : 1;
+    const int lane = wgrad_lane(net, l);
     int splits = 0;
     WgradGemm g = wgrad_gemm(net, l, level, splits);
     g.x = x;
@@ -299,7 +305,7 @@ void backward(lfrv_warmstart *net, const void *in) {
     for (int l = 0; l < kLayers; ++l) {
         int splits = 0;
         const WgradGemm g = wgrad_gemm(net, l, level_of[l], splits);
-        size_t &lane = partial[l < kMainWgradLayers ? 0 : 1];
+        size_t &lane = partial[wgrad_lane(net, l)];
         lane = std::max(lane, (size_t)splits * g.Mpad * g.Cout * sizeof(float));
     }
     for (int i = 0; i < 2; ++i) net->partial[i].ensure(partial[i]);
@@ -329,8 +335,10 @@ void backward(lfrv_warmstart *net, const void *in) {
     conv_wgrad(net, 1, b(A0), level_of[1], b(G1));
     conv_dgrad(net, 1, b(G1), 0, b(GS9), b(A0), b(G0));
     conv_wgrad(net, 0, in, level_of[0], b(G0));
-    LFRV_CUDA(cudaEventRecord(c->side_join, c->side_stream));
-    LFRV_CUDA(cudaStreamWaitEvent(c->stream, c->side_join, 0));
+    if (wgrad_lane(net, kLayers - 1)) {
+        LFRV_CUDA(cudaEventRecord(c->side_join, c->side_stream));
+        LFRV_CUDA(cudaStreamWaitEvent(c->stream, c->side_join, 0));
+    }
 }
 
 // Output head: prediction and/or the loss partials + dY of the last layer (asynchronous).
