@@ -5,15 +5,15 @@
 
 namespace lfrv {
 
-// Float offsets from a target's first float, N pixels: the image U (3 planes), the gradients gx and gy, CG's residual r
-// and exchanged borders dA and dB (3 planes each), 8 doubles of solver state, and for a target seeded by the learned warm
+// Float offsets from a target's first float, N pixels: the image U (3 planes), the gradients gx and gy, CG's
+// exchanged borders dA and dB (3 planes each), 8 doubles of solver state, and for a target seeded by the learned warm
 // start the seed (3 planes) and the network input (N x channels BF16 values). The kernels read and write these in pieces
 // of up to 16 bytes (k_cg_strip's borders as float2, the convolutions' input by TMA and 16-byte copies) whatever N is, so
 // every section, and with `size` every target, starts on kBatchAlign floats.
 constexpr size_t kBatchAlign = 64;  // 256 bytes, as cudaMalloc aligns the pool
 
 struct BatchLayout {
-    size_t U, gx, gy, r, dA, dB, state, seed, input, size;
+    size_t U, gx, gy, dA, dB, state, seed, input, size;
 };
 
 inline BatchLayout batch_layout(size_t N, bool seeded, size_t channels) {
@@ -26,7 +26,6 @@ inline BatchLayout batch_layout(size_t N, bool seeded, size_t channels) {
     L.U = place(3 * N);
     L.gx = place(N);
     L.gy = place(N);
-    L.r = place(3 * N);
     L.dA = place(3 * N);
     L.dB = place(3 * N);
     L.state = place(16);

@@ -1297,8 +1297,7 @@ static void warp(lfrv_ctx *c, int V, int w, int h, const float *depth, const lfr
     if (count_for && tau2) {
         const Buckets B = bucket_buffers(c, *count_for);
         LFRV_CUDA(cudaMemsetAsync(B.count, 0, sizeof(unsigned int) * B.nb, c->stream));
-        if (B.mask)
-            LFRV_CUDA(cudaMemsetAsync(B.mask, 0, sizeof(unsigned long long) * B.nb * B.mask_words, c->stream));
+        LFRV_CUDA(cudaMemsetAsync(B.mask, 0, sizeof(unsigned long long) * B.nb * B.mask_words, c->stream));
         bc.count = B.count;
         bc.mask = B.mask;
         bc.dsf = count_for->dsf;
@@ -2196,13 +2195,15 @@ static void render_views(lfrv_ctx *c, const lfrv_view_job *jobs, int count, lfrv
         const lfrv_stats *jst = jobs[sl.job].stats;
         const bool traced = jst && jst->energy_trace && jst->trace_capacity > 0;
         float *job = base + sl.off;
+        ws.r.ensure(sizeof(float) * 3 * sl.G.N);  // (the streamed form's; such jobs run one after another)
         const size_t np = (size_t)persistent_partials();
         double *part = partial_buf(c, 8 * np);
         const GridBarrier gb = fresh_barrier(c);
-        LFRV_CUDA(launch_cg_persistent(sl.G.W, sl.G.H, job + sl.at.gx, job + sl.at.gy, job + result(sl), job + sl.at.r,
-                                       job + sl.at.dA, job + sl.at.dB, part, part + 4 * np, gb, cfg.cg_max_iter,
-                                       cfg.cg_gap_tol, reinterpret_cast<double *>(job + sl.at.state), s, c->launches,
-                                       sl.seeded ? job + sl.at.U : nullptr, traced ? ws.trace.as<double>() + trace_off[q] : nullptr,
+        LFRV_CUDA(launch_cg_persistent(sl.G.W, sl.G.H, job + sl.at.gx, job + sl.at.gy, job + result(sl),
+                                       ws.r.as<float>(), job + sl.at.dA, job + sl.at.dB, part, part + 4 * np, gb,
+                                       cfg.cg_max_iter, cfg.cg_gap_tol, reinterpret_cast<double *>(job + sl.at.state), s,
+                                       c->launches, sl.seeded ? job + sl.at.U : nullptr,
+                                       traced ? ws.trace.as<double>() + trace_off[q] : nullptr,
                                        traced ? jst->trace_capacity : 0));
         check_launch("batched job CG");
         send(sl);

@@ -166,7 +166,6 @@ void launch_push_pull(int W, int H, bool faithful, const uint8_t *vis, float *U,
                       LaunchCounter &lc);
 
 // ---- IBR_gradient: hole filling and CG (kernels_cg.cu)
-int hole_fill_partials(int nholes);
 void launch_hole_list(int W, int H, const uint8_t *vis, int *holes, int *count, cudaStream_t st, LaunchCounter &lc);
 int cg_partials(int W, int H);
 

@@ -1519,8 +1519,6 @@ void launch_hole_list(int W, int H, const uint8_t *vis, int *holes, int *count, 
     lc.add(3);
 }
 
-int hole_fill_partials(int nholes) { return (nholes + 255) / 256; }
-
 // Blocks of a cooperative launch: every block must be resident at once (the grid barrier waits for all).
 static int coop_blocks(const void *kernel, int want, size_t smem = 0) {
     int dev = 0, sms = 0, per_sm = 0;

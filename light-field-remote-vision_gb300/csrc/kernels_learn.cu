@@ -745,14 +745,14 @@ __global__ void __launch_bounds__(kEpiThreads) k_conv_tma(const ConvGemm g, cons
             }
             __syncthreads();  // the next pass overwrites vs
         }
-    } else if (!s_fail) {
+    }
+    if constexpr (!UP) {
 #pragma unroll 1
-        for (int c0 = (warp >> 2) * 16; c0 < BN; c0 += 32) {
+        for (int c0 = (warp >> 2) * 16; !s_fail && c0 < BN; c0 += 32) {
             float v[16];
             tc_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
-            if constexpr (!UP) conv_store16(g, row, n0 + c0, v, in, s_bias + c0);
-            if constexpr (!UP)
-                if (c0 + 32 < BN) conv_load16(g, row, n0 + c0 + 32, in);
+            conv_store16(g, row, n0 + c0, v, in, s_bias + c0);
+            if (c0 + 32 < BN) conv_load16(g, row, n0 + c0 + 32, in);
         }
     }
     tc_fence_before();

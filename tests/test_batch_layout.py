@@ -24,11 +24,11 @@ int main() {
     for (size_t w = 2; w < 320; ++w)
         for (size_t h = 2; h < 48; ++h)
             for (int seeded = 0; seeded < 2; ++seeded) {
-                const size_t N = w * h, lens[9] = {3 * N, N, N, 3 * N, 3 * N, 3 * N, 16, 3 * N, 24 * N};
+                const size_t N = w * h, lens[8] = {3 * N, N, N, 3 * N, 3 * N, 16, 3 * N, 24 * N};
                 const BatchLayout L = batch_layout(N, seeded != 0, 48);
-                const size_t offs[9] = {L.U, L.gx, L.gy, L.r, L.dA, L.dB, L.state, L.seed, L.input};
+                const size_t offs[8] = {L.U, L.gx, L.gy, L.dA, L.dB, L.state, L.seed, L.input};
                 size_t end = 0;
-                for (int i = 0; i < (seeded ? 9 : 7); ++i) {
+                for (int i = 0; i < (seeded ? 8 : 6); ++i) {
                     bad += (offs[i] * 4) % 16 != 0 || offs[i] < end;  // in order, without overlap
                     end = offs[i] + lens[i];
                 }
@@ -70,6 +70,7 @@ BATCHES = [
     [(1, 27, 21, dict(dsf=3)), (2, 40, 36, {})],
     [(1, 1001, 541, {}), (1, 65, 65, {})],                        # the first needs more than half of the blocks
     [(1, 513 - 2 * k, 415, {}) for k in range(5)],                 # more than one launch holds
+    [(1, 3, 401, {}), (1, 33, 65, {})],                            # the first is too thin for the on-chip form
 ]
 
 
@@ -90,6 +91,23 @@ def test_odd_targets_match_single(ctx, specs):
         assert st.hole_fill_iterations == st1.hole_fill_iterations
         assert abs(st.gap - st1.gap) <= 1e-6 * max(st1.gap, 1e-12) + 1e-9
         assert np.max(np.abs(got - keep[2].cpu().numpy())) < 1e-5
+
+
+@pytest.mark.gpu
+def test_odd_targets_from_host_buffers(ctx):
+    import torch
+
+    made = [job(torch, 1, w, h, seed=k + 11) for k, (w, h) in enumerate([(65, 33), (75, 51), (48, 40)])]
+    ctx.render_views_dev([j for _, j in made])
+    torch.cuda.synchronize()
+    host = [[t.cpu() for t in keep] for keep, _ in made]
+    jobs = []
+    for (views, depth, out), (_, j) in zip(host, made):
+        out.zero_()
+        jobs.append(dict(j, d_views=views.data_ptr(), d_depth=depth.data_ptr(), d_out=out.data_ptr()))
+    ctx.render_views(jobs)
+    for (_, _, out), (keep, _) in zip(host, made):
+        np.testing.assert_array_equal(out.numpy(), keep[2].cpu().numpy())
 
 
 @pytest.mark.gpu
