@@ -976,7 +976,8 @@ static void color_solve(lfrv_ctx *c, const lfrv_config &cfg, const float *img, c
 
 // ------------------------------------------------------------------ IBR_gradient
 // Device state of the persistent solvers, read back after the stream completes (lfrv::finish_stats):
-// [0..2] CG delta, [3] CG energy, [4] CG certified gap, [5] CG iterations, [8] hole-fill iterations.
+// [0..2] CG delta, [3] CG energy, [4] CG certified gap, [5] CG iterations, [8] hole-fill iterations, [9..14] the faithful
+// CG's r0 . r0 and accumulated step denominators between the launches of one solve.
 static double *solver_state(lfrv_ctx *c) {
     c->ws.state.ensure(sizeof(double) * 16);
     return c->ws.state.as<double>();

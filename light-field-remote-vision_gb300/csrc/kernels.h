@@ -8,6 +8,10 @@
 
 namespace lfrv {
 
+// SMs of a GB300: what the tensor-core layers' splits, stages and lanes are sized for (any other count runs, at other
+// loads; grids that must be resident at once ask the device).
+constexpr int kSms = 152;
+
 struct KernelProfiler;
 
 // Counts kernel launches issued by a context; optionally times them per kernel name.

@@ -772,9 +772,9 @@ __global__ void __launch_bounds__(kPersistThreads) k_cg_persistent(int W, int H,
 // chunks and a warp's lanes, FP64 across warps and blocks. The streamed form adds fewer pixels a lane, but the lanes of a
 // warp in FP32; with FP32 up to the warp here too, 1792 products would be added before FP64.
 //
-// Measured against the shared-memory form with two barriers an iteration that stood here before: 1024^2 (152 blocks,
-// R = 28) 154 -> 100 us for 7 iterations, 512^2 12.1 -> 5.0 us an iteration, 64^2 9.3 -> 3.4 us. Bound at 1024^2 by the
-// walks (about 160 cycles a row of a warp, three warps a scheduler), below 512^2 by the reduction, the barrier and the
+// Measured against the shared-memory form with two barriers an iteration that stood here before, 25 iterations: 64^2 249 ->
+// 102 us, 384^2 275 -> 143, 512^2 322 -> 149, 768^2 422 -> 221, 1024^2 (152 blocks, R = 28) 547 -> 317. Bound at 1024^2 by
+// the walks (about 160 cycles a row of a warp, three warps a scheduler), below 512^2 by the reduction, the barrier and the
 // FP64 scalars between two iterations.
 constexpr int kStripWarps = kStripUnits * 3, kStripThreads = kStripWarps * 32;
 constexpr int kStripSlots = 7;                               // gamma x 3, delta x 3, the starting energy
@@ -1865,13 +1865,15 @@ void launch_cg_energy(int W, int H, const float *U, const float *U0, const float
 }  // namespace lfrv
 
 // ====================================================================== allocation-free CG entry point
-// lfrv_cg_solve_static runs k_cg_persistent with all of its scratch in one file-scope device array instead of
-// context buffers: r and the two direction buffers (3 planes of kStaticPixels floats each), the FP64 block
-// partials of phases A and B (4 doubles per block each), 16 doubles of solver state, 64 bytes of barrier words.
+// lfrv_cg_solve_static runs the corrected CG (k_cg_strip, or k_cg_persistent for images too thin for it) with all of its
+// scratch in one file-scope device array instead of context buffers: r and the two buffers of directions or borders (3
+// planes of kStaticPixels floats each), two arrays of FP64 block partials (7 doubles per block of k_cg_strip, one block per
+// SM; 4 per block of k_cg_persistent, at most two per SM), 16 doubles of solver state, 64 bytes of barrier words.
 namespace {
 
 constexpr size_t kStaticPixels = LFRV_CG_STATIC_MAX_PIXELS;
-constexpr int kStaticBlocks = 1024;  // cooperative blocks the partial slots hold (2 per SM for <= 512 SMs)
+constexpr int kStaticBlocks = 1024;  // blocks of k_cg_persistent the partial slots hold (2 per SM for <= 512 SMs)
+static_assert(lfrv::kStripSlots <= 2 * 4, "a block of k_cg_strip per SM needs no more than two of k_cg_persistent");
 constexpr size_t kStaticVecBytes = 9 * kStaticPixels * sizeof(float);
 constexpr size_t kStaticPartBytes = 2 * 4 * (size_t)kStaticBlocks * sizeof(double);
 constexpr size_t kStaticStateBytes = 16 * sizeof(double);
@@ -1951,7 +1953,7 @@ extern "C" int lfrv_cg_solve_static(void *stream, int W, int H, int max_iter, do
     gb.err = reinterpret_cast<int *>(bar + 4);
     LaunchCounter lc;
     e = launch_cg_persistent(W, H, gx, gy, U, r, dA, dB, partA, partB, gb, max_iter, gap_tol, state, st, lc);
-    if (e != cudaSuccess) return fail(LFRV_E_CUDA, "k_cg_persistent launch: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return fail(LFRV_E_CUDA, "CG launch: %s", cudaGetErrorString(e));
     if (iterations || gap) {
         double hs[16];
         int hb[8];

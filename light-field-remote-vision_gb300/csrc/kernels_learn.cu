@@ -1109,7 +1109,8 @@ __global__ void k_pack_weights(int Cout, int Cst, int Cin, int taps, int Kpad, i
 // ------------------------------------------------------------------ launchers
 // A forward layer starts setting up (tensor memory, barriers, indices) while the layer before it ends: twelve layers of one
 // 512^2 image 239 -> 222 us. The data gradients don't: their early blocks would hold shared memory that the weight
-// gradients beside them use (4 images of 256^2, the call without its copy: 690 us with, 665 without).
+// gradients beside them use (a training step with and without: four images of 256^2 735 and 706 us, sixteen 1877 and 1850,
+// one of 512^2 731 and 705; only the smallest would gain, one of 64^2 440 and 472).
 template <typename... Params, typename... Args>
 static cudaError_t launch_layer(const ConvGemm &g, void (*kernel)(Params...), dim3 grid, int threads, int smem,
                                 cudaStream_t st, Args... args) {
@@ -1169,7 +1170,7 @@ static bool tile_shape(const ConvGemm &g, int &R, int &BN, int &smem) {
             const int sm = (g.C / 8) * tile_lbo_px(r) * 16 + kTapStages * (g.C / 8) * (bn + 2) * 16 + 128;
             if (sm > 200 * 1024) continue;
             const int ctas = g.batch * (g.Ho / r) * (g.Wo / 128) * (g.N / bn);
-            const int score = std::min(ctas, 2 * 148);
+            const int score = std::min(ctas, 2 * kSms);
             if (score > best) {
                 best = score;
                 R = r;
@@ -1260,7 +1261,7 @@ static cudaError_t tma_launch(const ConvGemm &g, int bw, int bh, const CUtensorM
     // four stages (what fits of them) when the grid leaves each SM one or two CTAs; two when there are more, which then
     // hide each other's latency: with four the layers of four 256^2 images took 260 us forward, with two 243, and rings
     // of six or eight gave the one-CTA layers nothing
-    const int per_sm = ((int)(grid.x * grid.y * grid.z) + 151) / 152;
+    const int per_sm = ((int)(grid.x * grid.y * grid.z) + kSms - 1) / kSms;
     const int stages = std::min({nk, kTmaMaxStages, per_sm > 2 ? 2 : limit / per_sm / stage});
     return launch_layer(g, k_conv_tma<BN, PARITY, UP>, grid, kEpiThreads, stages * stage + 1024, st, g, mA, mB, bw, bh,
                         cblocks, stages, err);
@@ -1362,7 +1363,7 @@ cudaError_t launch_wgrad_tc(const WgradGemm &g, int splits, int Cout_real, float
         // threads per element: enough to fill the chip where the elements alone do not, at most one a partial
         const size_t vecs = (size_t)Kf * Cst / 4;
         int lanes = 1;
-        while (lanes < 64 && lanes < count && vecs * lanes < (size_t)152 * 2048) lanes *= 2;
+        while (lanes < 64 && lanes < count && vecs * lanes < (size_t)kSms * 2048) lanes *= 2;
         const int width = 256 / lanes;
         r = ReducePart{partial, out, stride, count, Cst, Kf, Cout, lanes, (int)((vecs + width - 1) / width)};
     };
@@ -1395,7 +1396,7 @@ cudaError_t launch_wgrad_tc(const WgradGemm &g, int splits, int Cout_real, float
     return cudaGetLastError();
 }
 
-static int ew_blocks(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 152 * 16); }
+static int ew_blocks(size_t n) { return (int)std::min<size_t>((n + 255) / 256, kSms * 16); }
 
 cudaError_t launch_down_sum(int batch, int Hl, int Wl, int C, const void *ds, void *dt, cudaStream_t st,
                             LaunchCounter &lc) {

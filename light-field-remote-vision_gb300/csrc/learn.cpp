@@ -90,8 +90,8 @@ namespace lfrv {
 
 namespace {
 
-constexpr int kBiasBlocks = 304;
-constexpr int kLossBlocks = 304;
+constexpr int kBiasBlocks = 2 * kSms;
+constexpr int kLossBlocks = 2 * kSms;
 constexpr size_t kParamSlack = 256;  // zeros after the last bias: the padded output head reads 16 bias values
 
 void net_check(lfrv_warmstart *net) {
@@ -236,7 +236,7 @@ WgradGemm wgrad_gemm(const lfrv_warmstart *net, int l, int level, int &splits) {
     g.Mpad = round_up(L.Kf, 128);
     const int P = net->batch * g.Ho * g.Wo;
     const int mt = g.Mpad / 128, max_splits = (P + 63) / 64;
-    splits = std::min(max_splits, std::max(1, (2 * 152 + mt - 1) / mt));
+    splits = std::min(max_splits, std::max(1, (2 * kSms + mt - 1) / mt));
     g.chunk = round_up((P + splits - 1) / splits, 64);
     splits = (P + g.chunk - 1) / g.chunk;
     return g;
@@ -244,8 +244,10 @@ WgradGemm wgrad_gemm(const lfrv_warmstart *net, int l, int level, int &splits) {
 
 // Layers whose weight gradients the context stream computes after the last data gradient; the side stream takes the
 // others. The data gradients take about half as long as the weight gradients, so the last layers, the first's with its
-// 48 channels at full resolution the longest of all, balance the two (4 images of 256^2, the call without its copy:
-// 715 us with none, 696 with one, 678 with two, 683 with three, 694 with four).
+// 48 channels at full resolution the longest of all, balance the two. The layers' shares of the work don't depend on the
+// image, and neither does the best number: a training step with 0, 1, 2, 3, 4 of them takes 467, 465, 472, 483, 498 us for
+// one 64^2 image, 476, 458, 450, 462, 468 for one of 256^2, 743, 716, 708, 711, 725 for four, 1903, 1866, 1852, 1852, 1867
+// for sixteen and 745, 715, 707, 711, 724 for one of 512^2.
 constexpr int kMainWgradLayers = 2;
 
 // The stream of layer l's weight gradient: 0 the context stream, 1 the side stream. With per-kernel profiling on, everything
@@ -469,7 +471,7 @@ static void conv_single(lfrv_ctx *c, int mode, int batch, int Hin, int Win, int 
         g.Kf = Kf;
         g.Mpad = round_up(Kf, 128);
         const int P = batch * Ho * Wo;
-        int splits = std::min((P + 63) / 64, std::max(1, (2 * 152 + g.Mpad / 128 - 1) / (g.Mpad / 128)));
+        int splits = std::min((P + 63) / 64, std::max(1, (2 * kSms + g.Mpad / 128 - 1) / (g.Mpad / 128)));
         g.chunk = round_up((P + splits - 1) / splits, 64);
         splits = (P + g.chunk - 1) / g.chunk;
         part.ensure((size_t)splits * g.Mpad * Cout * sizeof(float));
