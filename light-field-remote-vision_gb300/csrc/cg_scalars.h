@@ -32,5 +32,7 @@ LFRV_HD CgSum cg_add(CgSum a, CgSum b) {
     const float err = (a.hi - (s - t)) + (b.hi - t);
     return {s, (a.lo + b.lo) + err};
 }
+// The sum: the rounding errors of an infinite one are not numbers, and dropped.
+LFRV_HD CgSum cg_result(CgSum a) { return {a.hi, fabsf(a.hi) <= 3.402823466e38f ? a.lo : 0.f}; }
 
 }  // namespace lfrv

@@ -979,9 +979,9 @@ __global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem o
         if (energy) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) e = cg_add(e, from(e, o));
-            if (lane == 0) red[warp][2] = e;
+            if (lane == 0) red[warp][2] = cg_result(e);
         }
-        if ((lane & 15) == 0) red[warp][lane >> 4] = h;
+        if ((lane & 15) == 0) red[warp][lane >> 4] = cg_result(h);
         __syncthreads();
         if (threadIdx.x < 6) {
             const CgSum *v = &red[threadIdx.x % 3][threadIdx.x / 3];
@@ -1029,7 +1029,8 @@ __global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem o
             const double gam = sh[threadIdx.x], del = sh[3 + threadIdx.x];
             double beta = gam * s_ig[threadIdx.x], den = fma(-beta, gam * s_ia[threadIdx.x], del);
             if (!(den > 0.0)) {
-                beta = 0.0;
+                // (a residual whose square is infinite does not restart: infinity by infinity, the channel shows it)
+                beta = gam > 1e300 ? (double)NAN : 0.0;
                 den = del;
             }
             s_coef[threadIdx.x] = den > 0.0 ? cg_quotient(gam, den) : 0.f;
