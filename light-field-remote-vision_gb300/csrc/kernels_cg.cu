@@ -768,17 +768,17 @@ __global__ void __launch_bounds__(kPersistThreads) k_cg_persistent(int W, int H,
 // second exchange. Borders and block partials are double-buffered by iteration parity: a block that has passed the
 // barrier writes the next set while a slower one still reads this one. A step whose denominator is not positive
 // (rounding at FP32's floor, long after the certified gap) restarts from the residual (beta = 0).
-// Dot products: FP32 over the 8 rows of two columns that a lane adds, pairs of floats (CgSum, some 42 bits) across those
-// chunks and a warp's lanes, FP64 across warps and blocks. The streamed form adds fewer pixels a lane, but the lanes of a
+// Dot products: FP32 over four rows (eight where a unit has no more) of two columns that a lane adds, pairs of floats (CgSum,
+// some 42 bits) across those chunks and a warp's lanes, FP64 across warps and blocks. The streamed form adds fewer pixels a lane, but the lanes of a
 // warp in FP32; with FP32 up to the warp here too, 1792 products would be added before FP64.
 //
 // Measured against the shared-memory form with two barriers an iteration that stood here before, 25 iterations: 64^2 249 ->
-// 102 us, 384^2 275 -> 143, 512^2 322 -> 149, 768^2 422 -> 221, 1024^2 (152 blocks, R = 28) 547 -> 317. Bound at 1024^2 by
+// 103 us, 384^2 275 -> 143, 512^2 322 -> 151, 768^2 422 -> 217, 1024^2 (152 blocks, R = 28) 547 -> 315. Bound at 1024^2 by
 // the walks (about 160 cycles a row of a warp, three warps a scheduler), below 512^2 by the reduction, the barrier and the
 // FP64 scalars between two iterations.
 constexpr int kStripWarps = kStripUnits * 3, kStripThreads = kStripWarps * 32;
 constexpr int kStripSlots = 7;                               // gamma x 3, delta x 3, the starting energy
-constexpr int kStripChunk = 8;                               // rows that a lane adds in FP32
+constexpr int kStripChunk = 4;                               // rows that a lane adds in FP32 (the walk's unrolling)
 
 constexpr int kStripRow = kStripCols + 4;                    // a row of r: 2 words (ghost in the second), 64 columns, ghost
 
@@ -889,7 +889,7 @@ __global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem o
         auto start = [&](int px, int py, float &en) {
             return strip_start(W, H, min(max(px, 0), W - 1), min(max(py, 0), H - 1), P.gx, P.gy, U, U0, en);
         };
-        float e0, e1, es = 0.f, none;
+        float e0, e1, none;
         {
             // the ghost ring
             const float2 gt = make_float2(start(x, y0 - 1, none), start(x + 1, y0 - 1, none));
@@ -906,11 +906,7 @@ __global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem o
 #pragma unroll 4
         for (int j = 0; j < nrows; ++j) {
             pair(Rl + j * kStripRow) = make_float2(start(x, y0 + j, e0), start(x + 1, y0 + j, e1));
-            es += (ina ? e0 : 0.f) + (inb ? e1 : 0.f);
-            if ((j & (kStripChunk - 1)) == kStripChunk - 1 || j == nrows - 1) {
-                e = cg_add(e, {es, 0.f});
-                es = 0.f;
-            }
+            e = cg_add(e, {(ina ? e0 : 0.f) + (inb ? e1 : 0.f), 0.f});
             Ss[j * 32] = make_float2(0.f, 0.f);
         }
         __syncwarp();
@@ -964,7 +960,7 @@ __global__ void __launch_bounds__(kStripThreads, 1) k_cg_strip(const CgProblem o
                 g1 = fmaf(v.y, v.y, g1);
                 d0 = fmaf(v.x, w.x, d0);
                 d1 = fmaf(v.y, w.y, d1);
-                if (R > kStripChunk && (j & (kStripChunk - 1)) == kStripChunk - 1) fold();
+                if (R > 2 * kStripChunk && (j & (kStripChunk - 1)) == kStripChunk - 1) fold();
             });
             fold();
         }
