@@ -124,11 +124,11 @@ def algorithmic_bytes(kernel: str, V: int, n: int, N: int, ks: int, cg_iters: in
 # for the C5 target (80 views of 1024^2 -> 2048^2) the z-buffer splat's C2 capture scaled by its algorithmic
 # bytes (at C2 its traffic is 1.03 x its algorithmic bytes: depth maps read once, keys in L2).
 NCU_TRAFFIC_BYTES = {
-    ("zbuffer_splat", 1024 * 1024): 83.942912e6 + 2.418432e6 + 0.335616e6,
-    ("gradient_setup", 1024 * 1024): 221.8e6 + 15.8e6,
+    ("zbuffer_splat", 1024 * 1024): 83.9e6 + 2.8e6 + 0.3e6,
+    ("gradient_setup", 1024 * 1024): 228.4e6 + 16.4e6,
     ("cg_persistent", 1024 * 1024): 21.1e6 + 0.1e6,
     ("zbuffer_splat", 2048 * 2048): 1.03 * (12 * 80 * 1024 * 1024 + 8 * 2048 * 2048),
-    ("rof_persistent", 256 * 256): 3.427584e6 + 0.028928e6,
+    ("rof_persistent", 256 * 256): 3.4e6 + 0.1e6,
 }
 
 

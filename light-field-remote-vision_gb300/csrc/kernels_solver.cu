@@ -1126,7 +1126,7 @@ __global__ void k_sobel(int W, int H, const float *__restrict__ rgb, size_t in_s
 //
 // Bound by the chain of an iteration (two block barriers, shared-memory loads, the projection) and by the super-steps'
 // grid barriers, about 3 us each (waiting for the eight neighbouring blocks alone, with a flag each, took longer). 256^2,
-// 300 iterations (K = 8, TY = 16, V = 2, 128 blocks): 524 -> 352 us against the form before it with two scattered
+// 300 iterations (K = 8, TY = 16, V = 2, 128 blocks): 537 -> 325 us a launch against the form before it with two scattered
 // pixels per thread, border branches, and IEEE square roots and divisions; V = 4 saves instructions but leaves half the
 // warps (398). K, TY and V are picked per image size by the host's autotuner; all give the same values.
 constexpr int kRofTX = 32;

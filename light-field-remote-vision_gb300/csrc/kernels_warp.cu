@@ -308,7 +308,8 @@ __device__ __forceinline__ bool zsplat_vertices(const ViewCam &c, int m, int w, 
 // queue is full the quad is rasterised where it is.
 // The line between them is where each part has a full pass of its 32 lanes: below, sixteen warps would compute the corners
 // for the work of a few (target cameras ten times closer, splat and queue: 3 x 3 views of 256^2 at dsf 1, boxes of some 100
-// centres, 23 us a warp each, 59 split from 96 centres on, 22 now; 24 views of 128^2 at dsf 2, 400 centres: 32, 57 and 32).
+// centres, 23 us a warp each, 59 split from 96 centres on, 22 now; 24 views of 128^2 at dsf 2, 400 centres: 32, 57 and 32; 80 views of 1024^2 at dsf 2
+// with a few of thousands: 1432 split from 96 on, 1396 now).
 constexpr int kZdeferHead = 32, kZbigCap = 8192, kZbigParts = 16, kZbigBox = 32 * kZbigParts;
 struct ZDefer {
     unsigned int *q;
